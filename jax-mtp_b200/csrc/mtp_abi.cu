@@ -33,10 +33,6 @@ std::string g_create_error;
 struct DeviceSchedule {
   Schedule sched;
   uint2* d_entries = nullptr;
-  int* d_n3_pairs = nullptr;   // Schedule::n3_pairs / n3_off (level-structured bases)
-  int* d_n3_off = nullptr;
-  int* d_n3_pairs_half = nullptr;   // the same for the FP64 kernel's half-width groups
-  int* d_n3_off_half = nullptr;
   int* d_warp_steps = nullptr;  // [forward passes, reverse passes][lanes / 32] (Pass::wsteps)
 };
 
@@ -84,8 +80,9 @@ struct mtp_handle {
   // potential tables on the device
   double *d_radial = nullptr, *d_species = nullptr, *d_theta = nullptr, *d_seed_val = nullptr;
   int *d_mapping = nullptr, *d_seed_idx = nullptr, *d_zero = nullptr, *d_abc = nullptr, *d_mk = nullptr;
-  int* d_dense_k = nullptr;
-  int* d_dm_pos = nullptr;   // Schedule::dm_pos (the same for every schedule of the potential)
+  // tables that are the same for every schedule of the potential
+  int *d_dm_pos = nullptr, *d_dm_zero = nullptr, *d_n3_src = nullptr;
+  int *d_mono_word = nullptr, *d_mono_list = nullptr;
   int nseed = 0;
   // input / output / scratch buffers sized by the capacities
   int *d_itypes = nullptr, *d_js = nullptr, *d_jtypes = nullptr, *d_counts = nullptr;
@@ -184,16 +181,18 @@ DevModel make_model(mtp_handle* h, const DeviceSchedule& ds) {
   md.nzero = static_cast<int>(s.zero_list.size());
   md.mono_abc = h->d_abc;
   md.mono_k = h->d_mk;
-  md.dense_k = h->d_dense_k;
+  md.mono_word = h->d_mono_word;
+  md.mono_list = h->d_mono_list;
+  md.n_list = static_cast<int>(s.mono_list.size());
   md.dm_pos = h->d_dm_pos;
-  md.n3_pairs = ds.d_n3_pairs;
-  md.n3_off = ds.d_n3_off;
-  md.n3_pairs_half = ds.d_n3_pairs_half;
-  md.n3_off_half = ds.d_n3_off_half;
+  md.dm_zero = h->d_dm_zero;
+  md.ndm_zero = static_cast<int>(s.dm_zero.size());
+  md.chain_mode = s.chain_mode;
+  md.n3_len = s.n3_len;
+  md.n3_src = h->d_n3_src;
+  std::copy(s.n3_words.begin(), s.n3_words.end(), md.n3_words);
+  std::copy(s.n3_off.begin(), s.n3_off.end(), md.n3_off);
   md.warp_steps = ds.d_warp_steps;
-  md.Q = s.Q;
-  md.npairs = s.npairs;
-  md.tri = s.tri ? 1 : 0;
   for (int v = 0; v <= s.D; ++v) md.nmu[v] = s.nmu[v];
   md.S = h->pot.S;
   md.R = h->pot.R;
@@ -205,6 +204,7 @@ DevModel make_model(mtp_handle* h, const DeviceSchedule& ds) {
   md.Sa = h->pot.Sa;
   md.v_m = s.v_m;
   md.v_dm = s.v_dm;
+  md.n_dm = s.v_part - s.v_dm;
   md.v_zero = s.v_zero;
   md.v_one = s.v_one;
   md.v_size = s.v_size;
@@ -235,22 +235,15 @@ int get_schedule(mtp_handle* h, int lanes, int width, DeviceSchedule** out, bool
     std::string err;
     if (!build_schedule(h->pot, lanes, ds.sched, err, width)) return fail(h, MTP_E_FORMAT, err);
     if (h->d_abc == nullptr) {
-      MTP_CUDA(h, dalloc(&h->d_abc, ds.sched.mono_abc.size()));
-      MTP_CUDA(h, cudaMemcpy(h->d_abc, ds.sched.mono_abc.data(), ds.sched.mono_abc.size() * sizeof(int),
-                             cudaMemcpyHostToDevice));
-      MTP_CUDA(h, dalloc(&h->d_mk, ds.sched.mono_k.size()));
-      MTP_CUDA(h, cudaMemcpy(h->d_mk, ds.sched.mono_k.data(), ds.sched.mono_k.size() * sizeof(int),
-                             cudaMemcpyHostToDevice));
-      MTP_CUDA(h, dalloc(&h->d_dense_k, ds.sched.dense_k.size()));
-      MTP_CUDA(h, cudaMemcpy(h->d_dense_k, ds.sched.dense_k.data(), ds.sched.dense_k.size() * sizeof(int),
-                             cudaMemcpyHostToDevice));
-      MTP_CUDA(h, dalloc(&h->d_dm_pos, ds.sched.dm_pos.size()));
-      MTP_CUDA(h, cudaMemcpy(h->d_dm_pos, ds.sched.dm_pos.data(), ds.sched.dm_pos.size() * sizeof(int),
-                             cudaMemcpyHostToDevice));
-      MTP_CUDA(h, dalloc(&h->d_zero, ds.sched.zero_list.size()));
-      if (!ds.sched.zero_list.empty())
-        MTP_CUDA(h, cudaMemcpy(h->d_zero, ds.sched.zero_list.data(), ds.sched.zero_list.size() * sizeof(int),
-                               cudaMemcpyHostToDevice));
+      const Schedule& t = ds.sched;
+      const std::pair<int**, const std::vector<int>*> tables[] = {
+          {&h->d_abc, &t.mono_abc}, {&h->d_mk, &t.mono_k},   {&h->d_dm_pos, &t.dm_pos},     {&h->d_zero, &t.zero_list},
+          {&h->d_dm_zero, &t.dm_zero}, {&h->d_n3_src, &t.n3_src}, {&h->d_mono_word, &t.mono_word}, {&h->d_mono_list, &t.mono_list}};
+      for (const auto& x : tables) {
+        MTP_CUDA(h, dalloc(x.first, x.second->size()));
+        if (!x.second->empty())
+          MTP_CUDA(h, cudaMemcpy(*x.first, x.second->data(), x.second->size() * sizeof(int), cudaMemcpyHostToDevice));
+      }
     }
     it = h->scheds.emplace(key, ds).first;
   }
@@ -265,20 +258,6 @@ int get_schedule(mtp_handle* h, int lanes, int width, DeviceSchedule** out, bool
     for (const Pass& p : ds.sched.rev) ws.insert(ws.end(), p.wsteps.begin(), p.wsteps.end());
     MTP_CUDA(h, dalloc(&ds.d_warp_steps, ws.size()));
     MTP_CUDA(h, cudaMemcpy(ds.d_warp_steps, ws.data(), ws.size() * sizeof(int), cudaMemcpyHostToDevice));
-    if (ds.sched.tri) {
-      const auto& np = ds.sched.n3_pairs;
-      const auto& no = ds.sched.n3_off;
-      MTP_CUDA(h, dalloc(&ds.d_n3_pairs, np.size()));
-      MTP_CUDA(h, cudaMemcpy(ds.d_n3_pairs, np.data(), np.size() * sizeof(int), cudaMemcpyHostToDevice));
-      MTP_CUDA(h, dalloc(&ds.d_n3_off, no.size()));
-      MTP_CUDA(h, cudaMemcpy(ds.d_n3_off, no.data(), no.size() * sizeof(int), cudaMemcpyHostToDevice));
-      const auto& nph = ds.sched.n3_pairs_half;
-      const auto& noh = ds.sched.n3_off_half;
-      MTP_CUDA(h, dalloc(&ds.d_n3_pairs_half, nph.size()));
-      MTP_CUDA(h, cudaMemcpy(ds.d_n3_pairs_half, nph.data(), nph.size() * sizeof(int), cudaMemcpyHostToDevice));
-      MTP_CUDA(h, dalloc(&ds.d_n3_off_half, noh.size()));
-      MTP_CUDA(h, cudaMemcpy(ds.d_n3_off_half, noh.data(), noh.size() * sizeof(int), cudaMemcpyHostToDevice));
-    }
   }
   *out = &ds;
   return MTP_OK;
@@ -307,14 +286,12 @@ void free_handle(mtp_handle* h) {
   auto F = [](void* p) { if (p) cudaFree(p); };
   for (auto& kv : h->scheds) {
     F(kv.second.d_entries);
-    F(kv.second.d_n3_pairs);
-    F(kv.second.d_n3_off);
-    F(kv.second.d_n3_pairs_half);
-    F(kv.second.d_n3_off_half);
     F(kv.second.d_warp_steps);
   }
   F(h->d_radial); F(h->d_species); F(h->d_theta); F(h->d_seed_val);
-  F(h->d_mapping); F(h->d_seed_idx); F(h->d_zero); F(h->d_abc); F(h->d_mk); F(h->d_dense_k); F(h->d_dm_pos);
+  F(h->d_mapping); F(h->d_seed_idx); F(h->d_zero); F(h->d_abc); F(h->d_mk); F(h->d_dm_pos);
+  F(h->d_dm_zero); F(h->d_n3_src);
+  F(h->d_mono_word); F(h->d_mono_list);
   F(h->d_itypes); F(h->d_js); F(h->d_jtypes); F(h->d_counts); F(h->d_rijs);
   F(h->d_G); F(h->d_E); F(h->d_F); F(h->d_wown); F(h->d_vatom);
   F(h->d_in_cnt); F(h->d_in_ptr); F(h->d_in_cursor); F(h->d_in_slot); F(h->d_blk);

@@ -18,8 +18,7 @@
 //       no two threads ever add into the same value;
 //   N3  per neighbour: dE_i/dr_ij from dE_i/dm of the basic moments by nested
 //       Horner over the monomial simplex (the analytic form of
-//       jax.value_and_grad at jax_backend.py:56), two neighbours per thread
-//       in FP32 and one in FP64,
+//       jax.value_and_grad at jax_backend.py:56), one neighbour per lane,
 //       written to the per-slot gradient array.
 //
 // The A atoms of a block share every lane-program entry: their values are
@@ -65,19 +64,24 @@ struct DevModel {
   const int* zero_list;     // [nzero]
   const int* mono_abc;      // [P][4]
   const int* mono_k;        // [P][kMaxR]
-  const int* dense_k;       // [Q][kMaxR] basic moment of dense slot and mu, or -1
-  int nseed, nzero;
+  const int* mono_word;     // [P] Schedule::mono_word
+  const int* mono_list;     // [n_list] Schedule::mono_list
+  int n_list;
+  const int* dm_zero;       // [ndm_zero] adjoint positions no pass stores and no seed sets
+  int nseed, nzero, ndm_zero;
   int S, R, K, M, B, P, D, Sa;
-  int Q, npairs;
-  int tri;                  // Schedule::tri: step k of a force-phase chain has k / 2 + 1 radial functions,
-                            // and the basic moments' adjoints are in chain order (dm_pos)
+  int chain_mode;           // Schedule::chain_mode
+  int n3_len;               // Schedule::n3_len
+  const int* n3_src;        // [n3_len] adjoint position of each chain slot, or -1
+  // Schedule::n3_words and n3_off, here among the kernel's parameters: read
+  // with a warp-uniform index they are uniform values, so the chains' branches
+  // are uniform ones (from shared memory, every step of a chain paid for a
+  // possibly divergent branch)
+  int n3_words[kMaxChains];
+  unsigned char n3_off[kMaxRunOffsets];
   const int* dm_pos;        // [M] adjoint position of each moment (Schedule::dm_pos)
-  const int* n3_pairs;      // Schedule::n3_pairs / n3_off (level-structured bases)
-  const int* n3_off;
-  const int* n3_pairs_half;  // Schedule::n3_pairs_half / n3_off_half (the FP64 kernel)
-  const int* n3_off_half;
   int nmu[kMaxDegree + 1];  // radial functions with a basic moment of each degree
-  int v_m, v_dm, v_zero, v_one, v_size;
+  int v_m, v_dm, n_dm, v_zero, v_one, v_size;  // n_dm: slots of the adjoint region
   double scaling, rmin, rmax;
 };
 
@@ -95,46 +99,62 @@ struct DevIO {
   void* vscratch;           // [grid][v_size] value space when it lives in global memory
 };
 
-// Shared-memory carve of the evaluation kernel.
 // Lane-program entries requested ahead of use (registers), per thread.
 constexpr int kPrefetch = kStepAlign;
 
-// Radial-function values the basic-moment phase reads with one load: four
-// in FP32 (16 bytes; rows padded to match), one in FP64 (vector loads were
-// measured slower there).
+// Neighbours (or radial functions) one 16-byte shared-memory access covers.
 template <typename T>
-constexpr int kRadVec = sizeof(T) == 4 ? 4 : 1;
+constexpr int kVec = 16 / static_cast<int>(sizeof(T));
 
-// Shared-memory carve of the evaluation kernel for A atoms per block: the
+// Shared-memory carve of the evaluation kernel for A atoms per block.  The
 // value space is interleaved [slot][atom] so one vector access serves all A
-// atoms; neighbour staging is kept per atom.  The dense dE/dm table of the
-// force phase reuses the moment half of the value space (dead once the
-// reverse passes are done) when it fits there (Q R <= M); with the value
-// space in global memory, or when it does not fit, it gets its own region.
+// atoms.  Neighbour staging is kept per atom as rows over the kept neighbours
+// (radial functions f_mu, their derivatives, 1/d, the powers of u_x, u_y and
+// u_z), so that the basic moments read several neighbours with one 16-byte
+// load and the force phase, whose lanes are neighbours, reads without bank
+// conflicts.  The row stride is one 16-byte word more than a multiple of 128
+// bytes: 8 lanes that read 8 different rows at the same neighbour hit 8
+// different bank groups.  The force phase's chain copy of dE/dm ([atom][n3_len])
+// and its partial sums take the moment half of the value space (dead once the
+// reverse passes are done) when they fit there.
 struct SmemLayout {
-  int pws;        // stride of a power row (3 (D+1), rounded up to odd)
-  int rs;         // stride of a radial-function row (R rounded up to kRadVec)
-  bool dmt_in_v;  // dense table in the moment half of the value space
-  bool n3p_in_v;  // force-phase partial sums in the moment half of the value space
-  size_t v, rad, u, f, fp, pw, slot, dmt, n3p, red, cnt, total;
+  int qs;         // stride of a staging row
+  int rows;       // staging rows per atom: R (f), R (f'), 1 (1/d), 3 (D + 1) (powers)
+  int rp;         // radial functions per coefficient row (R rounded up to kVec)
+  int n3s;        // stride of one atom's chain copy
+  size_t v, rad, st, slot, mono, dmc, n3p, red, cnt, total;
 };
 
-// Values of the force phase's partial-sum buffer on level-structured bases:
-// (G_x, G_y, G_z, S) of 32 neighbours from each warp.
-__host__ __device__ inline int n3_partials(int threads) { return 4 * threads; }
+// Force-phase words: one FP64 value or a pair of FP32 ones (struct Force).
+constexpr int kForceBytes = 8;
+
+// Warps that share one chunk of neighbours (32 lanes of `items`) in the force
+// phase: as few as let every chunk of the block have a group (no partial sums
+// to exchange when it is one warp), for rows filled to three quarters.  A rule
+// on the launch alone: an atom's rounding must not depend on the atoms beside
+// it.
+__host__ __device__ inline int n3_group_warps(int NW, int A, int n_pad, int items) {
+  const int chunks = (A * n_pad * 3 / 4 + 32 * items - 1) / (32 * items);
+  int gw = NW;
+  while (gw > 1 && NW / gw < chunks) gw >>= 1;
+  return gw;
+}
 
 template <typename T>
-__host__ __device__ inline SmemLayout smem_layout(int v_size, int M, int S, int R, int K, int D, int n_pad,
-                                                  int threads, int A, bool tri) {
+__host__ __device__ inline int staging_stride(int n_pad) {
+  // long rows are rounded less: their padding would cost more than the bank conflicts
+  return n_pad <= 256 ? ((n_pad + 31) & ~31) + kVec<T> : ((n_pad + 3) & ~3) + 4;
+}
+
+template <typename T>
+__host__ __device__ inline SmemLayout smem_layout(int v_size, int M, int S, int R, int K, int D, int P, int n_list,
+                                                  int n3_len, int n_pad, int threads, int A) {
   SmemLayout L;
-  L.pws = 3 * (D + 1);
-  if ((L.pws & 1) == 0) L.pws += 1;
-  const int Q = (D + 1) * (D + 2) * (D + 3) / 6;
-  // level-structured bases need no dense table; their partial sums use the
-  // moment half of the value space (dead after the reverse passes) when it
-  // holds them
-  L.dmt_in_v = tri || (v_size > 0 && Q * R <= M);
-  L.n3p_in_v = tri && v_size > 0 && n3_partials(threads) <= M * A;
+  L.qs = staging_stride<T>(n_pad);
+  L.rows = 2 * R + 1 + 3 * (D + 1);
+  L.rp = (R + kVec<T> - 1) / kVec<T> * kVec<T>;
+  // an atom's copy starts one 16-byte word further into the banks than the one before
+  L.n3s = ((n3_len + 15) & ~15) + 2;
   size_t o = 0;
   auto take = [&](size_t bytes) {
     size_t at = (o + 31) & ~size_t(31);
@@ -142,17 +162,22 @@ __host__ __device__ inline SmemLayout smem_layout(int v_size, int M, int S, int 
     return at;
   };
   L.v = take(sizeof(T) * v_size * A);
-  L.rad = take(sizeof(T) * S * S * R * K);
-  L.u = take(sizeof(T) * 4 * n_pad * A);
-  L.rs = (R + kRadVec<T> - 1) / kRadVec<T> * kRadVec<T>;
-  L.f = take(sizeof(T) * L.rs * n_pad * A);
-  L.fp = take(sizeof(T) * L.rs * n_pad * A);
-  L.pw = take(sizeof(T) * L.pws * n_pad * A);
+  L.rad = take(sizeof(T) * S * S * L.rp * K);
+  L.st = take(sizeof(T) * L.rows * L.qs * A);
   L.slot = take(sizeof(int) * n_pad * A);
-  L.dmt = L.dmt_in_v ? L.v : take(sizeof(T) * R * Q * A);
-  L.n3p = !tri || L.n3p_in_v ? L.v : take(sizeof(T) * n3_partials(threads));
+  // tables that every iteration reads: with most of the SM's memory taken as
+  // shared memory there is next to no L1 left, and a load from L2 costs more
+  // than a monomial's work
+  L.mono = take(sizeof(int) * P + sizeof(uint16_t) * n_list);
+  const size_t dmc = kForceBytes * static_cast<size_t>(L.n3s) * A;
+  // (G_x, G_y, G_z, S) of each thread, exchanged where several warps share a chunk
+  const bool shared = n3_group_warps(threads / 32, A, n_pad, kForceBytes / static_cast<int>(sizeof(T))) > 1;
+  const size_t n3p = shared ? kForceBytes * 4 * static_cast<size_t>(threads) : 0;
+  const size_t dead = v_size > 0 ? sizeof(T) * M * A : 0;
+  L.dmc = dmc <= dead ? L.v : take(dmc);
+  L.n3p = L.dmc == L.v && dmc + n3p <= dead ? L.v + dmc : take(n3p);
   L.red = take(sizeof(double) * (threads / 32) * A);
-  L.cnt = take(sizeof(int) * (threads / 32 + 8));   // per-warp counts, then per-atom totals
+  L.cnt = take(sizeof(int) * (threads / 32 + A));   // per-warp counts, then the atoms' species
   L.total = (o + 31) & ~size_t(31);
   return L;
 }
@@ -191,17 +216,17 @@ __device__ __forceinline__ double entry_mult<double>(uint32_t y) {
 // any pass: nothing is bounds-tested.  Each entry feeds A atoms:
 // acc[a] += c * V[x][a] * V[y][a]; STORE/ADD flush into V[d][a].
 // Operands are read through Vr and flushes go through V: a pass never reads a
-// slot that it writes, so the two views do not alias.  kEarly: the operand
+// slot that it writes, so the two views do not alias.  The operand
 // gathers of all PF entries in flight are issued before any of their flushes
 // (allowed for the same reason); with the value space in global memory this
 // overlaps PF gathers' latencies (level-28 FP64 forward 54.1 -> 38.4 ms at
 // 32,000 atoms), in shared memory it gains 0.1-0.6 % at the tuned shapes
-// (2.5 % at 256 lanes x 1 atom in FP64).  Both use it.
-template <typename T, int A, int LANES, int PF, bool kEarly>
-__device__ __forceinline__ void run_pass(const uint2* __restrict__ ent, int steps, int tid, T* __restrict__ V,
+// (2.5 % at 256 lanes x 1 atom in FP64).
+template <typename T, int A, int LANES, int PF>
+__device__ __forceinline__ void run_pass(const uint2* __restrict__ ent, int steps, T* __restrict__ V,
                                          const T* __restrict__ Vr) {
   static_assert(PF >= 1 && kStepAlign % PF == 0, "prefetch depth must divide the pass step alignment");
-  const uint2* p = ent + tid;
+  const uint2* p = ent;
   uint2 buf[PF];
 #pragma unroll
   for (int k = 0; k < PF; ++k) buf[k] = __ldg(p + k * LANES);
@@ -215,20 +240,14 @@ __device__ __forceinline__ void run_pass(const uint2* __restrict__ ent, int step
 #pragma unroll
     for (int k = 0; k < PF; ++k) {
       ek[k] = buf[k];
-      if (kEarly) {
-        va[k] = *reinterpret_cast<const Pack<T, A>*>(Vr + (ek[k].x & 0xFFFFu) * A);
-        vb[k] = *reinterpret_cast<const Pack<T, A>*>(Vr + (ek[k].x >> 16) * A);
-      }
+      va[k] = *reinterpret_cast<const Pack<T, A>*>(Vr + (ek[k].x & 0xFFFFu) * A);
+      vb[k] = *reinterpret_cast<const Pack<T, A>*>(Vr + (ek[k].x >> 16) * A);
       buf[k] = __ldg(p + k * LANES);
     }
 #pragma unroll
     for (int k = 0; k < PF; ++k) {
       const uint2 e = ek[k];
       const T c = entry_mult<T>(e.y);
-      if (!kEarly) {
-        va[k] = *reinterpret_cast<const Pack<T, A>*>(Vr + (e.x & 0xFFFFu) * A);
-        vb[k] = *reinterpret_cast<const Pack<T, A>*>(Vr + (e.x >> 16) * A);
-      }
 #pragma unroll
       for (int a = 0; a < A; ++a) acc[a] = dev_fma(c * va[k].v[a], vb[k].v[a], acc[a]);
       if (e.y & (3u << kOpShift)) {
@@ -256,15 +275,6 @@ __device__ __forceinline__ void run_pass(const uint2* __restrict__ ent, int step
 __device__ __forceinline__ int warp_steps_of_lane(const DevModel& md, int tid, int NT) {
   const int p = tid & 31;
   return p < md.nfwd + md.nrev ? __ldg(md.warp_steps + p * (NT >> 5) + (tid >> 5)) : 0;
-}
-
-// run_pass for the block's lane count (128, 256 or 512 threads).
-template <typename T, int A, bool kEarly, int PF = kPrefetch>
-__device__ __forceinline__ void run_pass_n(const uint2* __restrict__ ent, int steps, int lanes, int tid,
-                                           T* __restrict__ V) {
-  if (lanes == 512) run_pass<T, A, 512, PF, kEarly>(ent, steps, tid, V, V);
-  else if (lanes == 256) run_pass<T, A, 256, PF, kEarly>(ent, steps, tid, V, V);
-  else run_pass<T, A, 128, PF, kEarly>(ent, steps, tid, V, V);
 }
 
 // Generic lane-program streamer (used by the dual-number kernels): every thread
@@ -308,230 +318,293 @@ __device__ __forceinline__ void stream_entries_n(const uint2* __restrict__ ent, 
   else stream_entries_t<128, PF, kEarly>(ent, steps, tid, body);
 }
 
-// Force-phase sums of one or (kTwo) two neighbours over this thread's share
-// of the monomial simplex.  With W_s = sum_mu Dm[s][mu] f_mu(d), W'_s the same with
-// f'_mu, and Q(u) = sum_s W_s u_x^a u_y^b u_z^c over slots s = (a, b, c):
-//   G = grad_u Q = (Gx, Gy, Gz),   S = sum_s W'_s u_x^a u_y^b u_z^c.
-// Each (a, b) pair is a Horner chain in u_z over c = D-a-b .. 0 (value and
-// z-derivative), scaled by the stored powers of u_x and u_y.  The dE/dm rows
-// are per atom, so two neighbours share every row load and their chains run
-// side by side.  The tpn threads of a neighbour pair take the (a, b)
-// pairs in snake order (sl, 2 tpn-1-sl, 2 tpn+sl, ...) of the pair order
-// (a + b ascending), so their shares differ by one pair at most.  dmt is the
-// dense table [slot][R] in pair order (bases without the level structure;
-// level-structured ones use n3_transposed).
-template <typename T, int R, bool kTwo>
-__device__ __forceinline__ void n3_sums(const T* __restrict__ dmt, int D,
-                                        int npairs, int D1, const T* __restrict__ fq0, const T* __restrict__ fpq0,
-                                        const T* __restrict__ fq1, const T* __restrict__ fpq1, bool two,
-                                        const T* __restrict__ pw0, const T* __restrict__ pw1, T uz0, T uz1, int sl,
-                                        int tpn, T (&S)[2], T (&Gx)[2], T (&Gy)[2], T (&Gz)[2]) {
-  T f0[R], fp0[R], f1[R], fp1[R];
+// Two FP32 values in a 64-bit register (one instruction for two FMAs).
+using Two = unsigned long long;
+__device__ __forceinline__ Two pack2(float a, float b) {
+  Two r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(Two a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+__device__ __forceinline__ Two mul2(Two a, Two b) {
+  Two r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ Two fma2(Two a, Two b, Two c) {
+  Two r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// What a lane of the force phase computes with: two neighbours of one atom
+// side by side in FP32 (two-wide instructions), one neighbour in FP64.
+template <typename T>
+struct Force;
+template <>
+struct Force<float> {
+  using P = Two;
+  static constexpr int kItems = 2;
+  static __device__ __forceinline__ P make(float a, float b) { return pack2(a, b); }
+  static __device__ __forceinline__ P fma(P a, P b, P c) { return fma2(a, b, c); }
+  static __device__ __forceinline__ P mul(P a, P b) { return mul2(a, b); }
+  static __device__ __forceinline__ float get(P a, int i) { return i ? unpack2(a).y : unpack2(a).x; }
+};
+template <>
+struct Force<double> {
+  using P = double;
+  static constexpr int kItems = 1;
+  static __device__ __forceinline__ P make(double a, double) { return a; }
+  static __device__ __forceinline__ P fma(P a, P b, P c) { return ::fma(a, b, c); }
+  static __device__ __forceinline__ P mul(P a, P b) { return a * b; }
+  static __device__ __forceinline__ double get(P a, int) { return a; }
+};
+
+// Radial functions at step k of a force-phase chain (k = D - degree) on a
+// level-structured basis of offset OFF (Schedule::chain_mode).
+template <int R, int OFF>
+__host__ __device__ constexpr int chain_nm(int k) {
+  return (k + OFF) / 2 + 1 < R ? (k + OFF) / 2 + 1 : R;
+}
+template <int R, int OFF>
+__host__ __device__ constexpr int chain_len(int top) {
+  int n = 0;
+  for (int k = 0; k <= top; ++k) n += chain_nm<R, OFF>(k);
+  return n;
+}
+
+// Horner chain in u_z of the monomial pair (a, b): steps k = 0 .. top go from
+// u_z^top down, step k adding sum_mu g f_mu (and g f'_mu) over its radial
+// functions.  h = sum_c w_c u_z^c, hz its u_z-derivative, hs the same sum with
+// f'.  The chain's adjoints g are contiguous (in FP32 each is there twice, for
+// the lane's two neighbours), so they come in 16-byte loads, requested kAhead
+// words before their use; the last requests may lie past the chain (and are
+// not used).  One body serves every length and stops at top: a body per length
+// was 10 KB of code that each warp walked through once a chain, and fetching
+// it cost more than the arithmetic.
+template <typename T, int R, int OFF>
+__device__ __forceinline__ void chain(int top, const typename Force<T>::P* __restrict__ g,
+                                      const typename Force<T>::P (&f)[R], const typename Force<T>::P (&fp)[R],
+                                      typename Force<T>::P uz, typename Force<T>::P& h, typename Force<T>::P& hz,
+                                      typename Force<T>::P& hs) {
+  using F = Force<T>;
+  using P = typename F::P;
+  constexpr int N = chain_len<R, OFF>(kMaxDegree), NV = (N + 1) / 2, kAhead = 3;
+  struct __align__(16) Word { P v[2]; };
+  const Word* gw = reinterpret_cast<const Word*>(g);
+  P v[NV * 2];
 #pragma unroll
-  for (int mu = 0; mu < R; ++mu) {
-    f0[mu] = fq0[mu];
-    fp0[mu] = fpq0[mu];
-    f1[mu] = kTwo && two ? fq1[mu] : T(0);
-    fp1[mu] = kTwo && two ? fpq1[mu] : T(0);
-  }
-  // diagonal s = a + b of the current pair, its first pair index, and the
-  // first dense slot of the diagonal (pair order: each pair of diagonal s
-  // owns D - s + 1 slots, so slot bases follow without a table lookup)
-  int s = 0, sb = 0, slot_sb = 0;
-  for (int k = 0;; ++k) {
-    const int i = (k >> 1) * 2 * tpn + ((k & 1) ? 2 * tpn - 1 - sl : sl);
-    if (i >= npairs) break;
-    while (i >= sb + s + 1) {
-      sb += s + 1;
-      slot_sb += (s + 1) * (D - s + 1);
-      ++s;
-    }
-    const int ea = i - sb, eb = s - ea, top = D - s;
-    const T* drow = dmt + (slot_sb + ea * (D - s + 1) + top) * R;
-    T h0 = T(0), hz0 = T(0), hs0 = T(0), h1 = T(0), hz1 = T(0), hs1 = T(0);
-    // one Horner step over the table row
-    auto step = [&](const T* row) {
-      T w0 = T(0), wp0 = T(0), w1 = T(0), wp1 = T(0);
+  for (int i = 0; i < kAhead; ++i) *reinterpret_cast<Word*>(v + 2 * i) = gw[i];
+  h = hz = hs = F::make(T(0), T(0));
+  int at = 0;
 #pragma unroll
-      for (int mu = 0; mu < R; ++mu) {
-        const T g = row[mu];
-        w0 = dev_fma(g, f0[mu], w0);
-        wp0 = dev_fma(g, fp0[mu], wp0);
-        if (kTwo) {
-          w1 = dev_fma(g, f1[mu], w1);
-          wp1 = dev_fma(g, fp1[mu], wp1);
-        }
-      }
-      hz0 = dev_fma(hz0, uz0, h0);
-      h0 = dev_fma(h0, uz0, w0);
-      hs0 = dev_fma(hs0, uz0, wp0);
-      if (kTwo) {
-        hz1 = dev_fma(hz1, uz1, h1);
-        h1 = dev_fma(h1, uz1, w1);
-        hs1 = dev_fma(hs1, uz1, wp1);
-      }
-    };
-#pragma unroll 1
-    for (int c = top; c >= 0; --c, drow -= R) step(drow);
-    {
-      const T xa = pw0[ea], yb = pw0[D1 + eb];
-      const T dxa = ea > 0 ? static_cast<T>(ea) * pw0[ea - 1] : T(0);
-      const T dyb = eb > 0 ? static_cast<T>(eb) * pw0[D1 + eb - 1] : T(0);
-      const T xy = xa * yb;
-      Gx[0] = dev_fma(dxa * yb, h0, Gx[0]);
-      Gy[0] = dev_fma(xa * dyb, h0, Gy[0]);
-      Gz[0] = dev_fma(xy, hz0, Gz[0]);
-      S[0] = dev_fma(xy, hs0, S[0]);
+  for (int k = 0; k <= kMaxDegree; ++k) {
+    if (k > top) break;
+    P w = F::make(T(0), T(0)), wp = w;
+#pragma unroll
+    for (int mu = 0; mu < chain_nm<R, OFF>(k); ++mu) {
+      if (at % 2 == 0 && at / 2 + kAhead < NV) *reinterpret_cast<Word*>(v + at + 2 * kAhead) = gw[at / 2 + kAhead];
+      w = F::fma(v[at], f[mu], w);
+      wp = F::fma(v[at], fp[mu], wp);
+      ++at;
     }
-    if (kTwo) {
-      const T xa = pw1[ea], yb = pw1[D1 + eb];
-      const T dxa = ea > 0 ? static_cast<T>(ea) * pw1[ea - 1] : T(0);
-      const T dyb = eb > 0 ? static_cast<T>(eb) * pw1[D1 + eb - 1] : T(0);
-      const T xy = xa * yb;
-      Gx[1] = dev_fma(dxa * yb, h1, Gx[1]);
-      Gy[1] = dev_fma(xa * dyb, h1, Gy[1]);
-      Gz[1] = dev_fma(xy, hz1, Gz[1]);
-      S[1] = dev_fma(xy, hs1, S[1]);
-    }
+    hz = F::fma(hz, uz, h);
+    h = F::fma(h, uz, w);
+    hs = F::fma(hs, uz, wp);
   }
 }
 
-// Force phase on level-structured bases.  The warps form groups of GW =
-// min(warps, kN3GroupWarps); group g takes the chunks of 32 kept neighbours
-// c = g, g + groups, ... (item j = 32 c + lane over the A atoms' lists in
-// turn), and the warps of a group take disjoint sets of monomial pairs
-// (Schedule::n3_pairs, at most 32 per warp; each lane holds one pair word and
-// the warp shuffles it out), so all lanes of a warp read the same adjoint row
-// at every step (one shared-memory wavefront per gather; the A atoms' values
-// of a slot are adjacent) and no lane reduces with its neighbours.  Per item
-// and pair: the Horner chain in u_z over steps k = 0 .. top with the radial
-// functions mu <= k / 2, then the powers of u_x and u_y; the group's partial
-// sums (G, S) meet in P ([4][warps][32]) and its first warp adds them in warp
-// order (deterministic) and writes the slot gradients.
-template <typename T, int A, int R>
-__device__ __forceinline__ void n3_transposed(const DevModel& md, const DevIO& io, const SmemLayout& L,
-                                              unsigned char* smem, const T* __restrict__ V,
-                                              const int (&nv_a)[A], int base, int tid, int NT, T* __restrict__ P) {
-  const int w = tid >> 5, lane = tid & 31, NW = NT >> 5;
-  // FP64 runs groups of half the width (fewer, shorter rounds for its fewer
-  // atoms per block; measured faster there, slower in FP32)
-  constexpr bool kHalf = sizeof(T) == 8;
-  const int* n3_off = kHalf ? md.n3_off_half : md.n3_off;
-  const int* n3_pairs = kHalf ? md.n3_pairs_half : md.n3_pairs;
-  const int GW = min(NW, kHalf ? kN3GroupWarps / 2 : kN3GroupWarps), g = w / GW, wg = w - g * GW, NG = NW / GW;
-  const int D1 = md.D + 1, pws = L.pws, n_pad = io.n_pad;
-  const int p0 = __ldg(n3_off + wg), np = __ldg(n3_off + wg + 1) - p0;
-  const int myword = lane < np ? __ldg(n3_pairs + p0 + lane) : 0;
-  int J = 0;
-#pragma unroll
-  for (int a = 0; a < A; ++a) J += nv_a[a];
-  // every group runs the same number of rounds (the block barriers match)
-  for (int c0 = 0; c0 < J; c0 += 32 * NG) {
-    const int j = c0 + 32 * g + lane;
-    const bool act = j < J;
-    int a = 0, q = act ? j : 0;
-#pragma unroll
-    for (int aa = 0; aa + 1 < A; ++aa)
-      if (a == aa && q >= nv_a[aa]) {
-        q -= nv_a[aa];
-        a = aa + 1;
-      }
-    const T* sF = reinterpret_cast<const T*>(smem + L.f) + (static_cast<size_t>(a) * n_pad + q) * L.rs;
-    const T* sFp = reinterpret_cast<const T*>(smem + L.fp) + (static_cast<size_t>(a) * n_pad + q) * L.rs;
-    const T* sU = reinterpret_cast<const T*>(smem + L.u) + (static_cast<size_t>(a) * n_pad + q) * 4;
-    const T* pw = reinterpret_cast<const T*>(smem + L.pw) + (static_cast<size_t>(a) * n_pad + q) * pws;
-    T f[R], fp[R];
+// The same chain on a basis without the level structure: every step has all R
+// radial functions (zero adjoints where the basis has no moment).
+template <typename T, int R>
+__device__ __forceinline__ void chain_dense(int top, const typename Force<T>::P* __restrict__ g,
+                                            const typename Force<T>::P (&f)[R], const typename Force<T>::P (&fp)[R],
+                                            typename Force<T>::P uz, typename Force<T>::P& h,
+                                            typename Force<T>::P& hz, typename Force<T>::P& hs) {
+  using F = Force<T>;
+  using P = typename F::P;
+  h = hz = hs = F::make(T(0), T(0));
+  for (int k = 0; k <= top; ++k, g += R) {
+    P w = F::make(T(0), T(0)), wp = w;
 #pragma unroll
     for (int mu = 0; mu < R; ++mu) {
-      f[mu] = sF[mu];
-      fp[mu] = sFp[mu];
+      w = F::fma(g[mu], f[mu], w);
+      wp = F::fma(g[mu], fp[mu], wp);
     }
-    const T uz = sU[2];
-    const T* dmv = V + static_cast<size_t>(md.v_dm) * A + a;
-    T Gx = T(0), Gy = T(0), Gz = T(0), Ss = T(0);
-    for (int pi = 0; pi < np; ++pi) {
-      const int word = __shfl_sync(0xffffffffu, myword, pi);
-      if (act) {
-        const int ea = word & 15, eb = (word >> 4) & 15, top = (word >> 8) & 15;
-        const T* drow = dmv + static_cast<size_t>(word >> 12) * A;
-        T h = T(0), hz = T(0), hs = T(0);
+    hz = F::fma(hz, uz, h);
+    h = F::fma(h, uz, w);
+    hs = F::fma(hs, uz, wp);
+  }
+}
+
+// Force phase.  A lane takes one kept neighbour (FP64) or two of one atom, q
+// and q + ceil(nv / 2) (FP32); chunk c holds the lanes j = 32 c + lane over the
+// A atoms' lists in turn.  Groups of GW warps take the chunks in turn; the
+// warps of a group split the monomial pairs (a, b), ordered by b and then a
+// descending, into runs of about equal cost (Schedule::n3_words).
+// Chains of one b are gathered by Horner in u_x as they come, so a pair costs
+// four multiply-adds beside its chain; a segment's end (the last pair of one b
+// or of the run) applies the powers of u_y and of the x-exponent where the
+// segment stopped.  With W_s = sum_mu Dm[s][mu] f_mu(d) over monomials s and
+// W'_s the same with f': G = grad_u sum_s W_s u^s and S = sum_s W'_s u^s.
+// Partial sums of a group's warps are added in warp order (deterministic).
+template <typename T, int A, int R, int MODE>
+__device__ __forceinline__ void force_phase(const DevModel& md, const DevIO& io, const SmemLayout& L,
+                                            unsigned char* smem, const int (&nv_a)[A], int base, int tid, int NT) {
+  using F = Force<T>;
+  using P = typename F::P;
+  constexpr int kItems = F::kItems;
+  const int w = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, NW = NT >> 5;   // known to be warp-uniform
+  const int GW = n3_group_warps(NW, A, io.n_pad, kItems), g = w / GW, wg = w - g * GW, NG = NW / GW;
+  const int lg = 31 - __clz(GW);
+  // offsets of the cut into 2^lg runs follow those of the cuts into fewer
+  const int i0 = md.n3_off[GW - 1 + lg + wg], i1 = md.n3_off[GW + lg + wg];
+  const int D1 = md.D + 1, qs = L.qs, n_pad = io.n_pad;
+  P* part = reinterpret_cast<P*>(smem + L.n3p);
+  int J = 0;
 #pragma unroll
-        for (int k = 0; k <= kMaxDegree; ++k) {
-          if (k > top) break;
-          const T* row = drow + (((k + 1) * (k + 1)) >> 2) * A;
-          T wv = T(0), wp = T(0);
+  for (int a = 0; a < A; ++a) J += (nv_a[a] + kItems - 1) / kItems;
+  // every group runs the same number of rounds (the block's barriers match)
+  for (int r0 = 0; r0 < J; r0 += 32 * NG) {
+    const int j = r0 + 32 * g + lane;
+    const bool act = j < J;
+    int a = 0, q = act ? j : r0, nv = nv_a[0];
 #pragma unroll
-          for (int mu = 0; mu < R; ++mu) {
-            if (mu <= k / 2) {
-              const T g = row[mu * A];
-              wv = dev_fma(g, f[mu], wv);
-              wp = dev_fma(g, fp[mu], wp);
-            }
-          }
-          hz = dev_fma(hz, uz, h);
-          h = dev_fma(h, uz, wv);
-          hs = dev_fma(hs, uz, wp);
+    for (int aa = 0; aa + 1 < A; ++aa)
+      if (a == aa && q >= (nv_a[aa] + kItems - 1) / kItems) {
+        q -= (nv_a[aa] + kItems - 1) / kItems;
+        a = aa + 1;
+        nv = nv_a[aa + 1];
+      }
+    const int h2 = (nv + 1) / 2;                             // the lane's second neighbour is q + h2
+    const int d2 = kItems == 2 && q + h2 < nv ? h2 : 0;      // (an odd list's last lane takes q twice)
+    const T* st = reinterpret_cast<const T*>(smem + L.st) + static_cast<size_t>(a) * L.rows * qs + q;
+    auto row = [&](int r) { return F::make(st[r * qs], st[r * qs + d2]); };
+    const int px = 2 * R + 1, py = px + D1, pz = py + D1;    // rows of the powers
+    const P* dmc = reinterpret_cast<const P*>(smem + L.dmc) + static_cast<size_t>(a) * L.n3s;
+    P f[R], fp[R];
+#pragma unroll
+    for (int mu = 0; mu < R; ++mu) {
+      f[mu] = row(mu);
+      fp[mu] = row(R + mu);
+    }
+    const P ux = row(px + 1), uz = row(pz + 1), zero = F::make(T(0), T(0));
+    P Gx = zero, Gy = zero, Gz = zero, Ss = zero, H = zero, Hx = zero, Hz = zero, Hs = zero;
+    const int iend = r0 + 32 * g < J ? i1 : i0;   // a group without a neighbour left has nothing to add
+    for (int i = i0; i < iend; ++i) {
+      const int word = md.n3_words[i];
+      const int top = word & 15;
+      P h, hz, hs;
+      if (MODE < 0) chain_dense<T, R>(top, dmc + (word >> 16) * 4, f, fp, uz, h, hz, hs);
+      else chain<T, R, MODE < 0 ? 0 : MODE>(top, dmc + (word >> 16) * 4, f, fp, uz, h, hz, hs);
+      Hx = F::fma(Hx, ux, H);
+      H = F::fma(H, ux, h);
+      Hz = F::fma(Hz, ux, hz);
+      Hs = F::fma(Hs, ux, hs);
+      const int ea = (word >> 4) & 15, eb = (word >> 8) & 15;
+      if (ea == 0 || i + 1 == iend) {
+        const P xa = row(px + ea), yb = row(py + eb);
+        const T ca = static_cast<T>(ea), cb = static_cast<T>(eb);
+        const P dxa = F::mul(F::make(ca, ca), row(px + max(ea - 1, 0)));   // 0 where the exponent is 0
+        const P dyb = F::mul(F::make(cb, cb), row(py + max(eb - 1, 0)));
+        const P xy = F::mul(xa, yb);
+        Gx = F::fma(yb, F::fma(xa, Hx, F::mul(dxa, H)), Gx);
+        Gy = F::fma(F::mul(xa, dyb), H, Gy);
+        Gz = F::fma(xy, Hz, Gz);
+        Ss = F::fma(xy, Hs, Ss);
+        H = Hx = Hz = Hs = zero;
+      }
+    }
+    if (GW > 1) {
+      P* mine = part + w * 32 + lane;
+      mine[0] = Gx;
+      mine[NT] = Gy;
+      mine[2 * NT] = Gz;
+      mine[3 * NT] = Ss;
+      __syncthreads();
+      if (wg == 0) {
+        const P one = F::make(T(1), T(1));
+        for (int x = 1; x < GW; ++x) {
+          const P* o = mine + x * 32;
+          Gx = F::fma(one, o[0], Gx);
+          Gy = F::fma(one, o[NT], Gy);
+          Gz = F::fma(one, o[2 * NT], Gz);
+          Ss = F::fma(one, o[3 * NT], Ss);
         }
-        const T xa = pw[ea], yb = pw[D1 + eb];
-        const T dxa = ea > 0 ? static_cast<T>(ea) * pw[ea - 1] : T(0);
-        const T dyb = eb > 0 ? static_cast<T>(eb) * pw[D1 + eb - 1] : T(0);
-        const T xy = xa * yb;
-        Gx = dev_fma(dxa * yb, h, Gx);
-        Gy = dev_fma(xa * dyb, h, Gy);
-        Gz = dev_fma(xy, hz, Gz);
-        Ss = dev_fma(xy, hs, Ss);
       }
     }
-    P[(0 * NW + w) * 32 + lane] = Gx;
-    P[(1 * NW + w) * 32 + lane] = Gy;
-    P[(2 * NW + w) * 32 + lane] = Gz;
-    P[(3 * NW + w) * 32 + lane] = Ss;
-    __syncthreads();
     if (wg == 0 && act) {
-      T gx_ = T(0), gy_ = T(0), gz_ = T(0), s_ = T(0);
-      for (int ww = w; ww < w + GW; ++ww) {
-        gx_ += P[(0 * NW + ww) * 32 + lane];
-        gy_ += P[(1 * NW + ww) * 32 + lane];
-        gz_ += P[(2 * NW + ww) * 32 + lane];
-        s_ += P[(3 * NW + ww) * 32 + lane];
+#pragma unroll
+      for (int k = 0; k < kItems; ++k) {
+        if (k == 1 && d2 == 0) break;
+        const T uxk = F::get(ux, k), uyk = st[(py + 1) * qs + (k ? d2 : 0)], uzk = F::get(uz, k);
+        const T inv_d = st[2 * R * qs + (k ? d2 : 0)];
+        const T Gxk = F::get(Gx, k), Gyk = F::get(Gy, k), Gzk = F::get(Gz, k), Sk = F::get(Ss, k);
+        const T ug = uxk * Gxk + uyk * Gyk + uzk * Gzk;
+        const T gx = uxk * Sk + (Gxk - uxk * ug) * inv_d;
+        const T gy = uyk * Sk + (Gyk - uyk * ug) * inv_d;
+        const T gz = uzk * Sk + (Gzk - uzk * ug) * inv_d;
+        const int slot = reinterpret_cast<const int*>(smem + L.slot)[a * n_pad + q + (k ? d2 : 0)];
+        double* grow = io.pair_grad + (static_cast<size_t>(base + a) * io.nbr_stride + slot) * 3;
+        grow[0] = static_cast<double>(gx);
+        grow[1] = static_cast<double>(gy);
+        grow[2] = static_cast<double>(gz);
+        if (!(isfinite(static_cast<double>(gx)) && isfinite(static_cast<double>(gy)) &&
+              isfinite(static_cast<double>(gz))))
+          atomicOr(io.err, kErrNonFinite);
       }
-      const T ux = sU[0], uy = sU[1], d = sU[3];
-      const T ug = ux * gx_ + uy * gy_ + uz * gz_;
-      const T inv_d = T(1) / d;
-      const T gx = ux * s_ + (gx_ - ux * ug) * inv_d;
-      const T gy = uy * s_ + (gy_ - uy * ug) * inv_d;
-      const T gz = uz * s_ + (gz_ - uz * ug) * inv_d;
-      const int atom = base + a;
-      const int slot = reinterpret_cast<const int*>(smem + L.slot)[a * n_pad + q];
-      double* grow = io.pair_grad + (static_cast<size_t>(atom) * io.nbr_stride + slot) * 3;
-      grow[0] = static_cast<double>(gx);
-      grow[1] = static_cast<double>(gy);
-      grow[2] = static_cast<double>(gz);
-      if (!(isfinite(static_cast<double>(gx)) && isfinite(static_cast<double>(gy)) &&
-            isfinite(static_cast<double>(gz))))
-        atomicOr(io.err, kErrNonFinite);
     }
-    __syncthreads();
+    // the next chunk's partial sums may only overwrite these once they are added
+    if (GW > 1 && r0 + 32 * NG < J) __syncthreads();
   }
 }
 
 // Basic moments of one (atom, monomial) task for NM radial functions:
-// acc[mu] = sum_q f_mu(d_q) u_x^a u_y^b u_z^c over the kept neighbours.  The
-// radial rows (stride rs) are read kRadVec values per load.
-template <typename T, int NM>
-__device__ __forceinline__ void moment_task(const T* __restrict__ sF, const T* __restrict__ sPw, int rs, int pws, int D1,
-                                            int nv, int ea, int eb, int ec, T (&acc)[kMaxR]) {
-  constexpr int VW = kRadVec<T>, NV = (NM + VW - 1) / VW;
-  using V4 = typename std::conditional<sizeof(T) == 4, float4, double>::type;
-#pragma unroll 4
-  for (int q = 0; q < nv; ++q) {
-    const T* pw = sPw + q * pws;
-    const T mono = pw[ea] * pw[D1 + eb] * pw[2 * D1 + ec];
-    T f[NV * VW];
+// acc[mu] = sum_q f_mu(d_q) u_x^a u_y^b u_z^c over the kept neighbours, kVec
+// neighbours per 16-byte load (rows are padded to that with f = 0).  FP32 sums
+// the even and the odd neighbours side by side in two-wide instructions.
+template <int NM>
+__device__ __forceinline__ void moment_task(const float* __restrict__ f, int qs, const float* __restrict__ px,
+                                            const float* __restrict__ py, const float* __restrict__ pz, int nv,
+                                            float (&acc)[kMaxR]) {
+  Two s[NM];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) *reinterpret_cast<V4*>(f + v * VW) = reinterpret_cast<const V4*>(sF + q * rs)[v];
+  for (int mu = 0; mu < NM; ++mu) s[mu] = pack2(0.f, 0.f);
+#pragma unroll 2
+  for (int q = 0; q < nv; q += 4) {
+    const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(px + q), y = *reinterpret_cast<const ulonglong2*>(py + q),
+                     z = *reinterpret_cast<const ulonglong2*>(pz + q);
+    const Two m0 = mul2(mul2(x.x, y.x), z.x), m1 = mul2(mul2(x.y, y.y), z.y);
 #pragma unroll
-    for (int mu = 0; mu < NM; ++mu) acc[mu] = dev_fma(f[mu], mono, acc[mu]);
+    for (int mu = 0; mu < NM; ++mu) {
+      const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(f + mu * qs + q);
+      s[mu] = fma2(g.x, m0, s[mu]);
+      s[mu] = fma2(g.y, m1, s[mu]);
+    }
+  }
+#pragma unroll
+  for (int mu = 0; mu < NM; ++mu) acc[mu] = unpack2(s[mu]).x + unpack2(s[mu]).y;
+}
+
+template <int NM>
+__device__ __forceinline__ void moment_task(const double* __restrict__ f, int qs, const double* __restrict__ px,
+                                            const double* __restrict__ py, const double* __restrict__ pz, int nv,
+                                            double (&acc)[kMaxR]) {
+#pragma unroll 2
+  for (int q = 0; q < nv; q += 2) {
+    const double2 x = *reinterpret_cast<const double2*>(px + q), y = *reinterpret_cast<const double2*>(py + q),
+                  z = *reinterpret_cast<const double2*>(pz + q);
+    const double m0 = x.x * y.x * z.x, m1 = x.y * y.y * z.y;
+#pragma unroll
+    for (int mu = 0; mu < NM; ++mu) {
+      const double2 g = *reinterpret_cast<const double2*>(f + mu * qs + q);
+      acc[mu] = fma(g.x, m0, acc[mu]);
+      acc[mu] = fma(g.y, m1, acc[mu]);
+    }
   }
 }
 
@@ -554,44 +627,134 @@ __device__ __forceinline__ void warp_partials(double (&v)[A], double* red) {
 // space (moments, adjoints, partials) is a private slice of global memory
 // (L1/L2-resident) instead of shared memory; used when it does not fit in
 // shared memory (level 28 in FP64).
-// Register budget per thread: the FP32 one-atom variant runs three 256-thread
-// blocks per SM (80 registers fit 768 threads); the others run one block of
-// up to 512 threads.
-template <typename T, bool kVGlobal, int A>
-struct EvalRegs {
-  static constexpr int value = (sizeof(T) == 4 && !kVGlobal && A == 1) ? 64 : 128;
+// One block's rows of a staging task (atom, slot), as they lie in memory.
+struct RowSlot {
+  double x, y, z;
+  int jt, it, cnt;
 };
 
+// Contraction tree of one block iteration: forward passes, the warps' parts of
+// the site energies (jax_backend.py:101-106), reverse passes.  Ends with a
+// barrier.
+template <typename T, int A, int LANES>
+__device__ __forceinline__ void run_tree(const DevModel& md, T* V, double* sRed, int my_wsteps, int tid) {
+  const uint2* ent = md.entries + tid;
+  // energy terms of this thread, requested before the last forward pass
+  double th[2] = {0.0, 0.0};
+  int at[2] = {0, 0};
+  auto request = [&]() {
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      if (tid + k * LANES < md.Sa) {
+        th[k] = __ldg(md.theta + tid + k * LANES);
+        at[k] = __ldg(md.mapping + tid + k * LANES);
+      }
+  };
+  if (md.nfwd == 0) request();
+  __syncthreads();   // basic moments and adjoint seeds are in place
+  for (int ps = 0; ps < md.nfwd; ++ps) {
+    if (ps == md.nfwd - 1) request();
+    run_pass<T, A, LANES, kPrefetch>(ent + md.fwd[ps].offset, __shfl_sync(0xFFFFFFFFu, my_wsteps, ps), V, V);
+    __syncthreads();
+  }
+  // energy: E_i = xi[t_i] + sum_alpha theta_alpha m[map_alpha] in FP64: warp
+  // sums now, the block sum after the reverse passes' barriers (no barrier of
+  // its own on the critical path)
+  {
+    double ep[A];
+#pragma unroll
+    for (int a = 0; a < A; ++a) ep[a] = 0.0;
+    auto add = [&](double t, int k) {
+      const Pack<T, A> m = *reinterpret_cast<const Pack<T, A>*>(V + (md.v_m + k) * A);
+#pragma unroll
+      for (int a = 0; a < A; ++a) ep[a] = fma(t, static_cast<double>(m.v[a]), ep[a]);
+    };
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      if (tid + k * LANES < md.Sa) add(th[k], at[k]);
+    for (int al = tid + 2 * LANES; al < md.Sa; al += LANES) add(__ldg(md.theta + al), __ldg(md.mapping + al));
+    warp_partials<A>(ep, sRed);
+  }
+  for (int ps = 0; ps < md.nrev; ++ps) {
+    run_pass<T, A, LANES, kPrefetch>(ent + md.rev[ps].offset, __shfl_sync(0xFFFFFFFFu, my_wsteps, md.nfwd + ps), V,
+                                     V);
+    __syncthreads();
+  }
+  if (md.nrev == 0) __syncthreads();
+}
+
 template <typename T, bool kVGlobal, int A>
-__global__ void __maxnreg__((EvalRegs<T, kVGlobal, A>::value)) k_mtp_eval(DevModel md, DevIO io) {
+__global__ void __launch_bounds__(512) k_mtp_eval(DevModel md, DevIO io) {
   extern __shared__ __align__(32) unsigned char smem[];
   const int NT = blockDim.x;
   const int tid = threadIdx.x;
   // this warp's step count of pass p (forward passes, then reverse ones) is
   // held by lane p and shuffled out at the pass: no load before a pass
   const int my_wsteps = warp_steps_of_lane(md, tid, NT);
-  const SmemLayout L = smem_layout<T>(kVGlobal ? 0 : md.v_size, md.M, md.S, md.R, md.K, md.D, io.n_pad, NT, A,
-                                     md.tri != 0);
+  const SmemLayout L = smem_layout<T>(kVGlobal ? 0 : md.v_size, md.M, md.S, md.R, md.K, md.D, md.P, md.n_list, md.n3_len,
+                                      io.n_pad, NT, A);
   T* V = kVGlobal ? reinterpret_cast<T*>(io.vscratch) + static_cast<size_t>(blockIdx.x) * md.v_size * A
                   : reinterpret_cast<T*>(smem + L.v);
   T* sRad = reinterpret_cast<T*>(smem + L.rad);
+  T* sSt = reinterpret_cast<T*>(smem + L.st);
   double* sRed = reinterpret_cast<double*>(smem + L.red);
   int* sCnt = reinterpret_cast<int*>(smem + L.cnt);
-  const int n_pad = io.n_pad;
+  int* sType = sCnt + (NT >> 5);
+  const int n_pad = io.n_pad, qs = L.qs;
+  constexpr int VW = kVec<T>;
 
-  const int S = md.S, R = md.R, K = md.K, P = md.P, D1 = md.D + 1, pws = L.pws;
-  // per-block constants
-  for (int x = tid; x < S * S * R * K; x += NT) sRad[x] = static_cast<T>(md.radial[x]);
+  const int S = md.S, R = md.R, K = md.K, P = md.P, D1 = md.D + 1;
+  // per-block constants; radial coefficients as [pair][n][mu], rows padded to whole 16-byte words
+  for (int x = tid; x < S * S * K * L.rp; x += NT) {
+    const int mu = x % L.rp, n = x / L.rp % K, st = x / (L.rp * K);
+    sRad[x] = mu < R ? static_cast<T>(md.radial[(st * R + mu) * K + n]) : T(0);
+  }
   for (int a = tid; a < A; a += NT) {
     V[md.v_zero * A + a] = T(0);
     V[md.v_one * A + a] = T(1);
   }
+  int* sMono = reinterpret_cast<int*>(smem + L.mono);
+  uint16_t* sList = reinterpret_cast<uint16_t*>(sMono + P);
+  for (int x = tid; x < P; x += NT) sMono[x] = md.mono_word[x];
+  for (int x = tid; x < md.n_list; x += NT) sList[x] = static_cast<uint16_t>(md.mono_list[x]);
   const T rmax = static_cast<T>(md.rmax);
   const T inv_range = static_cast<T>(1.0 / (md.rmax - md.rmin));
   const T rsum = static_cast<T>(md.rmin + md.rmax);
   const T scal = static_cast<T>(md.scaling);
+
+  // staging tasks (atom, slot) with each atom's slots padded to whole warps,
+  // so a warp's ballot covers one atom.  When the block has twice as many
+  // threads as tasks, every task has two threads (role 0: tid < NV, role 1:
+  // the thread NV above it): both load and test the slot (the same ballot),
+  // role 0 stores 1/d and the radial functions, role 1 the powers
+  const int S32 = (io.nbr_stride + 31) & ~31;
+  const int NV = A * S32;
+  const bool split = 2 * NV <= NT;
+  const int span = split ? NV : NT;   // tasks per sweep
+  const int role = split ? (tid < NV ? 0 : tid < 2 * NV ? 1 : 2) : 0;
+  auto load_slot = [&](int at, int v0) {
+    RowSlot r{0.0, 0.0, 0.0, -1, 0, 0};
+    const int v = v0 + (split ? tid - role * NV : tid);
+    const int a = (role < 2 && v < NV) ? v / S32 : A;
+    const int s = v - a * S32, atom = at + a;
+    if (a < A && atom < io.natoms) {
+      r.it = __ldg(io.itypes + atom);
+      r.cnt = io.counts ? __ldg(io.counts + atom) : io.nbr_stride;
+      if (s < io.nbr_stride) {
+        const size_t x = static_cast<size_t>(atom) * io.nbr_stride + s;
+        r.jt = __ldg(io.jtypes + x);
+        r.x = __ldg(io.rijs + 3 * x);
+        r.y = __ldg(io.rijs + 3 * x + 1);
+        r.z = __ldg(io.rijs + 3 * x + 2);
+      }
+    }
+    return r;
+  };
   __syncthreads();
 
+  // the first sweep's rows of the next atoms are loaded before the force
+  // phase of the current ones
+  RowSlot ahead = load_slot(blockIdx.x * A, 0);
   for (int base = blockIdx.x * A; base < io.natoms; base += gridDim.x * A) {
     // ask L2 for the rows of this block's next atoms now, so their staging
     // loads find them there instead of in DRAM (a hint; nothing waits on it)
@@ -609,65 +772,54 @@ __global__ void __maxnreg__((EvalRegs<T, kVGlobal, A>::value)) k_mtp_eval(DevMod
       }
     }
     // moments that are read but never written (the force phase of the
-    // previous atom may have reused their slots for its dense table)
+    // previous atom may have reused their slots), adjoints that no pass stores
+    // and the adjoint seeds
     for (int x = tid; x < md.nzero * A; x += NT) V[(md.v_m + md.zero_list[x / A]) * A + x % A] = T(0);
-    int it_a[A], nv_a[A], cnt_a[A];
-    // ---- N1: staging of every atom of the block ---------------------------
+    for (int x = tid; x < md.ndm_zero * A; x += NT) V[(md.v_dm + md.dm_zero[x / A]) * A + x % A] = T(0);
+    // (requested here, stored after the staging, which hides their latency)
+    int seed_at[2];
+    double seed_v[2];
 #pragma unroll
-    for (int a = 0; a < A; ++a) {
-      const int atom = base + a;
-      const bool real = atom < io.natoms;
-      int it = real ? __ldg(io.itypes + atom) : 0;
-      if (it < 0 || it >= S) {
-        if (tid == 0) atomicOr(io.err, kErrSpecies);
-        it = 0;
-      }
-      it_a[a] = it;
-      int cnt = real ? (io.counts ? __ldg(io.counts + atom) : io.nbr_stride) : 0;
-      if (cnt > n_pad || cnt < 0) {
-        if (tid == 0) atomicOr(io.err, kErrCapacity);
-        cnt = cnt < 0 ? 0 : n_pad;
-      }
-      cnt_a[a] = cnt;
-      nv_a[a] = 0;
+    for (int k = 0; k < 2; ++k) {
+      const int x = tid + k * NT;
+      seed_at[k] = x < md.nseed ? __ldg(md.seed_idx + x) : -1;
+      seed_v[k] = x < md.nseed ? __ldg(md.seed_val + x) : 0.0;
     }
-    // tasks (atom, slot) with each atom's slots padded to whole warps, so a
-    // warp's ballot covers one atom.  In FP64, when the block has twice as
-    // many threads as tasks, every task has two threads (role 0: tid < NV,
-    // role 1: the thread NV above it): both load and test the slot (the same
-    // ballot), role 0 stores the direction and the radial functions, role 1
-    // the powers (measured faster in FP64, not in FP32)
-    const int S32 = (io.nbr_stride + 31) & ~31;
-    const int NV = A * S32;
-    const bool split = sizeof(T) == 8 && 2 * NV <= NT;
-    const int span = split ? NV : NT;   // tasks per sweep
-    const int role = split ? (tid < NV ? 0 : tid < 2 * NV ? 1 : 2) : 0;
+    auto put_seed = [&](int at, double v) {
+      Pack<T, A> p;
+#pragma unroll
+      for (int a = 0; a < A; ++a) p.v[a] = static_cast<T>(v);
+      *reinterpret_cast<Pack<T, A>*>(V + (md.v_dm + at) * A) = p;
+    };
+    int nv_a[A];
+#pragma unroll
+    for (int a = 0; a < A; ++a) nv_a[a] = 0;
+    // ---- N1: staging of every atom of the block ---------------------------
     for (int v0 = 0; v0 < NV; v0 += span) {
+      const RowSlot row = v0 == 0 ? ahead : load_slot(base, v0);
       const int v = v0 + (split ? tid - role * NV : tid);
       const int a = (role < 2 && v < NV) ? v / S32 : A;
-      const int s = v - a * S32;
-      int it = 0, cnt = 0;
-#pragma unroll
-      for (int aa = 0; aa < A; ++aa)
-        if (aa == a) {
-          it = it_a[aa];
-          cnt = cnt_a[aa];
-        }
-      const int atom = base + a;
+      const int s = v - a * S32, atom = base + a;
       const bool real = a < A && atom < io.natoms;
-      const size_t arow = static_cast<size_t>(real ? atom : 0) * io.nbr_stride;
-      const double* rrow = io.rijs + arow * 3;
-      const int* trow = io.jtypes + arow;
-      double* grow = io.pair_grad + arow * 3;
+      int it = row.it, cnt = row.cnt;
+      if (real && (it < 0 || it >= S)) {
+        if (s == 0) atomicOr(io.err, kErrSpecies);
+        it = 0;
+      }
+      if (real && (cnt > n_pad || cnt < 0)) {
+        if (s == 0) atomicOr(io.err, kErrCapacity);
+        cnt = cnt < 0 ? 0 : n_pad;
+      }
+      if (a < A && s == 0) sType[a] = it;
       bool valid = false;
       T rx = T(0), ry = T(0), rz = T(0), d = T(0);
       int jt = -1;
       if (real && s < io.nbr_stride) {
         if (s < cnt) {
-          jt = __ldg(trow + s);
-          rx = static_cast<T>(__ldg(rrow + 3 * s));
-          ry = static_cast<T>(__ldg(rrow + 3 * s + 1));
-          rz = static_cast<T>(__ldg(rrow + 3 * s + 2));
+          jt = row.jt;
+          rx = static_cast<T>(row.x);
+          ry = static_cast<T>(row.y);
+          rz = static_cast<T>(row.z);
           if (jt >= S) {
             atomicOr(io.err, kErrSpecies);
             jt = -1;
@@ -677,75 +829,61 @@ __global__ void __maxnreg__((EvalRegs<T, kVGlobal, A>::value)) k_mtp_eval(DevMod
           valid = (jt >= 0) && (r2 > T(0)) && (d < rmax);
         }
         if (!valid && role == 0) {
-          grow[3 * s] = 0.0;
-          grow[3 * s + 1] = 0.0;
-          grow[3 * s + 2] = 0.0;
+          double* grow = io.pair_grad + (static_cast<size_t>(atom) * io.nbr_stride + s) * 3;
+          grow[0] = 0.0;
+          grow[1] = 0.0;
+          grow[2] = 0.0;
         }
       }
       const unsigned bal = __ballot_sync(0xffffffffu, valid);
-      const int w = tid >> 5, l = tid & 31, nw = NT >> 5;
+      const int w = tid >> 5, l = tid & 31;
       const int wt = w - role * (NV >> 5);   // the role-0 warp of these tasks
       if (l == 0 && role == 0) sCnt[w] = __popc(bal);
       __syncthreads();
-      if (tid == 0) {
-        // exclusive offsets of each warp within its atom's kept slots of this
-        // sweep; per-atom totals after the warp counts
-        int accn = 0, cur = -1;
-        for (int i = 0; i < (span >> 5); ++i) {
-          const int ai = (v0 + 32 * i) / S32;
-          if (ai != cur) {
-            if (cur >= 0 && cur < A) sCnt[nw + cur] = accn;
-            cur = ai;
-            accn = 0;
-          }
-          const int c = sCnt[i];
-          sCnt[i] = accn;
-          accn += c;
-        }
-        if (cur >= 0 && cur < A) sCnt[nw + cur] = accn;
-      }
-      __syncthreads();
-      if (valid) {
-        int nv = 0;
+      // lane l looks at the count of warp l: sums over the warps of an atom,
+      // and over those before this one
+      const int nws = span >> 5;   // at most 16
+      const int wa = l < nws ? (v0 + 32 * l) / S32 : A;
+      const int wc = l < nws ? sCnt[l] : 0;
+      const int before = __reduce_add_sync(0xffffffffu, wa == a && l < wt ? wc : 0);
+      int nv = 0;
 #pragma unroll
-        for (int aa = 0; aa < A; ++aa)
-          if (aa == a) nv = nv_a[aa];
-        const int q = nv + sCnt[wt] + __popc(bal & ((1u << l) - 1u));
-        T* sU = reinterpret_cast<T*>(smem + L.u) + static_cast<size_t>(a) * 4 * n_pad;
-        T* sF = reinterpret_cast<T*>(smem + L.f) + static_cast<size_t>(a) * L.rs * n_pad;
-        T* sFp = reinterpret_cast<T*>(smem + L.fp) + static_cast<size_t>(a) * L.rs * n_pad;
-        T* sPw = reinterpret_cast<T*>(smem + L.pw) + static_cast<size_t>(a) * pws * n_pad;
-        int* sSlot = reinterpret_cast<int*>(smem + L.slot) + a * n_pad;
+      for (int aa = 0; aa < A; ++aa)
+        if (aa == a) nv = nv_a[aa];
+#pragma unroll
+      for (int aa = 0; aa < A; ++aa) nv_a[aa] += __reduce_add_sync(0xffffffffu, wa == aa ? wc : 0);
+      if (valid) {
+        const int q = nv + before + __popc(bal & ((1u << l) - 1u));
+        T* st = sSt + static_cast<size_t>(a) * L.rows * qs + q;
         const T inv_d = T(1) / d;
-        const T ux = rx * inv_d, uy = ry * inv_d, uz = rz * inv_d;
         if (role == 0) {
-          sU[4 * q] = ux;
-          sU[4 * q + 1] = uy;
-          sU[4 * q + 2] = uz;
-          sU[4 * q + 3] = d;
-          sSlot[q] = s;
+          st[2 * R * qs] = inv_d;
+          reinterpret_cast<int*>(smem + L.slot)[a * n_pad + q] = s;
           // Chebyshev T_n(x) and dT_n/dx by their recurrences, folded into
           // sum_n c[t_i, t_j, mu, n] T_n for every mu as the terms appear
           const T x = (T(2) * d - rsum) * inv_range;
           const T dxdd = T(2) * inv_range;
-          const T* c = sRad + (static_cast<size_t>(it) * S + jt) * R * K;
+          struct __align__(16) Word { T v[VW]; };
+          const Word* c = reinterpret_cast<const Word*>(sRad + (static_cast<size_t>(it) * S + jt) * K * L.rp);
+          const int nw = L.rp / VW;
           T bas[kMaxR], dbas[kMaxR];
 #pragma unroll
-          for (int mu = 0; mu < kMaxR; ++mu) {
-            bas[mu] = mu < R ? c[mu * K] : T(0);   // T_0 = 1, T_0' = 0
-            dbas[mu] = T(0);
-          }
-          T t_prev = T(1), t_cur = x, dt_prev = T(0), dt_cur = T(1);
-          for (int n = 1; n < K; ++n) {
+          for (int mu = 0; mu < kMaxR; ++mu) bas[mu] = dbas[mu] = T(0);
+          T t_prev = T(0), t_cur = T(1), dt_prev = T(0), dt_cur = T(0);   // T_0 = 1, T_0' = 0
+          for (int n = 0; n < K; ++n) {
 #pragma unroll
-            for (int mu = 0; mu < kMaxR; ++mu) {
-              if (mu < R) {
-                bas[mu] = dev_fma(c[mu * K + n], t_cur, bas[mu]);
-                dbas[mu] = dev_fma(c[mu * K + n], dt_cur, dbas[mu]);
+            for (int i = 0; i < kMaxR / VW; ++i) {
+              if (i < nw) {
+                const Word cw = c[n * nw + i];
+#pragma unroll
+                for (int k = 0; k < VW; ++k) {
+                  bas[i * VW + k] = dev_fma(cw.v[k], t_cur, bas[i * VW + k]);
+                  dbas[i * VW + k] = dev_fma(cw.v[k], dt_cur, dbas[i * VW + k]);
+                }
               }
             }
-            const T t_next = T(2) * x * t_cur - t_prev;
-            const T dt_next = T(2) * t_cur + T(2) * x * dt_cur - dt_prev;
+            const T t_next = n == 0 ? x : T(2) * x * t_cur - t_prev;
+            const T dt_next = n == 0 ? T(1) : T(2) * t_cur + T(2) * x * dt_cur - dt_prev;
             t_prev = t_cur;
             t_cur = t_next;
             dt_prev = dt_cur;
@@ -756,224 +894,137 @@ __global__ void __maxnreg__((EvalRegs<T, kVGlobal, A>::value)) k_mtp_eval(DevMod
 #pragma unroll
           for (int mu = 0; mu < kMaxR; ++mu) {
             if (mu < R) {
-              sF[q * L.rs + mu] = scal * smooth * bas[mu];
-              sFp[q * L.rs + mu] = scal * (T(-2) * gap * bas[mu] + smooth * dbas[mu] * dxdd);
+              st[mu * qs] = scal * smooth * bas[mu];
+              st[(R + mu) * qs] = scal * (T(-2) * gap * bas[mu] + smooth * dbas[mu] * dxdd);
             }
           }
         }
         if (role == 1 || !split) {
-          T* pw = sPw + q * pws;
+          const T ux = rx * inv_d, uy = ry * inv_d, uz = rz * inv_d;
+          T* pw = st + (2 * R + 1) * qs;
           T px = T(1), py = T(1), pz = T(1);
           for (int e = 0; e < D1; ++e) {
-            pw[e] = px;
-            pw[D1 + e] = py;
-            pw[2 * D1 + e] = pz;
+            pw[e * qs] = px;
+            pw[(D1 + e) * qs] = py;
+            pw[(2 * D1 + e) * qs] = pz;
             px *= ux;
             py *= uy;
             pz *= uz;
           }
         }
       }
-      // atoms touched by this sweep add its kept count
-#pragma unroll
-      for (int aa = 0; aa < A; ++aa) {
-        const int first = v0 / S32, last = (v0 + span - 1) / S32;
-        if (aa >= first && aa <= last) nv_a[aa] += sCnt[nw + aa];
-      }
-      __syncthreads();
+      if (v0 + span < NV) __syncthreads();   // the next sweep overwrites the counts
     }
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      if (seed_at[k] >= 0) put_seed(seed_at[k], seed_v[k]);
+    for (int x = tid + 2 * NT; x < md.nseed; x += NT) put_seed(__ldg(md.seed_idx + x), __ldg(md.seed_val + x));
+    // rows end at a whole 16-byte word: the slots past the last neighbour
+    // count nothing (f = 0, finite powers)
+    for (int x = tid; x < A * L.rows * VW; x += NT) {
+      const int k = x % VW, a = x / (L.rows * VW), r = x / VW % L.rows;
+      int nv = 0;
+#pragma unroll
+      for (int aa = 0; aa < A; ++aa)
+        if (aa == a) nv = nv_a[aa];
+      if (k >= nv % VW && nv % VW) sSt[(static_cast<size_t>(a) * L.rows + r) * qs + nv / VW * VW + k] = T(0);
+    }
+    __syncthreads();
     // ---- N2: basic moments m[(mu, a, b, c)] of every atom of the block ------
     // tasks (atom, monomial), most radial functions first: monomials are
     // sorted by degree (descending), so monomial P-1-j has the j-th most.  A
     // warp takes 32 consecutive monomials of one atom (one radial-function
     // count and one neighbour list per warp; the warp's largest count is
-    // used), warp slots go round-robin over the atoms, and odd rounds run the
-    // slots in reverse (snake), so each thread's rounds add up to about the
-    // same cost and the last, partial round gets the cheapest monomials.
+    // used), warp slots go round-robin over the atoms, and the rounds after
+    // the first run the slots in reverse, so each warp's rounds add up to
+    // about the same cost and the last, partial round goes to the warps that
+    // have the least.
     const int P32 = (P + 31) & ~31;
     for (int t0 = 0; t0 < A * P32; t0 += NT) {
-      const int pos = t0 + (((t0 / NT) & 1) ? NT - 1 - tid : tid);
+      const int pos = t0 + (t0 ? NT - 1 - tid : tid);
       const int blk = pos >> 5, j = (blk / A) * 32 + (pos & 31);
       const bool act = pos < A * P32 && j < P;
       const int a = act ? blk % A : 0, p = act ? P - 1 - j : 0;
-      const int4 abc = __ldg(reinterpret_cast<const int4*>(md.mono_abc) + p);
+      const int word = sMono[p];   // exponents, radial functions, first entry of sList
       int nv = 0;
 #pragma unroll
       for (int aa = 0; aa < A; ++aa)
         if (act && aa == a) nv = nv_a[aa];
-      const int nm = __reduce_max_sync(0xffffffffu, act ? md.nmu[abc.w] : 0);
-      const T* sF = reinterpret_cast<const T*>(smem + L.f) + static_cast<size_t>(a) * L.rs * n_pad;
-      const T* sPw = reinterpret_cast<const T*>(smem + L.pw) + static_cast<size_t>(a) * pws * n_pad;
+      const int nm = __reduce_max_sync(0xffffffffu, act ? word >> 12 & 15 : 0);
+      const T* f = sSt + static_cast<size_t>(a) * L.rows * qs;
+      const T* px = f + (2 * R + 1 + (word & 15)) * qs;
+      const T* py = f + (2 * R + 1 + D1 + (word >> 4 & 15)) * qs;
+      const T* pz = f + (2 * R + 1 + 2 * D1 + (word >> 8 & 15)) * qs;
       T acc[kMaxR];
 #pragma unroll
       for (int mu = 0; mu < kMaxR; ++mu) acc[mu] = T(0);
       switch (nm) {
         case 0: break;
-        case 1: moment_task<T, 1>(sF, sPw, L.rs, pws, D1, nv, abc.x, abc.y, abc.z, acc); break;
-        case 2: moment_task<T, 2>(sF, sPw, L.rs, pws, D1, nv, abc.x, abc.y, abc.z, acc); break;
-        case 3: moment_task<T, 3>(sF, sPw, L.rs, pws, D1, nv, abc.x, abc.y, abc.z, acc); break;
-        case 4: moment_task<T, 4>(sF, sPw, L.rs, pws, D1, nv, abc.x, abc.y, abc.z, acc); break;
-        case 5: moment_task<T, 5>(sF, sPw, L.rs, pws, D1, nv, abc.x, abc.y, abc.z, acc); break;
-        case 6: moment_task<T, 6>(sF, sPw, L.rs, pws, D1, nv, abc.x, abc.y, abc.z, acc); break;
-        case 7: moment_task<T, 7>(sF, sPw, L.rs, pws, D1, nv, abc.x, abc.y, abc.z, acc); break;
-        default: moment_task<T, 8>(sF, sPw, L.rs, pws, D1, nv, abc.x, abc.y, abc.z, acc); break;
+#define MTP_MOMENTS(NM) \
+  case NM: moment_task<NM>(f, qs, px, py, pz, nv, acc); break;
+        MTP_MOMENTS(1) MTP_MOMENTS(2) MTP_MOMENTS(3) MTP_MOMENTS(4) MTP_MOMENTS(5) MTP_MOMENTS(6) MTP_MOMENTS(7)
+        default: moment_task<8>(f, qs, px, py, pz, nv, acc); break;
+#undef MTP_MOMENTS
       }
       if (act) {
+        const uint16_t* k = sList + (static_cast<unsigned>(word) >> 16);
 #pragma unroll
-        for (int mu = 0; mu < kMaxR; ++mu) {
-          if (mu < nm) {
-            const int k = __ldg(md.mono_k + kMaxR * p + mu);
-            if (k >= 0) V[(md.v_m + k) * A + a] = acc[mu];
-          }
-        }
+        for (int mu = 0; mu < kMaxR; ++mu)
+          if (mu < (word >> 12 & 15) && k[mu] != 0xFFFFu) V[(md.v_m + k[mu]) * A + a] = acc[mu];
       }
     }
-    // adjoint seeds
-    for (int x = tid; x < md.M * A; x += NT) V[md.v_dm * A + x] = T(0);
-    __syncthreads();
-    for (int x = tid; x < md.nseed * A; x += NT)
-      V[(md.v_dm + md.seed_idx[x / A]) * A + x % A] = static_cast<T>(md.seed_val[x / A]);
 
-    // ---- T: forward contraction passes ----------------------------------
-    for (int ps = 0; ps < md.nfwd; ++ps) {
-      run_pass_n<T, A, true>(md.entries + md.fwd[ps].offset, __shfl_sync(0xFFFFFFFFu, my_wsteps, ps), NT, tid,
-                                 V);
-      __syncthreads();
-    }
-    // energy: E_i = xi[t_i] + sum_alpha theta_alpha m[map_alpha] in FP64
-    {
-      double ep[A];
-#pragma unroll
-      for (int a = 0; a < A; ++a) ep[a] = 0.0;
-      for (int al = tid; al < md.Sa; al += NT) {
-        const double th = __ldg(md.theta + al);
-        const int k = md.v_m + __ldg(md.mapping + al);
-#pragma unroll
-        for (int a = 0; a < A; ++a) ep[a] = fma(th, static_cast<double>(V[k * A + a]), ep[a]);
-      }
-      // warp sums now; the block sum waits for the reverse passes' barriers
-      // (no barrier of its own on the critical path)
-      warp_partials<A>(ep, sRed);
-    }
-
-    // ---- R: reverse passes (dE/dm) ---------------------------------------
-    for (int ps = 0; ps < md.nrev; ++ps) {
-      run_pass_n<T, A, true>(md.entries + md.rev[ps].offset,
-                                 __shfl_sync(0xFFFFFFFFu, my_wsteps, md.nfwd + ps), NT, tid, V);
-      __syncthreads();
-    }
+    // ---- T, R: contraction passes and their reverse -----------------------
+    if (NT == 512) run_tree<T, A, 512>(md, V, sRed, my_wsteps, tid);
+    else if (NT == 256) run_tree<T, A, 256>(md, V, sRed, my_wsteps, tid);
+    else run_tree<T, A, 128>(md, V, sRed, my_wsteps, tid);
 
     // site energies: thread a adds atom a's warp sums in warp order
-    if (md.nrev == 0) __syncthreads();
-#pragma unroll
-    for (int a = 0; a < A; ++a) {
-      if (tid == a && base + a < io.natoms) {
-        double ep = 0.0;
-        for (int i = 0; i < (NT >> 5); ++i) ep += sRed[a * (NT >> 5) + i];
-        const double e = __ldg(md.species + it_a[a]) + ep;
-        io.site_energy[base + a] = e;
-        if (!isfinite(e)) atomicOr(io.err, kErrNonFinite);
-      }
+    if (tid < A && base + tid < io.natoms) {
+      double ep = 0.0;
+      for (int i = 0; i < (NT >> 5); ++i) ep += sRed[tid * (NT >> 5) + i];
+      const double e = __ldg(md.species + sType[tid]) + ep;
+      io.site_energy[base + tid] = e;
+      if (!isfinite(e)) atomicOr(io.err, kErrNonFinite);
     }
 
     // ---- N3: dE_i/dr_ij per kept neighbour -------------------------------
-    // level-structured bases read the basic moments' adjoints in place (chain
-    // order); otherwise a dense table Dm[a][slot][mu] = dE/dm of basic moment
-    // (mu, slot) over the full monomial simplex in pair order (0 where the
-    // basis has no moment) is filled first
-    if (md.tri) {
-      T* P = L.n3p_in_v ? V + static_cast<size_t>(md.v_m) * A : reinterpret_cast<T*>(smem + L.n3p);
+    // adjoints of the basic moments, each atom's in chain order
+    for (int x = tid; x < md.n3_len; x += NT) {
+      const int k = md.chain_mode >= 0 ? x : __ldg(md.n3_src + x);   // structured: placed in chain order
+      Pack<T, A> p;
+      if (k >= 0) {
+        p = *reinterpret_cast<const Pack<T, A>*>(V + (md.v_dm + k) * A);
+      } else {
+#pragma unroll
+        for (int a = 0; a < A; ++a) p.v[a] = T(0);
+      }
+      typename Force<T>::P* o = reinterpret_cast<typename Force<T>::P*>(smem + L.dmc) + x;
+#pragma unroll
+      for (int a = 0; a < A; ++a) o[a * L.n3s] = Force<T>::make(p.v[a], p.v[a]);
+    }
+    ahead = load_slot(base + gridDim.x * A, 0);
+    __syncthreads();
+#define MTP_FORCES(RR, MODE) \
+  case RR: force_phase<T, A, RR, MODE>(md, io, L, smem, nv_a, base, tid, NT); break;
+    if (md.chain_mode == 0) {
       switch (R) {
-#define MTP_N3T_CASE(RR) \
-  case RR: n3_transposed<T, A, RR>(md, io, L, smem, V, nv_a, base, tid, NT, P); break;
-        MTP_N3T_CASE(1) MTP_N3T_CASE(2) MTP_N3T_CASE(3) MTP_N3T_CASE(4)
-        MTP_N3T_CASE(5) MTP_N3T_CASE(6) MTP_N3T_CASE(7) MTP_N3T_CASE(8)
-#undef MTP_N3T_CASE
+        MTP_FORCES(1, 0) MTP_FORCES(2, 0) MTP_FORCES(3, 0) MTP_FORCES(4, 0)
+        MTP_FORCES(5, 0) MTP_FORCES(6, 0) MTP_FORCES(7, 0) MTP_FORCES(8, 0)
         default: break;
       }
-      __syncthreads();
-      continue;
-    }
-    T* sDm = L.dmt_in_v ? V + md.v_m * A : reinterpret_cast<T*>(smem + L.dmt);
-    const int QR = md.Q * R;
-    for (int x = tid; x < QR * A; x += NT) {
-      const int a = x / QR, r = x - a * QR;
-      const int k = __ldg(md.dense_k + (r / R) * kMaxR + r % R);
-      sDm[x] = k >= 0 ? V[(md.v_dm + __ldg(md.dm_pos + k)) * A + a] : T(0);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int a = 0; a < A; ++a) {
-      const int atom = base + a;
-      const int nv = nv_a[a];
-      const T* sU = reinterpret_cast<T*>(smem + L.u) + static_cast<size_t>(a) * 4 * n_pad;
-      const T* sF = reinterpret_cast<T*>(smem + L.f) + static_cast<size_t>(a) * L.rs * n_pad;
-      const T* sFp = reinterpret_cast<T*>(smem + L.fp) + static_cast<size_t>(a) * L.rs * n_pad;
-      const T* sPw = reinterpret_cast<T*>(smem + L.pw) + static_cast<size_t>(a) * pws * n_pad;
-      const int* sSlot = reinterpret_cast<int*>(smem + L.slot) + a * n_pad;
-      double* grow = io.pair_grad + static_cast<size_t>(atom < io.natoms ? atom : 0) * io.nbr_stride * 3;
-      // FP32: threads take pairs of neighbours (q, q + nt), which share every
-      // table-row load; FP64: one neighbour per thread (the second
-      // neighbour's registers would spill at the 128-register budget)
-      constexpr bool kTwoN = sizeof(T) == 4;
-      const int nt = kTwoN ? (nv + 1) >> 1 : nv;
-      int tpn = 32;
-      while (tpn > 1 && tpn * nt > NT) tpn >>= 1;
-      const int total = nt * tpn;
-      for (int b0 = 0; b0 < total; b0 += NT) {
-        const int idx = b0 + tid;
-        const bool active = idx < total;
-        const int q0 = active ? idx / tpn : 0;
-        const int q1 = q0 + nt;
-        const bool two = kTwoN && active && q1 < nv;
-        const int sl = idx & (tpn - 1);
-        T Ssum[2] = {T(0), T(0)}, Gx[2] = {T(0), T(0)}, Gy[2] = {T(0), T(0)}, Gz[2] = {T(0), T(0)};
-        if (active) {
-          const T* dmt = sDm + static_cast<size_t>(a) * QR;
-          const int qb = two ? q1 : q0;
-          switch (R) {
-#define MTP_N3_CASE(RR)                                                                                        \
-  case RR:                                                                                                     \
-    n3_sums<T, RR, kTwoN>(dmt, md.D, md.npairs, D1, sF + q0 * L.rs, sFp + q0 * L.rs, sF + qb * L.rs, \
-                                   sFp + qb * L.rs, two, sPw + q0 * pws, sPw + qb * pws, sU[4 * q0 + 2],         \
-                                   sU[4 * qb + 2], sl, tpn, Ssum, Gx, Gy, Gz);                                \
-    break;
-            MTP_N3_CASE(1) MTP_N3_CASE(2) MTP_N3_CASE(3) MTP_N3_CASE(4)
-            MTP_N3_CASE(5) MTP_N3_CASE(6) MTP_N3_CASE(7) MTP_N3_CASE(8)
-#undef MTP_N3_CASE
-            default: break;
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          for (int o = tpn >> 1; o > 0; o >>= 1) {
-            Ssum[j] += __shfl_xor_sync(0xffffffffu, Ssum[j], o);
-            Gx[j] += __shfl_xor_sync(0xffffffffu, Gx[j], o);
-            Gy[j] += __shfl_xor_sync(0xffffffffu, Gy[j], o);
-            Gz[j] += __shfl_xor_sync(0xffffffffu, Gz[j], o);
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const int q = j ? q1 : q0;
-          if (active && sl == 0 && (j == 0 || two)) {
-            const T ux = sU[4 * q], uy = sU[4 * q + 1], uz = sU[4 * q + 2], d = sU[4 * q + 3];
-            const T ug = ux * Gx[j] + uy * Gy[j] + uz * Gz[j];
-            const T inv_d = T(1) / d;
-            const T gx = ux * Ssum[j] + (Gx[j] - ux * ug) * inv_d;
-            const T gy = uy * Ssum[j] + (Gy[j] - uy * ug) * inv_d;
-            const T gz = uz * Ssum[j] + (Gz[j] - uz * ug) * inv_d;
-            const int s = sSlot[q];
-            grow[3 * s] = static_cast<double>(gx);
-            grow[3 * s + 1] = static_cast<double>(gy);
-            grow[3 * s + 2] = static_cast<double>(gz);
-            if (!(isfinite(static_cast<double>(gx)) && isfinite(static_cast<double>(gy)) &&
-                  isfinite(static_cast<double>(gz))))
-              atomicOr(io.err, kErrNonFinite);
-          }
-        }
+    } else if (md.chain_mode == 1) {
+      force_phase<T, A, 6, 1>(md, io, L, smem, nv_a, base, tid, NT);
+    } else if (md.chain_mode == 2) {
+      force_phase<T, A, 6, 2>(md, io, L, smem, nv_a, base, tid, NT);
+    } else {
+      switch (R) {
+        MTP_FORCES(1, -1) MTP_FORCES(2, -1) MTP_FORCES(3, -1) MTP_FORCES(4, -1)
+        MTP_FORCES(5, -1) MTP_FORCES(6, -1) MTP_FORCES(7, -1) MTP_FORCES(8, -1)
+        default: break;
       }
     }
+#undef MTP_FORCES
     __syncthreads();
   }
 }

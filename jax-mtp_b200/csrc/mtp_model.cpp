@@ -422,11 +422,11 @@ void emit_jobs(const std::vector<Job>& jobs, int lanes, int width, bool allow_sw
 
 }  // namespace
 
-bool adjoint_layout(const Potential& pot, std::vector<int>& dm_pos) {
+int adjoint_layout(const Potential& pot, std::vector<int>& dm_pos) {
   const int M = pot.M, B = pot.B;
   dm_pos.resize(M);
   for (int k = 0; k < M; ++k) dm_pos[k] = k;
-  if (B == 0) return false;
+  if (B == 0) return -1;
   int D = 0;
   std::map<std::array<int, 4>, int> basic_of;
   for (int k = 0; k < B; ++k) {
@@ -434,23 +434,28 @@ bool adjoint_layout(const Potential& pot, std::vector<int>& dm_pos) {
     D = std::max(D, r[1] + r[2] + r[3]);
     basic_of[{r[0], r[1], r[2], r[3]}] = k;
   }
-  std::vector<int> pos(B, -1);
-  int next = 0;
-  for (int sum = 0; sum <= D; ++sum) {
-    for (int a = 0; a <= sum; ++a) {
-      const int b = sum - a, top = D - sum;
-      for (int k = 0; k <= top; ++k) {
-        for (int mu = 0; mu <= k / 2; ++mu) {
-          auto it = basic_of.find({mu, a, b, top - k});
-          if (it == basic_of.end()) return false;   // a hole: not level-structured
-          pos[it->second] = next++;
-        }
+  for (int mode = 0; mode <= 2; ++mode) {
+    if (mode > 0 && pot.R != 6) break;   // the force phase has these offsets for six radial functions
+    std::vector<int> pos(B, -1);
+    int next = 0, found = 0;
+    bool ok = true;
+    for (int b = 0; b <= D && ok; ++b)
+      for (int a = D - b; a >= 0 && ok; --a) {
+        const int top = D - a - b;
+        for (int k = 0; k <= top && ok; ++k)
+          for (int mu = 0; mu < std::min(pot.R, (k + mode) / 2 + 1) && ok; ++mu) {
+            auto it = basic_of.find({mu, a, b, top - k});
+            if (it == basic_of.end()) ok = false;   // a hole: another structure
+            else pos[it->second] = next++, ++found;
+          }
+        next = (next + 3) & ~3;
       }
-    }
+    if (!ok || found != B) continue;               // found < B: basic moments outside the pattern
+    for (int k = 0; k < B; ++k) dm_pos[k] = pos[k];
+    for (int k = B; k < M; ++k) dm_pos[k] = next + k - B;
+    return mode;
   }
-  if (next != B) return false;                      // basic moments outside the pattern
-  for (int k = 0; k < B; ++k) dm_pos[k] = pos[k];
-  return true;
+  return -1;
 }
 
 void seed_list(const Potential& pot, std::vector<int>& idx, std::vector<double>& val) {
@@ -493,9 +498,10 @@ bool build_schedule(const Potential& pot, int lanes, Schedule& s, std::string& e
   s.max_depth = maxd;
 
   // value-space layout (partials resolved at the end)
+  s.chain_mode = adjoint_layout(pot, s.dm_pos);
   s.v_m = 0;
   s.v_dm = M;
-  s.v_part = 2 * M;
+  s.v_part = M + (M ? 1 + *std::max_element(s.dm_pos.begin(), s.dm_pos.end()) : 0);
 
   // monomials
   std::map<std::tuple<int, int, int>, int> mono_of;
@@ -540,66 +546,48 @@ bool build_schedule(const Potential& pot, int lanes, Schedule& s, std::string& e
     const int v = pot.basic[4 * k + 1] + pot.basic[4 * k + 2] + pot.basic[4 * k + 3];
     s.nmu[v] = std::max(s.nmu[v], pot.basic[4 * k] + 1);
   }
-  // dense simplex in pair order
-  s.npairs = (s.D + 1) * (s.D + 2) / 2;
-  s.Q = (s.D + 1) * (s.D + 2) * (s.D + 3) / 6;
-  s.dense_k.assign(static_cast<size_t>(s.Q) * kMaxR, -1);
-  {
-    int slot = 0;
-    for (int sum = 0; sum <= s.D; ++sum) {
-      for (int a = 0; a <= sum; ++a) {
-        const int b = sum - a;
-        for (int c = 0; c <= s.D - sum; ++c, ++slot) {
-          auto it = mono_of.find(std::make_tuple(a, b, c));
-          if (it == mono_of.end()) continue;
-          for (int mu = 0; mu < kMaxR; ++mu)
-            s.dense_k[static_cast<size_t>(slot) * kMaxR + mu] = s.mono_k[kMaxR * it->second + mu];
+  for (int p = 0; p < s.P; ++p) {
+    int n = 0;
+    for (int mu = 0; mu < kMaxR; ++mu)
+      if (s.mono_k[kMaxR * p + mu] >= 0) n = mu + 1;
+    const int* e = &s.mono_abc[4 * p];
+    s.mono_word.push_back(e[0] | (e[1] << 4) | (e[2] << 8) | (n << 12) | (static_cast<int>(s.mono_list.size()) << 16));
+    for (int mu = 0; mu < n; ++mu) s.mono_list.push_back(s.mono_k[kMaxR * p + mu] < 0 ? 0xFFFF : s.mono_k[kMaxR * p + mu]);
+  }
+  // force-phase chains
+  struct Chain { int word, cost; };
+  std::vector<Chain> chains;
+  for (int b = 0; b <= s.D; ++b)
+    for (int a = s.D - b; a >= 0; --a) {
+      const int top = s.D - a - b, first = static_cast<int>(s.n3_src.size());
+      for (int k = 0; k <= top; ++k) {
+        const auto it = mono_of.find(std::make_tuple(a, b, top - k));
+        const int nm = s.chain_mode < 0 ? pot.R : std::min(pot.R, (k + s.chain_mode) / 2 + 1);
+        for (int mu = 0; mu < nm; ++mu) {
+          const int m = it == mono_of.end() ? -1 : s.mono_k[kMaxR * it->second + mu];
+          s.n3_src.push_back(m < 0 ? -1 : s.dm_pos[m]);
         }
       }
+      const int n = static_cast<int>(s.n3_src.size()) - first;
+      while (s.n3_src.size() % 4) s.n3_src.push_back(-1);
+      // multiply-adds of the terms and Horner steps, 16-byte loads, the rest of a pair
+      chains.push_back({top | (a << 4) | (b << 8) | ((first / 4) << 16), 2 * n + 3 * (top + 1) + n / 4 + 12});
     }
+  s.n3_len = static_cast<int>(s.n3_src.size());
+  long all = 0;
+  for (const Chain& c : chains) {
+    s.n3_words.push_back(c.word);
+    all += c.cost;
   }
-  s.tri = adjoint_layout(pot, s.dm_pos);
-  if (s.tri) {
-    // pairs (a, b) in pair order with their chain base; longest chain first
-    // onto the least loaded warp (cost ~ adjoint loads and multiply-adds of the
-    // chain's steps plus its Horner steps and tail)
-    struct P3 { int word, cost; };
-    std::vector<P3> pairs;
-    int base = 0;
-    for (int sum = 0; sum <= s.D; ++sum)
-      for (int a = 0; a <= sum; ++a) {
-        const int b = sum - a, top = s.D - sum;
-        int cost = 10;
-        for (int k = 0; k <= top; ++k) cost += 3 * (k / 2 + 1) + 3;
-        pairs.push_back({a | (b << 4) | (top << 8) | (base << 12), cost});
-        base += ((top + 2) * (top + 2)) / 4;
-      }
-    std::vector<int> order(pairs.size());
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return pairs[x].cost > pairs[y].cost; });
-    // one list per group width (kN3GroupWarps: the FP32 kernel; half of it:
-    // the FP64 kernel)
-    for (int gi = 0; gi < 2; ++gi) {
-      const int warps = std::min(lanes / 32, gi == 0 ? kN3GroupWarps : kN3GroupWarps / 2);
-      std::vector<std::vector<int>> wl(warps);
-      std::vector<long> load(warps, 0);
-      for (int i : order) {
-        int w = 0;
-        for (int v = 1; v < warps; ++v)
-          if (load[v] < load[w] || (load[v] == load[w] && wl[v].size() < wl[w].size())) w = v;
-        wl[w].push_back(pairs[i].word);
-        load[w] += pairs[i].cost;
-      }
-      std::vector<int>& np = gi == 0 ? s.n3_pairs : s.n3_pairs_half;
-      std::vector<int>& no = gi == 0 ? s.n3_off : s.n3_off_half;
-      no.assign(1, 0);
-      for (int w = 0; w < warps; ++w) {
-        if (wl[w].size() > 32) s.tri = false;    // one pair per lane at most
-        np.insert(np.end(), wl[w].begin(), wl[w].end());
-        no.push_back(static_cast<int>(np.size()));
-      }
+  for (int W = 1; W <= kMaxGroupWarps; W *= 2) {
+    size_t i = 0;
+    long done = 0;
+    for (int w = 0; w < W; ++w) {
+      s.n3_off.push_back(static_cast<int>(i));
+      // up to the chain whose middle passes this run's share
+      while (i < chains.size() && (w + 1 == W || 2 * done + chains[i].cost <= 2 * all * (w + 1) / W)) done += chains[i++].cost;
     }
-    if (base >= (1 << 20) || s.D > 15) s.tri = false;
+    s.n3_off.push_back(static_cast<int>(chains.size()));
   }
   // moments that are read but never written stay zero for the whole run
   std::vector<char> read(M, 0);
@@ -669,7 +657,10 @@ bool build_schedule(const Potential& pot, int lanes, Schedule& s, std::string& e
       }
     }
     emit_jobs(jobs, lanes, width, false, rev, parts);
+    for (const auto& kv : job_of) written[kv.first] = 1;
   }
+  for (int k = 0; k < M; ++k)
+    if (!seeded[k] && !written[k]) s.dm_zero.push_back(s.dm_pos[k]);
   s.n_part = parts;
   s.v_zero = s.v_part + parts;
   s.v_one = s.v_zero + 1;
@@ -889,7 +880,7 @@ double emulate_schedule(const Potential& pot, const Schedule& s, std::vector<dou
   for (const Pass& p : s.fwd) run(p);
   double e = 0.0;
   for (int a = 0; a < pot.Sa; ++a) e += pot.moment[a] * V[s.v_m + pot.mapping[a]];
-  for (int k = 0; k < pot.M; ++k) V[s.v_dm + k] = 0.0;
+  for (int k = s.v_dm; k < s.v_part; ++k) V[k] = 0.0;
   std::vector<int> si;
   std::vector<double> sv;
   seed_list(pot, si, sv);

@@ -35,8 +35,10 @@ constexpr int kMaxR = 8;       // radial functions supported by the kernels
 constexpr int kMaxK = 16;      // Chebyshev terms supported by the kernels
 constexpr int kMaxDegree = 12; // monomial degree supported by the kernels
 constexpr int kMaxPasses = 16;
-constexpr int kStepAlign = 4;
-constexpr int kN3GroupWarps = 8;  // warps that share one neighbour chunk in the FP32 force phase (half in FP64)   // pass steps are a multiple of this; as many no-op rows end the program
+constexpr int kStepAlign = 4;  // pass steps are a multiple of this; as many no-op rows end the program
+constexpr int kMaxGroupWarps = 16;  // warps of the largest block, which the force phase may group on one neighbour chunk
+constexpr int kMaxChains = (kMaxDegree + 1) * (kMaxDegree + 2) / 2;
+constexpr int kMaxRunOffsets = 36;  // 2 + 3 + 5 + 9 + 17: offsets of the cuts into 1, 2, 4, 8 and 16 runs
 
 struct Potential {
   std::string version, potential_name, potential_tag, radial_basis_type;
@@ -74,7 +76,7 @@ struct Schedule {
   int width = 4;          // bytes per operand access the entry order was tuned for
   // Value-space layout (indices into the per-atom value array V):
   int v_m = 0;            // moments m[0..M)
-  int v_dm = 0;           // adjoints dE/dm[0..M)
+  int v_dm = 0;           // adjoints dE/dm (dm_pos)
   int v_part = 0;         // partial sums of split lists
   int n_part = 0;
   int v_zero = 0;         // constant 0
@@ -86,28 +88,29 @@ struct Schedule {
   std::vector<int> mono_abc;    // [P][4] (a, b, c, degree), degree descending
   std::vector<int> nmu;         // [D + 1] radial functions with a basic moment of each degree
   std::vector<int> mono_k;      // [P][kMaxR] basic-moment index for each mu or -1
-  // The full monomial simplex a + b + c <= D in "pair order": pairs (a, b)
-  // by s = a + b ascending, then a ascending; each pair owns the run of
-  // slots c = 0 .. D - s.  Used by the force phase (nested Horner in z, y).
-  int Q = 0;                    // (D+1)(D+2)(D+3)/6 slots
-  int npairs = 0;               // (D+1)(D+2)/2 pairs
-  std::vector<int> dense_k;     // [Q][kMaxR] basic-moment index of slot and mu, or -1
-  // Level-structured basis (adjoint_layout): radial function mu meets exactly
-  // the monomials of degree <= D - 2 mu.  Then a force-phase Horner step
-  // k = D - degree has the radial functions mu <= k / 2, and the adjoints of
-  // the basic moments are laid out in that chain order (dm_pos), so the force
-  // phase reads them in place.
-  bool tri = false;
-  // dE/dm of moment k lives at v_dm + dm_pos[k] (a permutation of [0, M))
+  // the same for the evaluation kernel: a | b << 4 | c << 8 | n << 12 |
+  // (first of n entries in mono_list) << 16 with n = 1 + the monomial's
+  // largest mu; mono_list holds basic-moment indices, 0xFFFF for none
+  std::vector<int> mono_word, mono_list;
+  // Force phase: the monomials are taken as Horner chains in u_z, one per pair
+  // (a, b) with a + b <= D, b ascending and a descending; step k = 0 .. top =
+  // D - a - b of a chain holds the monomial u_x^a u_y^b u_z^(top - k).
+  // chain_mode >= 0: a level-structured basis (adjoint_layout) whose step k has
+  // the radial functions mu < min(R, (k + chain_mode) / 2 + 1); -1: every step
+  // has all R (adjoint 0 where the basis has no moment).  Chain slots are
+  // steps in order, radial functions within a step, each chain padded to a
+  // multiple of four; n3_src[slot] is the adjoint position it copies, or -1.
+  int chain_mode = -1;
+  int n3_len = 0;
+  std::vector<int> n3_src;      // [n3_len]
+  // dE/dm of moment k lives at v_dm + dm_pos[k]; the adjoint region ends at v_part
   std::vector<int> dm_pos;
-  // Force phase on level-structured bases: the block's warps form groups of
-  // min(lanes / 32, kN3GroupWarps) (FP32 kernel; n3_*_half: of half that,
-  // FP64 kernel) that take neighbour chunks in turn, and warp w of a group
-  // takes the monomial pairs n3_pairs[n3_off[w] .. n3_off[w + 1]) (at most
-  // 32, balanced by chain cost), each one word a | b << 4 | top << 8 |
-  // chain base << 12 (top = D - a - b; chain base = the pair's first
-  // adjoint position).
-  std::vector<int> n3_pairs, n3_off, n3_pairs_half, n3_off_half;
+  // One word per chain, top | a << 4 | b << 8 | (first slot / 4) << 16, and the
+  // list cut into W = 1, 2, 4, 8 and 16 runs of about equal cost (one per warp
+  // of a group): run w of W is n3_words[n3_off[o + w] .. n3_off[o + w + 1])
+  // with o = W - 1 + log2 W.
+  std::vector<int> n3_words, n3_off;
+  std::vector<int> dm_zero;     // adjoint positions that no pass stores and no seed sets (must read as 0)
   std::vector<int> zero_list;   // non-basic moments never written (must read as 0)
   std::vector<Pass> fwd, rev;   // passes in execution order
   std::vector<uint32_t> entries;  // pairs (x, y) per entry: 2 words; kStepAlign no-op rows at the end
@@ -135,17 +138,16 @@ void refine_schedule(Schedule& s);
 // coefficients), and returns sum_alpha theta_alpha m[map_alpha].
 double emulate_schedule(const Potential& pot, const Schedule& s, std::vector<double>& V);
 
-// Position of every moment's adjoint within the adjoint region (dm_pos, a
-// permutation of [0, M)); returns whether the basis is level-structured:
-// every basic moment (mu, a, b, c) has 2 mu <= D - (a + b + c) and every such
-// (mu, monomial) is a basic moment.  Then the basic moments' adjoints take
-// positions [0, B) in force-phase chain order: monomial pairs (a, b) by
-// a + b, then a; within a pair k = D - a - b - c = 0 .. D - a - b, and within
-// a step mu = 0 .. k / 2, so step k of a pair starts floor((k + 1)^2 / 4)
-// after the pair's first position and a pair of s = a + b holds
-// floor((D - s + 2)^2 / 4).  Otherwise (and for every non-basic moment)
-// dm_pos[k] = k.
-bool adjoint_layout(const Potential& pot, std::vector<int>& dm_pos);
+// Position of every moment's adjoint within the adjoint region (dm_pos,
+// distinct); returns Schedule::chain_mode: o >= 0 if the basis is
+// level-structured with that offset, that is, its basic moments (mu, a, b, c)
+// are those with a + b + c <= D and mu < min(R, (D - a - b - c + o) / 2 + 1)
+// (the MLIP templates up to level 24: o = 0; 26 and 28: o = 1 and 2, with six
+// radial functions), else -1.  On such a basis the basic moments' adjoints
+// take their force-phase chain slots as positions (each chain padded to a
+// multiple of four) and the others follow, so the copy into chain slots is a
+// copy in a row; otherwise dm_pos[k] = k.
+int adjoint_layout(const Potential& pot, std::vector<int>& dm_pos);
 
 // Seeds of the reverse pass: unique moments of the mapping with summed theta.
 void seed_list(const Potential& pot, std::vector<int>& idx, std::vector<double>& val);

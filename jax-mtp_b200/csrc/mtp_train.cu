@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
         }
       }
     }
-    for (int x = tid; x < md.M; x += NT) V[md.v_dm + x] = Dual2<T>::make(T(0), T(0));
+    for (int x = tid; x < md.n_dm; x += NT) V[md.v_dm + x] = Dual2<T>::make(T(0), T(0));
     __syncthreads();
     for (int x = tid; x < md.nseed; x += NT) {
       const T sv = static_cast<T>(md.seed_val[x]);
