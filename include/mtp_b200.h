@@ -239,10 +239,11 @@ int mtp_adjoint_batch_device(mtp_handle* h, int natoms, int nbr_stride, int ncon
                              const double* d_gS, double* d_gspecies, double* d_gmoment,
                              double* d_gradial);
 
-/* Launch shape of the evaluation kernel: threads per block (128/256/512),
- * blocks per SM (0 = as many as fit) and atoms evaluated together per block
- * (0 = chosen by occupancy, or 1/2/4; FP64 supports 1/2).  Used by the
- * autotuner. */
+/* Launch shape of the evaluation kernel: at most this many threads per block
+ * (128/256/512), blocks per SM (0 = as many as fit) and atoms evaluated
+ * together per block (0 = any, or 1/2/4; FP64 supports 1/2).  Among the shapes
+ * allowed, each call takes the one expected to be fastest for its number of
+ * atoms; until this is called, all are.  Used by the autotuner. */
 int mtp_set_launch(mtp_handle* h, int threads_per_block, int blocks_per_sm, int atoms_per_block);
 
 /* Last evaluation kernel's launch: out5 = threads, blocks, dynamic shared bytes,

@@ -70,13 +70,14 @@ struct mtp_handle {
   double cutoff = 0.0;
   int device = 0, sm_count = 0;
   cudaStream_t own_stream = nullptr, stream = nullptr;
-  int threads = 256, blocks_per_sm = 0;
+  int threads = 0, blocks_per_sm = 0;   // requested launch (mtp_set_launch); 0 threads: automatic
   int last_threads = 0, last_blocks = 0, last_bps = 0;
   bool last_vglobal = false;
   void* d_vscratch = nullptr;
   size_t vscratch_bytes = 0;
   size_t last_smem = 0;
   std::map<int, DeviceSchedule> scheds;
+  std::map<int, DeviceSchedule> sizes;   // by lanes: schedules without programs, to size launches
   // potential tables on the device
   double *d_radial = nullptr, *d_species = nullptr, *d_theta = nullptr, *d_seed_val = nullptr;
   int *d_mapping = nullptr, *d_seed_idx = nullptr, *d_zero = nullptr, *d_abc = nullptr, *d_mk = nullptr;
@@ -97,12 +98,12 @@ struct mtp_handle {
   int* h_err = nullptr;      // pinned [1]
   TrainWorkspace train;
   CellScratch cells;
-  // launch decisions by (requested lanes, stride, precision): no occupancy
-  // queries after the first call, so later calls can be graph-captured
-  struct LaunchChoice { int lanes, bps; bool vglobal; size_t smem; int A; };
+  // blocks per SM of a (lanes, atoms per block, stride, precision, value-space
+  // placement): no occupancy queries after the first, so later calls can be
+  // graph-captured
   int apb = 0;          // requested atoms per block (0: chosen by occupancy)
   int last_apb = 1;
-  std::map<long long, LaunchChoice> launch_cache;
+  std::map<long long, int> occupancy;
   // profiling of the evaluation kernel
   bool profiling = false;
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> prof_events;
@@ -221,45 +222,63 @@ inline int access_width(bool fp64, int atoms_per_block) { return (fp64 ? 8 : 4) 
 // Dynamic shared memory one block of this part can opt in to.
 constexpr size_t kMaxSmemPerBlock = 227 * 1024;
 
-// Schedule for `lanes` threads and `width`-byte operand accesses, built on
-// first use.  With `upload` (every call that launches with it) its programs
-// also go to the device on first use, after refine_schedule where the value
-// space can sit in shared memory (bank order matters only there); a schedule
-// that is only sized (launch-shape candidates) is neither refined nor
-// uploaded, and no launch ever sees an unrefined copy of a refined one.
-int get_schedule(mtp_handle* h, int lanes, int width, DeviceSchedule** out, bool upload = true) {
+// Schedule without programs for `lanes` threads: what a launch needs to be sized.
+int get_sizes(mtp_handle* h, int lanes, const DeviceSchedule** out) {
+  auto it = h->sizes.find(lanes);
+  if (it == h->sizes.end()) {
+    DeviceSchedule ds;
+    std::string err;
+    if (!build_schedule(h->pot, lanes, ds.sched, err, 4, false)) return fail(h, MTP_E_FORMAT, err);
+    it = h->sizes.emplace(lanes, std::move(ds)).first;
+  }
+  *out = &it->second;
+  return MTP_OK;
+}
+
+bool schedule_uploaded(const mtp_handle* h, int lanes, int width) {
+  return h->scheds.count(lanes * 64 + width) > 0;
+}
+
+// Schedule for `lanes` threads and `width`-byte operand accesses, built and
+// uploaded on first use; refine_schedule runs where the value space can sit in
+// shared memory (bank order matters only there).
+int get_schedule(mtp_handle* h, int lanes, int width, const DeviceSchedule** out) {
   const int key = lanes * 64 + width;
   auto it = h->scheds.find(key);
   if (it == h->scheds.end()) {
     DeviceSchedule ds;
     std::string err;
     if (!build_schedule(h->pot, lanes, ds.sched, err, width)) return fail(h, MTP_E_FORMAT, err);
+    if (static_cast<size_t>(ds.sched.v_size) * width <= kMaxSmemPerBlock) refine_schedule(ds.sched);
     if (h->d_abc == nullptr) {
       const Schedule& t = ds.sched;
       const std::pair<int**, const std::vector<int>*> tables[] = {
           {&h->d_abc, &t.mono_abc}, {&h->d_mk, &t.mono_k},   {&h->d_dm_pos, &t.dm_pos},     {&h->d_zero, &t.zero_list},
-          {&h->d_dm_zero, &t.dm_zero}, {&h->d_n3_src, &t.n3_src}, {&h->d_mono_word, &t.mono_word}, {&h->d_mono_list, &t.mono_list}};
+          {&h->d_dm_zero, &t.dm_zero}, {&h->d_n3_src, &t.n3_src}, {&h->d_mono_word, &t.mono_word},
+          {&h->d_mono_list, &t.mono_list}};
       for (const auto& x : tables) {
         MTP_CUDA(h, dalloc(x.first, x.second->size()));
         if (!x.second->empty())
           MTP_CUDA(h, cudaMemcpy(*x.first, x.second->data(), x.second->size() * sizeof(int), cudaMemcpyHostToDevice));
       }
     }
-    it = h->scheds.emplace(key, ds).first;
-  }
-  DeviceSchedule& ds = it->second;
-  if (upload && ds.d_entries == nullptr) {
-    if (static_cast<size_t>(ds.sched.v_size) * width <= kMaxSmemPerBlock) refine_schedule(ds.sched);
     const auto& ent = ds.sched.entries;
-    MTP_CUDA(h, dalloc(&ds.d_entries, ent.size() / 2));
-    MTP_CUDA(h, cudaMemcpy(ds.d_entries, ent.data(), ent.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     std::vector<int> ws;
     for (const Pass& p : ds.sched.fwd) ws.insert(ws.end(), p.wsteps.begin(), p.wsteps.end());
     for (const Pass& p : ds.sched.rev) ws.insert(ws.end(), p.wsteps.begin(), p.wsteps.end());
-    MTP_CUDA(h, dalloc(&ds.d_warp_steps, ws.size()));
-    MTP_CUDA(h, cudaMemcpy(ds.d_warp_steps, ws.data(), ws.size() * sizeof(int), cudaMemcpyHostToDevice));
+    cudaError_t e = dalloc(&ds.d_entries, ent.size() / 2);
+    if (e == cudaSuccess)
+      e = cudaMemcpy(ds.d_entries, ent.data(), ent.size() * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = dalloc(&ds.d_warp_steps, ws.size());
+    if (e == cudaSuccess) e = cudaMemcpy(ds.d_warp_steps, ws.data(), ws.size() * sizeof(int), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+      cudaFree(ds.d_entries);
+      cudaFree(ds.d_warp_steps);
+      return cuda_fail(h, e, "upload schedule");
+    }
+    it = h->scheds.emplace(key, std::move(ds)).first;
   }
-  *out = &ds;
+  *out = &it->second;
   return MTP_OK;
 }
 
@@ -316,72 +335,87 @@ void free_handle(mtp_handle* h) {
   delete h;
 }
 
-// Launch shape for the evaluation kernel.  Candidates are (lanes, atoms per
-// block) with the value space in shared memory; the one with the most atoms
-// in flight per SM (A x blocks/SM) wins, ties going to more warps.  When none
-// fits, the value space moves to global memory (A = 1).  Decisions are cached
-// per (request, stride, precision), so later calls make no occupancy queries.
-int pick_launch(mtp_handle* h, int natoms, int stride, DeviceSchedule** ds_out, int* blocks_out, bool fp64,
-                bool* vglobal_out) {
-  const long long key = (static_cast<long long>(h->threads) << 40) | (static_cast<long long>(h->apb) << 36) |
-                        (static_cast<long long>(h->blocks_per_sm) << 28) | (static_cast<long long>(stride) << 2) |
-                        (fp64 ? 1 : 0);
-  auto hit = h->launch_cache.find(key);
-  mtp_handle::LaunchChoice c{};
-  if (hit != h->launch_cache.end()) {
-    c = hit->second;
-  } else {
-    std::vector<int> lanes_c = {h->threads};
-    for (int alt : {256, 128})
-      if (alt < h->threads) lanes_c.push_back(alt);
-    std::vector<int> a_c;
-    if (h->apb > 0) a_c = {h->apb};
-    else if (fp64) a_c = {2, 1};
-    else a_c = {4, 2, 1};
-    int best = -1;
-    for (int lanes : lanes_c) {
-      for (int A : a_c) {
-        if (!eval_variant_exists(fp64, false, A)) continue;
-        DeviceSchedule* ds = nullptr;
-        int st = get_schedule(h, lanes, access_width(fp64, A), &ds, false);
-        if (st != MTP_OK) return st;
-        const DevModel md = make_model(h, *ds);
-        int bps = eval_blocks_per_sm(md, stride, lanes, fp64, false, A);
-        if (h->blocks_per_sm > 0) bps = std::min(bps, h->blocks_per_sm);
-        if (bps <= 0) continue;
-        const int score = (A * bps) * 1024 + bps * lanes / 32;
-        if (score > best) {
-          best = score;
-          c = mtp_handle::LaunchChoice{lanes, bps, false, 0, A};
-        }
-      }
-    }
-    if (best < 0) {
-      // value space in global memory: 512 lanes give an SM 16 warps with one
-      // block, so the blocks' value spaces stay within L2
-      const int lanes = 512;
-      DeviceSchedule* ds = nullptr;
-      int st = get_schedule(h, lanes, access_width(fp64, 1), &ds, false);
-      if (st != MTP_OK) return st;
-      int bps = eval_blocks_per_sm(make_model(h, *ds), stride, lanes, fp64, true, 1);
-      if (h->blocks_per_sm > 0) bps = std::min(bps, h->blocks_per_sm);
-      if (bps <= 0)
-        return fail(h, MTP_E_CAPACITY, "the evaluation block does not fit in shared memory for this basis and max_nbr");
-      c = mtp_handle::LaunchChoice{lanes, std::min(bps, 1), true, 0, 1};
-    }
-    DeviceSchedule* ds = nullptr;
-    int st = get_schedule(h, c.lanes, access_width(fp64, c.A), &ds);
+// Blocks of one launch shape an SM holds (0: it does not fit), asked once.
+int launch_occupancy(mtp_handle* h, int lanes, int stride, bool fp64, bool vglobal, int A, int* bps) {
+  const long long key = (static_cast<long long>(stride) << 20) | (lanes << 4) | (A << 2) | (vglobal ? 2 : 0) | (fp64 ? 1 : 0);
+  auto it = h->occupancy.find(key);
+  if (it == h->occupancy.end()) {
+    const DeviceSchedule* ds = nullptr;
+    int st = get_sizes(h, lanes, &ds);
     if (st != MTP_OK) return st;
-    c.smem = eval_smem_bytes(make_model(h, *ds), stride, c.lanes, fp64, c.vglobal, c.A);
-    h->launch_cache[key] = c;
+    it = h->occupancy.emplace(key, eval_blocks_per_sm(make_model(h, *ds), stride, lanes, fp64, vglobal, A)).first;
   }
-  DeviceSchedule* ds = nullptr;
-  int st = get_schedule(h, c.lanes, access_width(fp64, c.A), &ds);
+  *bps = h->blocks_per_sm > 0 ? std::min(it->second, h->blocks_per_sm) : it->second;
+  return MTP_OK;
+}
+
+// Expected time (us) of an evaluation of natoms with `bps` blocks of `lanes`
+// threads and A atoms per SM.  A block iteration costs a fixed latency, the
+// program's steps (each lane walks T / lanes of the T products three times
+// over) and the throughput of the atoms that share an SM; the blocks run it
+// once per round.  The constants are fitted to 512, 256 and 128 lanes x 1, 2
+// and 4 atoms on 16 to 32,000 atoms at levels 16, 20 and 24 (T = 969, 6,349
+// and 36,170).  Level 24 mixed, measured / estimated: 512 x 1 alone 36 / 36,
+// 512 x 4 alone 54 / 51, 256 x 2 two on an SM 60 / 61, 128 x 1 alone 68 / 68;
+// level 16 FP64 128 x 1 21 / 24, 128 x 2 24 / 27.
+// The rule it replaces took the most atoms in flight whatever the number of
+// atoms, then the most warps: level 24 mixed ran 256 x 1 (7.35 ms at 55,296
+// atoms; 512 x 4 4.15 ms), 16 atoms of level 16 128 x 4 (29 us; 128 x 1 21 us).
+double launch_estimate(const Potential& pot, bool fp64, int lanes, int A, int bps, int sms, long long natoms) {
+  const long long groups = (natoms + A - 1) / A;
+  const long long rounds = std::max(1LL, (groups + static_cast<long long>(bps) * sms - 1) / (static_cast<long long>(bps) * sms));
+  const long long resident = std::max(1LL, std::min<long long>(bps, (groups + sms - 1) / sms));
+  const double atom = fp64 ? 2.5 + 2.5e-4 * pot.T : 1.7 + 9e-5 * pot.T;
+  return rounds * (20.0 + 0.15 * pot.T / lanes + atom * A * resident);
+}
+
+// Launch shape for the evaluation kernel on natoms: the (lanes, atoms per
+// block) within the handle's request with the least expected time
+// (launch_estimate) among those whose value space fits in shared memory; when
+// none fits, the value space moves to global memory (A = 1).
+// While the stream is being captured nothing can be uploaded, so a shape whose
+// programs are not on the device yet gives way to the best one whose are.
+int pick_launch(mtp_handle* h, long long natoms, int stride, const DeviceSchedule** ds_out, int* blocks_out, bool fp64,
+                bool* vglobal_out) {
+  struct Choice { int lanes = 0, A = 1, bps = 0; double est = 0.0; };
+  Choice best, ready;
+  for (int lanes : {512, 256, 128}) {
+    if (h->threads > 0 && lanes > h->threads) continue;
+    for (int A : {4, 2, 1}) {
+      if (h->apb > 0 && A != h->apb) continue;
+      if (!eval_variant_exists(fp64, false, A)) continue;
+      int bps = 0;
+      const int st = launch_occupancy(h, lanes, stride, fp64, false, A, &bps);
+      if (st != MTP_OK) return st;
+      if (bps <= 0) continue;
+      const Choice c{lanes, A, bps, launch_estimate(h->pot, fp64, lanes, A, bps, h->sm_count, natoms)};
+      if (best.lanes == 0 || c.est < best.est) best = c;
+      if (schedule_uploaded(h, lanes, access_width(fp64, A)) && (ready.lanes == 0 || c.est < ready.est)) ready = c;
+    }
+  }
+  bool vglobal = false;
+  if (best.lanes == 0) {
+    // value space in global memory: 512 lanes give an SM 16 warps with one
+    // block, so the blocks' value spaces stay within L2
+    vglobal = true;
+    best.lanes = 512;
+    const int st = launch_occupancy(h, best.lanes, stride, fp64, true, 1, &best.bps);
+    if (st != MTP_OK) return st;
+    if (best.bps <= 0)
+      return fail(h, MTP_E_CAPACITY, "the evaluation block does not fit in shared memory for this basis and max_nbr");
+    best.bps = 1;
+  } else if (ready.lanes > 0 && !schedule_uploaded(h, best.lanes, access_width(fp64, best.A))) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) cudaGetLastError();
+    if (cs != cudaStreamCaptureStatusNone) best = ready;
+  }
+  const DeviceSchedule* ds = nullptr;
+  const int st = get_schedule(h, best.lanes, access_width(fp64, best.A), &ds);
   if (st != MTP_OK) return st;
-  const long long groups = (static_cast<long long>(natoms) + c.A - 1) / c.A;
-  const long long blocks = std::max(1LL, std::min<long long>(static_cast<long long>(c.bps) * h->sm_count, groups));
-  if (c.vglobal) {
-    const size_t need = static_cast<size_t>(blocks) * ds->sched.v_size * c.A * (fp64 ? sizeof(double) : sizeof(float));
+  const long long groups = (natoms + best.A - 1) / best.A;
+  const long long blocks = std::max(1LL, std::min<long long>(static_cast<long long>(best.bps) * h->sm_count, groups));
+  if (vglobal) {
+    const size_t need = static_cast<size_t>(blocks) * ds->sched.v_size * (fp64 ? sizeof(double) : sizeof(float));
     if (need > h->vscratch_bytes) {
       if (h->d_vscratch) cudaFree(h->d_vscratch);
       h->d_vscratch = nullptr;
@@ -393,26 +427,28 @@ int pick_launch(mtp_handle* h, int natoms, int stride, DeviceSchedule** ds_out, 
   }
   *ds_out = ds;
   *blocks_out = static_cast<int>(blocks);
-  *vglobal_out = c.vglobal;
-  h->last_threads = c.lanes;
+  *vglobal_out = vglobal;
+  h->last_threads = best.lanes;
   h->last_blocks = static_cast<int>(blocks);
-  h->last_bps = c.bps;
-  h->last_vglobal = c.vglobal;
-  h->last_smem = c.smem;
-  h->last_apb = c.A;
+  h->last_bps = best.bps;
+  h->last_vglobal = vglobal;
+  h->last_smem = eval_smem_bytes(make_model(h, *ds), stride, best.lanes, fp64, vglobal, best.A);
+  h->last_apb = best.A;
   return MTP_OK;
 }
 
-// Evaluation kernel on atoms [lo, lo + n) of device rows (site energies and
-// per-slot gradients of those atoms).
-int eval_range(mtp_handle* h, int lo, int n, int stride, const int* itypes, const double* rijs, const int* jtypes,
+// Evaluation kernel on atoms [lo, lo + n) of a system of `natoms` in device
+// rows (site energies and per-slot gradients of those atoms).  The launch
+// shape is that of the whole system, so the parts round as one launch would.
+int eval_range(mtp_handle* h, int natoms, int lo, int n, int stride, const int* itypes, const double* rijs, const int* jtypes,
                const int* counts) {
   const bool fp64 = h->precision == MTP_PRECISION_FP64;
-  DeviceSchedule* ds = nullptr;
+  const DeviceSchedule* ds = nullptr;
   int blocks = 0;
   bool vglobal = false;
-  int st = pick_launch(h, n, stride, &ds, &blocks, fp64, &vglobal);
+  int st = pick_launch(h, natoms, stride, &ds, &blocks, fp64, &vglobal);
   if (st != MTP_OK) return st;
+  blocks = std::max(1, std::min(blocks, (n + h->last_apb - 1) / h->last_apb));
   DevModel md = make_model(h, *ds);
   const size_t rows = static_cast<size_t>(lo) * stride;
   DevIO io{};
@@ -458,7 +494,7 @@ int run_device(mtp_handle* h, int natoms, int stride, const int* itypes, const d
   cudaEvent_t e1 = nullptr;
   int st = prof_begin(h, &e1);
   if (st != MTP_OK) return st;
-  st = eval_range(h, 0, natoms, stride, itypes, rijs, jtypes, counts);
+  st = eval_range(h, natoms, 0, natoms, stride, itypes, rijs, jtypes, counts);
   if (st != MTP_OK) return st;
   if (e1) MTP_CUDA(h, cudaEventRecord(e1, h->stream));
   MTP_CUDA(h, launch_force_gather(natoms, stride, rijs, counts, h->d_G, h->d_in_ptr, h->d_in_slot, forces,
@@ -509,7 +545,7 @@ int run_host_pipelined_body(mtp_handle* h, int natoms, int stride, const int* it
       int st = prof_begin(h, &e1);
       if (st != MTP_OK) return st;
     }
-    int st = eval_range(h, lo, hi - lo, stride, h->d_itypes, h->d_rijs, h->d_jtypes, counts ? h->d_counts : nullptr);
+    int st = eval_range(h, natoms, lo, hi - lo, stride, h->d_itypes, h->d_rijs, h->d_jtypes, counts ? h->d_counts : nullptr);
     if (st != MTP_OK) return st;
   }
   if (e1) MTP_CUDA(h, cudaEventRecord(e1, s));
@@ -790,8 +826,8 @@ int mtp_create(const char* mtp_path, int max_atoms, int max_nbr, double cutoff, 
     return bail(cuda_fail(h, cudaGetLastError(), "upload mapping"));
   int st = upload_coeffs(h);
   if (st != MTP_OK) return bail(st);
-  DeviceSchedule* ds = nullptr;
-  st = get_schedule(h, h->threads, access_width(precision == MTP_PRECISION_FP64, 1), &ds, false);
+  const DeviceSchedule* ds = nullptr;
+  st = get_sizes(h, 256, &ds);   // checks the tables
   if (st != MTP_OK) return bail(st);
   if (h->debug >= 1) {
     std::fprintf(stderr, "[mtp_b200] %s: S=%d R=%d K=%d M=%d B=%d T=%d Sa=%d; %d fwd + %d rev passes, %d value slots\n",
@@ -1211,9 +1247,9 @@ int mtp_adjoint_batch_device(mtp_handle* h, int natoms, int stride, int nconfig,
     return fail(h, MTP_E_INVALID, "null pointer");
   // with the value space in global memory, 512 lanes give the SM twice the
   // warps for the same L2 footprint
-  int lanes = h->threads;
-  DeviceSchedule* ds = nullptr;
-  int st = get_schedule(h, lanes, access_width(true, 1), &ds, false);
+  int lanes = h->threads > 0 ? h->threads : 256;
+  const DeviceSchedule* ds = nullptr;
+  int st = get_sizes(h, lanes, &ds);
   if (st != MTP_OK) return st;
   if (lanes < 512 && !adjoint_fits_shared(make_model(h, *ds), stride, lanes)) lanes = 512;
   st = get_schedule(h, lanes, access_width(true, 1), &ds);
@@ -1467,11 +1503,12 @@ int mtp_compute_device_noalloc(mtp_handle* h, int natoms, int stride, const int*
   // for, within the handle's launch limits (mtp_set_launch); the value space
   // must fit in shared memory (its global-memory form would need an allocation)
   const DeviceSchedule* ds = nullptr;
-  int lanes = 0, A = 1, bps = 0, best = -1;
+  int lanes = 0, A = 1, bps = 0;
+  double best = 0.0;
   for (const auto& kv : h->scheds) {
     const DevModel md = make_model(h, kv.second);
     const int sl = kv.second.sched.lanes;
-    if (sl > h->threads) continue;
+    if (h->threads > 0 && sl > h->threads) continue;
     for (int a : {4, 2, 1}) {
       if (!eval_variant_exists(fp64, false, a)) continue;
       if (h->apb > 0 && a != h->apb) continue;
@@ -1479,9 +1516,9 @@ int mtp_compute_device_noalloc(mtp_handle* h, int natoms, int stride, const int*
       int b = eval_blocks_per_sm(md, stride, sl, fp64, false, a);
       if (h->blocks_per_sm > 0) b = std::min(b, h->blocks_per_sm);
       if (b <= 0) continue;
-      const int score = (a * b) * 1024 + b * sl / 32;
-      if (score > best) {
-        best = score;
+      const double est = launch_estimate(h->pot, fp64, sl, a, b, h->sm_count, natoms);
+      if (!ds || est < best) {
+        best = est;
         ds = &kv.second;
         lanes = sl;
         A = a;

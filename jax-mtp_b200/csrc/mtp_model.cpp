@@ -389,8 +389,8 @@ RawPass lay_out(const std::vector<Job>& jobs, int lanes, int width, bool allow_s
 // Split long jobs into chunks writing partial slots; returns the main pass and,
 // when anything was split, the combine pass.  `parts_used` gets the number of
 // partial slots the pass pair needs.
-void emit_jobs(const std::vector<Job>& jobs, int lanes, int width, bool allow_swap, std::vector<RawPass>& out,
-               int& parts_used) {
+void emit_jobs(const std::vector<Job>& jobs, int lanes, int width, bool allow_swap, bool programs,
+               std::vector<RawPass>& out, int& parts_used) {
   size_t total = 0;
   for (const Job& j : jobs) total += j.sides.size();
   if (total == 0) return;
@@ -415,8 +415,8 @@ void emit_jobs(const std::vector<Job>& jobs, int lanes, int width, bool allow_sw
     }
     comb_jobs.push_back(std::move(comb));
   }
-  out.push_back(lay_out(main_jobs, lanes, width, allow_swap));
-  if (!comb_jobs.empty()) out.push_back(lay_out(comb_jobs, lanes, width, false));
+  out.push_back(programs ? lay_out(main_jobs, lanes, width, allow_swap) : RawPass());
+  if (!comb_jobs.empty()) out.push_back(programs ? lay_out(comb_jobs, lanes, width, false) : RawPass());
   parts_used = std::max(parts_used, parts);
 }
 
@@ -469,7 +469,7 @@ void seed_list(const Potential& pot, std::vector<int>& idx, std::vector<double>&
   }
 }
 
-bool build_schedule(const Potential& pot, int lanes, Schedule& s, std::string& err, int width) {
+bool build_schedule(const Potential& pot, int lanes, Schedule& s, std::string& err, int width, bool programs) {
   s = Schedule();
   s.lanes = lanes;
   s.width = width;
@@ -614,7 +614,7 @@ bool build_schedule(const Potential& pot, int lanes, Schedule& s, std::string& e
       jobs[it->second].sides.push_back(
           Side{static_cast<uint32_t>(s.v_m + r[0]), static_cast<uint32_t>(s.v_m + r[1]), static_cast<uint32_t>(r[2])});
     }
-    emit_jobs(jobs, lanes, width, true, fwd, parts);
+    emit_jobs(jobs, lanes, width, true, programs, fwd, parts);
   }
   // reverse: passes for target depth maxd..1 gather sides whose source has
   // depth >= 1; every side into a depth-0 source waits for one final pass.
@@ -642,7 +642,7 @@ bool build_schedule(const Potential& pot, int lanes, Schedule& s, std::string& e
       if (depth[r[0]] >= 1) add_side(jobs, job_of, r[0], r[3], r[1], r[2]);
       if (depth[r[1]] >= 1) add_side(jobs, job_of, r[1], r[3], r[0], r[2]);
     }
-    emit_jobs(jobs, lanes, width, false, rev, parts);
+    emit_jobs(jobs, lanes, width, false, programs, rev, parts);
     for (const auto& kv : job_of) written[kv.first] = 1;
   }
   {
@@ -656,7 +656,7 @@ bool build_schedule(const Potential& pot, int lanes, Schedule& s, std::string& e
         if (depth[r[1]] == 0) add_side(jobs, job_of, r[1], r[3], r[0], r[2]);
       }
     }
-    emit_jobs(jobs, lanes, width, false, rev, parts);
+    emit_jobs(jobs, lanes, width, false, programs, rev, parts);
     for (const auto& kv : job_of) written[kv.first] = 1;
   }
   for (int k = 0; k < M; ++k)
@@ -687,7 +687,7 @@ bool build_schedule(const Potential& pot, int lanes, Schedule& s, std::string& e
       p.offset = static_cast<int>(s.entries.size() / 2);
       p.steps = (rp.steps + kStepAlign - 1) / kStepAlign * kStepAlign;
       p.wsteps.assign(lanes / 32, 0);
-      for (int l = 0; l < lanes; ++l)
+      for (int l = 0; l < lanes && programs; ++l)
         p.wsteps[l / 32] = std::max(p.wsteps[l / 32], (rp.lane_len[l] + kStepAlign - 1) / kStepAlign * kStepAlign);
       for (const RawEntry& r : rp.e) {
         uint32_t a = resolve(r.a), b = resolve(r.b), d = resolve(r.dst);

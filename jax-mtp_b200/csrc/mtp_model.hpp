@@ -121,7 +121,10 @@ struct Schedule {
 // `width` bytes (sizeof(real) x atoms per block; it sets the bank model the
 // entry order is tuned for).  Fails (false, err) if the table does not have a
 // write-before-read order, or exceeds index limits.
-bool build_schedule(const Potential& pot, int lanes, Schedule& out, std::string& err, int width = 4);
+// With `programs` false everything but the programs is made (value-space size,
+// tables, all checks of the table): enough to size a launch.
+bool build_schedule(const Potential& pot, int lanes, Schedule& out, std::string& err, int width = 4,
+                    bool programs = true);
 
 // Local search over a built schedule against shared-memory bank conflicts:
 // an entry whose bank key sets a gather's wavefront count trades steps with
