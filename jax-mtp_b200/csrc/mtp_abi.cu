@@ -89,13 +89,13 @@ struct mtp_handle {
   int *d_itypes = nullptr, *d_js = nullptr, *d_jtypes = nullptr, *d_counts = nullptr;
   double* d_rijs = nullptr;
   double *d_G = nullptr, *d_E = nullptr, *d_F = nullptr, *d_wown = nullptr, *d_vatom = nullptr;
-  int *d_in_cnt = nullptr, *d_in_ptr = nullptr, *d_in_cursor = nullptr, *d_in_slot = nullptr, *d_blk = nullptr;
+  int *d_in_cnt = nullptr, *d_in_ptr = nullptr, *d_in_slot = nullptr, *d_blk = nullptr;
   double *d_partials = nullptr, *d_tot = nullptr;
   int* d_err = nullptr;
   int* d_cfg_ptr = nullptr;
   int cfg_cap = 0;
-  double* h_tot = nullptr;   // pinned [7]
-  int* h_err = nullptr;      // pinned [1]
+  double* h_tot = nullptr;   // pinned [8]: totals, error flags
+  int* h_err = nullptr;      // the flags' word of h_tot
   TrainWorkspace train;
   CellScratch cells;
   // blocks per SM of a (lanes, atoms per block, stride, precision, value-space
@@ -313,7 +313,7 @@ void free_handle(mtp_handle* h) {
   F(h->d_mono_word); F(h->d_mono_list);
   F(h->d_itypes); F(h->d_js); F(h->d_jtypes); F(h->d_counts); F(h->d_rijs);
   F(h->d_G); F(h->d_E); F(h->d_F); F(h->d_wown); F(h->d_vatom);
-  F(h->d_in_cnt); F(h->d_in_ptr); F(h->d_in_cursor); F(h->d_in_slot); F(h->d_blk);
+  F(h->d_in_cnt); F(h->d_in_ptr); F(h->d_in_slot); F(h->d_blk);
   F(h->d_partials); F(h->d_tot); F(h->d_err); F(h->d_cfg_ptr); F(h->d_vscratch);
   F(h->d_xall); F(h->d_spall); F(h->d_owner); F(h->d_neigh); F(h->d_numneigh);
   train_free(h->train);
@@ -324,7 +324,6 @@ void free_handle(mtp_handle* h) {
     cudaEventDestroy(ev.second);
   }
   if (h->h_tot) cudaFreeHost(h->h_tot);
-  if (h->h_err) cudaFreeHost(h->h_err);
   for (auto ev : h->chunk_events) cudaEventDestroy(ev);
   if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
   if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
@@ -488,8 +487,8 @@ int prof_begin(mtp_handle* h, cudaEvent_t* e1) {
 int run_device(mtp_handle* h, int natoms, int stride, const int* itypes, const double* rijs, const int* js,
                const int* jtypes, const int* counts, bool rebuild_incoming, double* forces, double* vatom) {
   if (rebuild_incoming) {
-    MTP_CUDA(h, launch_incoming(natoms, stride, js, jtypes, counts, h->d_in_cnt, h->d_in_ptr, h->d_in_cursor,
-                                h->d_in_slot, h->d_blk, h->stream));
+    MTP_CUDA(h, launch_incoming(natoms, stride, js, jtypes, counts, h->d_in_cnt, h->d_in_ptr, h->d_in_slot,
+                                h->d_blk, h->stream));
   }
   cudaEvent_t e1 = nullptr;
   int st = prof_begin(h, &e1);
@@ -497,8 +496,33 @@ int run_device(mtp_handle* h, int natoms, int stride, const int* itypes, const d
   st = eval_range(h, natoms, 0, natoms, stride, itypes, rijs, jtypes, counts);
   if (st != MTP_OK) return st;
   if (e1) MTP_CUDA(h, cudaEventRecord(e1, h->stream));
-  MTP_CUDA(h, launch_force_gather(natoms, stride, rijs, counts, h->d_G, h->d_in_ptr, h->d_in_slot, forces,
-                                  h->d_wown, vatom, h->stream));
+  MTP_CUDA(h, launch_force_gather(natoms, stride, rijs, counts, h->d_G, h->d_in_ptr, h->d_in_slot,
+                                  rebuild_incoming, forces, h->d_wown, vatom, h->stream));
+  return MTP_OK;
+}
+
+// True where a kernel can write through p (device, managed or page-locked
+// host memory).
+bool device_writable(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type != cudaMemoryTypeUnregistered && a.devicePointer == p;
+}
+
+// Totals into the caller's device buffers (null: not asked for), by the kernel
+// itself or, where it cannot write there, by copies that report the error.
+int write_totals(mtp_handle* h, int natoms, const double* site_energy, const double* wown, double* partials,
+                 double* tot, double* d_energy, double* d_virial) {
+  const bool e = d_energy && device_writable(d_energy), v = d_virial && device_writable(d_virial);
+  MTP_CUDA(h, launch_totals(natoms, site_energy, wown, partials, tot, h->d_err, e ? d_energy : nullptr,
+                            v ? d_virial : nullptr, h->stream));
+  if (d_energy && !e)
+    MTP_CUDA(h, cudaMemcpyAsync(d_energy, tot, sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+  if (d_virial && !v)
+    MTP_CUDA(h, cudaMemcpyAsync(d_virial, tot + 1, 6 * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
   return MTP_OK;
 }
 
@@ -550,9 +574,9 @@ int run_host_pipelined_body(mtp_handle* h, int natoms, int stride, const int* it
   }
   if (e1) MTP_CUDA(h, cudaEventRecord(e1, s));
   MTP_CUDA(h, launch_incoming(natoms, stride, h->d_js, h->d_jtypes, counts ? h->d_counts : nullptr, h->d_in_cnt,
-                              h->d_in_ptr, h->d_in_cursor, h->d_in_slot, h->d_blk, s));
+                              h->d_in_ptr, h->d_in_slot, h->d_blk, s));
   MTP_CUDA(h, launch_force_gather(natoms, stride, h->d_rijs, counts ? h->d_counts : nullptr, h->d_G, h->d_in_ptr,
-                                  h->d_in_slot, h->d_F, h->d_wown, vatom, s));
+                                  h->d_in_slot, true, h->d_F, h->d_wown, vatom, s));
   return MTP_OK;
 }
 
@@ -618,15 +642,14 @@ int enqueue_small_call(mtp_handle* h, int natoms, int stride, const int* itypes,
   int st = run_device(h, natoms, stride, h->d_itypes, h->d_rijs, h->d_js, h->d_jtypes, counts ? h->d_counts : nullptr,
                       true, h->d_F, (flags & MTP_VATOM) ? h->d_vatom : nullptr);
   if (st != MTP_OK) return st;
-  MTP_CUDA(h, launch_totals(natoms, h->d_E, h->d_wown, h->d_partials, h->d_tot, s));
+  MTP_CUDA(h, launch_totals(natoms, h->d_E, h->d_wown, h->d_partials, h->d_tot, h->d_err, nullptr, nullptr, s));
   if (natoms > 0) {
     MTP_CUDA(h, cudaMemcpyAsync(forces, h->d_F, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, s));
     if (flags & MTP_EATOM) MTP_CUDA(h, cudaMemcpyAsync(eatom, h->d_E, N * sizeof(double), cudaMemcpyDeviceToHost, s));
     if (flags & MTP_VATOM)
       MTP_CUDA(h, cudaMemcpyAsync(vatom, h->d_vatom, 6 * N * sizeof(double), cudaMemcpyDeviceToHost, s));
   }
-  MTP_CUDA(h, cudaMemcpyAsync(h->h_tot, h->d_tot, 7 * sizeof(double), cudaMemcpyDeviceToHost, s));
-  MTP_CUDA(h, cudaMemcpyAsync(h->h_err, h->d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+  MTP_CUDA(h, cudaMemcpyAsync(h->h_tot, h->d_tot, 8 * sizeof(double), cudaMemcpyDeviceToHost, s));   // flags in the last
   return MTP_OK;
 }
 
@@ -807,21 +830,22 @@ int mtp_create(const char* mtp_path, int max_atoms, int max_nbr, double cutoff, 
             dalloc(&h->d_E, N) == cudaSuccess && dalloc(&h->d_F, 3 * N) == cudaSuccess &&
             dalloc(&h->d_wown, 6 * N) == cudaSuccess && dalloc(&h->d_vatom, 6 * N) == cudaSuccess &&
             dalloc(&h->d_in_cnt, N) == cudaSuccess && dalloc(&h->d_in_ptr, N + 1) == cudaSuccess &&
-            dalloc(&h->d_in_cursor, N) == cudaSuccess && dalloc(&h->d_in_slot, NS) == cudaSuccess &&
+            dalloc(&h->d_in_slot, NS) == cudaSuccess &&
             dalloc(&h->d_blk, (N + 1023) / 1024 + 1) == cudaSuccess &&
-            dalloc(&h->d_partials, 7 * kReduceBlocks) == cudaSuccess && dalloc(&h->d_tot, 8) == cudaSuccess &&
+            dalloc(&h->d_partials, 7 * kReduceBlocks) == cudaSuccess && dalloc(&h->d_tot, kTotals) == cudaSuccess &&
             dalloc(&h->d_err, 1) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
     h->err = "device allocation failed for the requested capacities";
     return bail(MTP_E_OOM);
   }
-  if (cudaMallocHost(&h->h_tot, 8 * sizeof(double)) != cudaSuccess ||
-      cudaMallocHost(&h->h_err, sizeof(int)) != cudaSuccess) {
+  if (cudaMallocHost(&h->h_tot, 8 * sizeof(double)) != cudaSuccess) {
     h->err = "pinned host allocation failed";
     return bail(MTP_E_OOM);
   }
+  h->h_err = reinterpret_cast<int*>(h->h_tot + 7);
   cudaMemset(h->d_err, 0, sizeof(int));
+  cudaMemset(h->d_tot, 0, kTotals * sizeof(double));
   if (cudaMemcpy(h->d_mapping, p.mapping.data(), p.Sa * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
     return bail(cuda_fail(h, cudaGetLastError(), "upload mapping"));
   int st = upload_coeffs(h);
@@ -937,11 +961,9 @@ int mtp_compute_device(mtp_handle* h, int natoms, int stride, const int* d_itype
                       (flags & MTP_VATOM) ? d_vatom : nullptr);
   if (st != MTP_OK) return st;
   if (flags & (MTP_EFLAG | MTP_VFLAG)) {
-    MTP_CUDA(h, launch_totals(natoms, h->d_E, h->d_wown, h->d_partials, h->d_tot, h->stream));
-    if (flags & MTP_EFLAG)
-      MTP_CUDA(h, cudaMemcpyAsync(d_energy, h->d_tot, sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    if (flags & MTP_VFLAG)
-      MTP_CUDA(h, cudaMemcpyAsync(d_virial, h->d_tot + 1, 6 * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+    st = write_totals(h, natoms, h->d_E, h->d_wown, h->d_partials, h->d_tot, (flags & MTP_EFLAG) ? d_energy : nullptr,
+                      (flags & MTP_VFLAG) ? d_virial : nullptr);
+    if (st != MTP_OK) return st;
   }
   if ((flags & MTP_EATOM) && natoms > 0)
     MTP_CUDA(h, cudaMemcpyAsync(d_eatom, h->d_E, natoms * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
@@ -972,11 +994,9 @@ int mtp_compute_positions_device(mtp_handle* h, int nlocal, int nall, const doub
                       h->d_counts, true, d_forces, (flags & MTP_VATOM) ? d_vatom : nullptr);
   if (st != MTP_OK) return st;
   if (flags & (MTP_EFLAG | MTP_VFLAG)) {
-    MTP_CUDA(h, launch_totals(nlocal, h->d_E, h->d_wown, h->d_partials, h->d_tot, h->stream));
-    if (flags & MTP_EFLAG)
-      MTP_CUDA(h, cudaMemcpyAsync(d_energy, h->d_tot, sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-    if (flags & MTP_VFLAG)
-      MTP_CUDA(h, cudaMemcpyAsync(d_virial, h->d_tot + 1, 6 * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+    st = write_totals(h, nlocal, h->d_E, h->d_wown, h->d_partials, h->d_tot, (flags & MTP_EFLAG) ? d_energy : nullptr,
+                      (flags & MTP_VFLAG) ? d_virial : nullptr);
+    if (st != MTP_OK) return st;
   }
   if ((flags & MTP_EATOM) && nlocal > 0)
     MTP_CUDA(h, cudaMemcpyAsync(d_eatom, h->d_E, nlocal * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
@@ -1016,7 +1036,7 @@ int mtp_compute(mtp_handle* h, int natoms, int stride, const int* itypes, const 
       cudaStreamSynchronize(s);   // copies from the caller's buffers complete before the error returns
       return st;
     }
-    MTP_CUDA(h, launch_totals(natoms, h->d_E, h->d_wown, h->d_partials, h->d_tot, s));
+    MTP_CUDA(h, launch_totals(natoms, h->d_E, h->d_wown, h->d_partials, h->d_tot, h->d_err, nullptr, nullptr, s));
     MTP_CUDA(h, cudaMemcpyAsync(forces, h->d_F, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, s));
     if (flags & MTP_EATOM) MTP_CUDA(h, cudaMemcpyAsync(eatom, h->d_E, N * sizeof(double), cudaMemcpyDeviceToHost, s));
     if (flags & MTP_VATOM)
@@ -1096,7 +1116,7 @@ int mtp_compute_positions(mtp_handle* h, int nlocal, int nall, const double* x, 
     int st = run_device(h, nlocal, stride, nlocal > 0 ? h->d_spall : h->d_itypes, h->d_rijs, h->d_js, h->d_jtypes,
                         h->d_counts, true, h->d_F, (flags & MTP_VATOM) ? h->d_vatom : nullptr);
     if (st != MTP_OK) return st;
-    MTP_CUDA(h, launch_totals(nlocal, h->d_E, h->d_wown, h->d_partials, h->d_tot, s));
+    MTP_CUDA(h, launch_totals(nlocal, h->d_E, h->d_wown, h->d_partials, h->d_tot, h->d_err, nullptr, nullptr, s));
     if (nlocal > 0) {
       MTP_CUDA(h, cudaMemcpyAsync(forces, h->d_F, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, s));
       if (flags & MTP_EATOM)
@@ -1104,8 +1124,7 @@ int mtp_compute_positions(mtp_handle* h, int nlocal, int nall, const double* x, 
       if (flags & MTP_VATOM)
         MTP_CUDA(h, cudaMemcpyAsync(vatom, h->d_vatom, 6 * N * sizeof(double), cudaMemcpyDeviceToHost, s));
     }
-    MTP_CUDA(h, cudaMemcpyAsync(h->h_tot, h->d_tot, 7 * sizeof(double), cudaMemcpyDeviceToHost, s));
-    MTP_CUDA(h, cudaMemcpyAsync(h->h_err, h->d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    MTP_CUDA(h, cudaMemcpyAsync(h->h_tot, h->d_tot, 8 * sizeof(double), cudaMemcpyDeviceToHost, s));   // flags in the last
     return MTP_OK;
   };
   HostCallKey key;
@@ -1425,7 +1444,7 @@ namespace {
 constexpr size_t al256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 
 struct NoAllocLayout {
-  size_t grad, energy, wown, in_cnt, in_ptr, in_cursor, in_slot, blk, partials, tot, total;
+  size_t grad, energy, wown, in_cnt, in_ptr, in_slot, blk, partials, tot, total;
 };
 
 constexpr NoAllocLayout noalloc_layout() {
@@ -1437,11 +1456,10 @@ constexpr NoAllocLayout noalloc_layout() {
   L.wown = o;      o = al256(o + atoms * 6 * sizeof(double));
   L.in_cnt = o;    o = al256(o + atoms * sizeof(int));
   L.in_ptr = o;    o = al256(o + (atoms + 1) * sizeof(int));
-  L.in_cursor = o; o = al256(o + atoms * sizeof(int));
   L.in_slot = o;   o = al256(o + slots * sizeof(int));
   L.blk = o;       o = al256(o + (atoms / 1024 + 2) * sizeof(int));
   L.partials = o;  o = al256(o + 7 * kReduceBlocks * sizeof(double));
-  L.tot = o;       o = al256(o + 8 * sizeof(double));
+  L.tot = o;       o = al256(o + kTotals * sizeof(double));
   L.total = o;
   return L;
 }
@@ -1537,14 +1555,14 @@ int mtp_compute_device_noalloc(mtp_handle* h, int natoms, int stride, const int*
   double* wown = reinterpret_cast<double*>(base + kNoAlloc.wown);
   int* in_cnt = reinterpret_cast<int*>(base + kNoAlloc.in_cnt);
   int* in_ptr = reinterpret_cast<int*>(base + kNoAlloc.in_ptr);
-  int* in_cursor = reinterpret_cast<int*>(base + kNoAlloc.in_cursor);
   int* in_slot = reinterpret_cast<int*>(base + kNoAlloc.in_slot);
   int* blk = reinterpret_cast<int*>(base + kNoAlloc.blk);
   double* partials = reinterpret_cast<double*>(base + kNoAlloc.partials);
   double* tot = reinterpret_cast<double*>(base + kNoAlloc.tot);
 
   // The array keeps the previous call's contents.  The incoming-slot counters
-  // must start at zero (launch_incoming clears in_cnt and in_cursor first);
+  // must start at zero (launch_incoming clears them first) and the totals' counter
+  // does (it ends every launch at zero);
   // every other piece is fully rewritten before it is read: each slot's
   // gradient (zero for skipped slots), each site energy and per-atom virial,
   // the scan blocks, the partials and the totals.
@@ -1564,14 +1582,12 @@ int mtp_compute_device_noalloc(mtp_handle* h, int natoms, int stride, const int*
   const long long groups = (static_cast<long long>(natoms) + A - 1) / A;
   const int blocks = static_cast<int>(std::max(1LL, std::min<long long>(static_cast<long long>(bps) * h->sm_count,
                                                                          groups)));
-  MTP_CUDA(h, launch_incoming(natoms, stride, d_js, d_jtypes, d_counts, in_cnt, in_ptr, in_cursor, in_slot, blk,
-                              h->stream));
+  MTP_CUDA(h, launch_incoming(natoms, stride, d_js, d_jtypes, d_counts, in_cnt, in_ptr, in_slot, blk, h->stream));
   MTP_CUDA(h, launch_eval(md, io, lanes, blocks, fp64, false, A, h->stream));
-  MTP_CUDA(h, launch_force_gather(natoms, stride, d_rijs, d_counts, grad, in_ptr, in_slot, d_forces, wown, nullptr,
+  MTP_CUDA(h, launch_force_gather(natoms, stride, d_rijs, d_counts, grad, in_ptr, in_slot, true, d_forces, wown, nullptr,
                                   h->stream));
-  MTP_CUDA(h, launch_totals(natoms, energy, wown, partials, tot, h->stream));
-  MTP_CUDA(h, cudaMemcpyAsync(d_energy, tot, sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
-  MTP_CUDA(h, cudaMemcpyAsync(d_virial, tot + 1, 6 * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+  st = write_totals(h, natoms, energy, wown, partials, tot, d_energy, d_virial);
+  if (st != MTP_OK) return st;
   h->calls++;
   return MTP_OK;
 }

@@ -184,9 +184,50 @@ __global__ void k_scan_add(int n, int* out, const int* block_off) {
   if (i < n) out[i] += block_off[blockIdx.x];
 }
 
+// The whole scan in one block: thread t sums the `per` consecutive values it
+// owns, the block scans the sums, and the thread writes its prefixes.  For
+// small n (a LAMMPS-size call) it replaces three launches.
+__global__ void k_scan_one_block(int n, int per, const int* __restrict__ in, int* __restrict__ out) {
+  __shared__ int wsum[32];
+  const int l = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int b = min(n, static_cast<int>(threadIdx.x) * per), e = min(n, b + per);
+  int v = 0;
+  for (int i = b; i < e; ++i) v += in[i];
+  int x = v;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (l >= o) x += y;
+  }
+  if (l == 31) wsum[w] = x;
+  __syncthreads();
+  if (w == 0) {
+    int s = wsum[l];
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, s, o);
+      if (l >= o) s += y;
+    }
+    wsum[l] = s;
+  }
+  __syncthreads();
+  int run = x - v + (w > 0 ? wsum[w - 1] : 0);
+  for (int i = b; i < e; ++i) {
+    out[i] = run;
+    run += in[i];
+  }
+  if (threadIdx.x == 1023) out[n] = run;
+}
+
+// Up to this many values one block scans all (8 per thread: 4 us at 8,192
+// values; the three kernels take 6 us with their gaps).
+constexpr int kOneBlockScan = 8192;
+
 // out[0..n) = exclusive prefix sums of in, out[n] = total; blk holds n/1024 + 1 ints.
 cudaError_t scan_exclusive(int n, const int* in, int* out, int* blk, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
+  if (n <= kOneBlockScan) {
+    k_scan_one_block<<<1, 1024, 0, st>>>(n, (n + 1023) / 1024, in, out);
+    return cudaGetLastError();
+  }
   const int nb = (n + 1023) / 1024;
   k_scan_blocks<<<nb, 1024, 0, st>>>(n, in, out, blk);
   k_scan_totals<<<1, 1024, 0, st>>>(nb, blk, out + n);
@@ -194,30 +235,28 @@ cudaError_t scan_exclusive(int n, const int* in, int* out, int* blk, cudaStream_
   return cudaGetLastError();
 }
 
+// Every slot takes a place in its neighbour's list; the counts run down to
+// zero as they hand the places out.
 __global__ void k_fill_incoming(int natoms, int stride, const int* js, const int* jtypes, const int* counts,
-                                const int* in_ptr, int* in_cursor, int* in_slot) {
+                                const int* in_ptr, int* in_cnt, int* in_slot) {
   const size_t n = static_cast<size_t>(natoms) * stride;
   for (size_t x = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; x < n;
        x += static_cast<size_t>(gridDim.x) * blockDim.x) {
     int j;
     if (scatter_slot(static_cast<int>(x / stride), static_cast<int>(x % stride), natoms, stride, js, jtypes,
                      counts, j)) {
-      const int pos = atomicAdd(in_cursor + j, 1);
+      const int pos = atomicSub(in_cnt + j, 1) - 1;
       in_slot[in_ptr[j] + pos] = static_cast<int>(x);
     }
   }
 }
 
-// Sort each atom's incoming list by slot id: the gather order, and so the
-// rounding of the forces, no longer depends on the fill race above.  One warp
-// per atom: lists of up to 64 slots are ranked in registers (slot ids are
-// distinct, so each value's rank is the count of smaller values); longer
-// lists fall back to an insertion sort by the warp's first lane.
-__global__ void k_sort_incoming(int natoms, const int* in_ptr, int* in_slot) {
-  const int atom = static_cast<int>((blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (atom >= natoms) return;   // the whole warp leaves together
-  const int b = in_ptr[atom], n = in_ptr[atom + 1] - b;
+// Sort one atom's incoming list by slot id (one warp): the gather order, and
+// so the rounding of the forces, no longer depends on the fill race above.
+// Lists of up to 64 slots are ranked in registers (slot ids are distinct, so
+// each value's rank is the count of smaller values); longer lists fall back to
+// an insertion sort by the warp's first lane.
+__device__ __forceinline__ void sort_incoming(int b, int n, int lane, int* in_slot) {
   if (n <= 64) {
     const int v0 = lane < n ? in_slot[b + lane] : INT_MAX;
     const int v1 = lane + 32 < n ? in_slot[b + lane + 32] : INT_MAX;
@@ -241,26 +280,21 @@ __global__ void k_sort_incoming(int natoms, const int* in_ptr, int* in_slot) {
       in_slot[y + 1] = v;
     }
   }
+  __syncwarp();
 }
 
 cudaError_t launch_incoming(int natoms, int stride, const int* js, const int* jtypes, const int* counts,
-                            int* in_cnt, int* in_ptr, int* in_cursor, int* in_slot, int* block_tmp,
-                            cudaStream_t st) {
+                            int* in_cnt, int* in_ptr, int* in_slot, int* block_tmp, cudaStream_t st) {
   if (natoms <= 0) return cudaSuccess;
-  // both counters must start at zero (the allocation-free path reuses a
-  // shared array that still holds the previous call's values)
+  // the counts start at zero (the allocation-free path reuses a shared array)
   cudaError_t e = cudaMemsetAsync(in_cnt, 0, sizeof(int) * natoms, st);
-  if (e != cudaSuccess) return e;
-  e = cudaMemsetAsync(in_cursor, 0, sizeof(int) * natoms, st);
   if (e != cudaSuccess) return e;
   const size_t n = static_cast<size_t>(natoms) * stride;
   const int gb = static_cast<int>(std::min<size_t>((n + 255) / 256, 148 * 32));
   k_count_incoming<<<gb, 256, 0, st>>>(natoms, stride, js, jtypes, counts, in_cnt);
   e = scan_exclusive(natoms, in_cnt, in_ptr, block_tmp, st);
   if (e != cudaSuccess) return e;
-  k_fill_incoming<<<gb, 256, 0, st>>>(natoms, stride, js, jtypes, counts, in_ptr, in_cursor, in_slot);
-  k_sort_incoming<<<static_cast<unsigned>((static_cast<size_t>(natoms) * 32 + 255) / 256), 256, 0, st>>>(
-      natoms, in_ptr, in_slot);
+  k_fill_incoming<<<gb, 256, 0, st>>>(natoms, stride, js, jtypes, counts, in_ptr, in_cnt, in_slot);
   return cudaGetLastError();
 }
 
@@ -276,9 +310,12 @@ __device__ __forceinline__ void sym_rg(const double* r, const double* g, double*
   w[5] += sgn * 0.5 * (r[1] * g[2] + r[2] * g[1]);
 }
 
+// kSort: the incoming lists are fresh from launch_incoming and this atom's is
+// sorted first (here rather than in a launch of its own).
+template <bool kSort>
 __global__ void k_force_gather(int natoms, int stride, const double* __restrict__ rijs,
                                const int* __restrict__ counts, const double* __restrict__ G,
-                               const int* __restrict__ in_ptr, const int* __restrict__ in_slot,
+                               const int* __restrict__ in_ptr, int* in_slot,
                                double* __restrict__ forces, double* __restrict__ wown,
                                double* __restrict__ vatom) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -299,8 +336,9 @@ __global__ void k_force_gather(int natoms, int stride, const double* __restrict_
     sym_rg(rr, gg, Wo, -1.0);
   }
   const int b = __ldg(in_ptr + i), e = __ldg(in_ptr + i + 1);
+  if (kSort) sort_incoming(b, e - b, lane, in_slot);
   for (int x = b + lane; x < e; x += 32) {
-    const size_t slot = static_cast<size_t>(__ldg(in_slot + x));
+    const size_t slot = static_cast<size_t>(in_slot[x]);
     const double* g = G + 3 * slot;
     double gg[3] = {__ldg(g), __ldg(g + 1), __ldg(g + 2)};
     F[0] -= gg[0];
@@ -329,13 +367,17 @@ __global__ void k_force_gather(int natoms, int stride, const double* __restrict_
 }
 
 cudaError_t launch_force_gather(int natoms, int stride, const double* rijs, const int* counts,
-                                const double* pair_grad, const int* in_ptr, const int* in_slot,
+                                const double* pair_grad, const int* in_ptr, int* in_slot, bool sort,
                                 double* forces, double* wown, double* vatom, cudaStream_t st) {
   if (natoms <= 0) return cudaSuccess;
   const int threads = 256;
   const int blocks = (natoms * 32 + threads - 1) / threads;
-  k_force_gather<<<blocks, threads, 0, st>>>(natoms, stride, rijs, counts, pair_grad, in_ptr, in_slot, forces,
-                                             wown, vatom);
+  if (sort)
+    k_force_gather<true><<<blocks, threads, 0, st>>>(natoms, stride, rijs, counts, pair_grad, in_ptr, in_slot, forces,
+                                                     wown, vatom);
+  else
+    k_force_gather<false><<<blocks, threads, 0, st>>>(natoms, stride, rijs, counts, pair_grad, in_ptr, in_slot, forces,
+                                                      wown, vatom);
   return cudaGetLastError();
 }
 
@@ -353,34 +395,58 @@ __device__ __forceinline__ double block_reduce_256(double v, double* red) {
   return s;
 }
 
-__global__ void k_partial_totals(int natoms, const double* __restrict__ e, const double* __restrict__ w,
-                                 double* __restrict__ partials) {
-  __shared__ double red[8];
+// Totals of the site energies and virials in one launch: every block sums its
+// chunk, and the block that finishes last adds the blocks' partials (which
+// block that is does not matter: the order is fixed).  One warp per total
+// there: lane l adds partials l, l + 32, ... in order, then a fixed butterfly
+// over the lanes.  out[0..6] = totals, out[7] = the device error flags so far
+// (low 32 bits), so a host call reads both back with one copy; d_energy and
+// d_virial, where given, get theirs.  The ticket at out + 8 starts at zero and
+// ends at zero.  Two launches and two copies took 9 us of a 2,000-atom call.
+__global__ void k_totals(int natoms, const double* __restrict__ e, const double* __restrict__ w, double* partials,
+                         double* out, const int* err, double* d_energy, double* d_virial) {
+  __shared__ double red[7][8];
+  __shared__ bool last;
   const int chunk = (natoms + gridDim.x - 1) / gridDim.x;
-  const int b = blockIdx.x * chunk, en = min(natoms, b + chunk);
+  const int b = min(natoms, static_cast<int>(blockIdx.x) * chunk), en = min(natoms, b + chunk);
   double acc[7] = {0, 0, 0, 0, 0, 0, 0};
   for (int i = b + threadIdx.x; i < en; i += blockDim.x) {
     acc[0] += e[i];
     for (int c = 0; c < 6; ++c) acc[1 + c] += w[6 * i + c];
   }
-  for (int c = 0; c < 7; ++c) {
-    double s = block_reduce_256(acc[c], red);
-    if (threadIdx.x == 0) partials[7 * blockIdx.x + c] = s;
-  }
-}
-
-// One warp per total (7 warps): lane l adds partials l, l + 32, ... in order,
-// then a fixed butterfly over the lanes, so the order is the same on every
-// GPU and every run (a single thread walking all partials was a 256-add
-// dependent chain, 18 us of a 2,000-atom call).
-__global__ void k_final_totals(int nb, const double* __restrict__ partials, double* __restrict__ out) {
-  const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (c >= 7) return;   // whole warps leave
-  double s = 0.0;
-  for (int b = lane; b < nb; b += 32) s += partials[7 * b + c];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) out[c] = s;
+  for (int c = 0; c < 7; ++c) {
+    for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    if (lane == 0) red[c][warp] = acc[c];
+  }
+  __syncthreads();
+  if (threadIdx.x < 7) {
+    double s = 0.0;
+    for (int k = 0; k < 8; ++k) s += red[threadIdx.x][k];
+    partials[7 * blockIdx.x + threadIdx.x] = s;
+    __threadfence();
+  }
+  __syncthreads();
+  int* ticket = reinterpret_cast<int*>(out + 8);
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1) == static_cast<int>(gridDim.x) - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (warp < 7) {
+    double s = 0.0;
+    for (int k = lane; k < static_cast<int>(gridDim.x); k += 32) s += __ldcg(partials + 7 * k + warp);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) {
+      out[warp] = s;
+      if (warp == 0 && d_energy) *d_energy = s;
+      if (warp > 0 && d_virial) d_virial[warp - 1] = s;
+    }
+  } else if (lane == 0) {
+    out[7] = __hiloint2double(0, *reinterpret_cast<const volatile int*>(err));
+    *ticket = 0;
+  }
 }
 
 // Neighbour rows from positions, one warp per local atom: the candidates of
@@ -452,13 +518,8 @@ cudaError_t launch_rows_from_positions(int nlocal, int nall, const double* x, co
 }
 
 cudaError_t launch_totals(int natoms, const double* site_energy, const double* wown, double* partials,
-                          double* out, cudaStream_t st) {
-  if (natoms <= 0) {
-    cudaMemsetAsync(out, 0, 7 * sizeof(double), st);
-    return cudaGetLastError();
-  }
-  k_partial_totals<<<kReduceBlocks, 256, 0, st>>>(natoms, site_energy, wown, partials);
-  k_final_totals<<<1, 7 * 32, 0, st>>>(kReduceBlocks, partials, out);
+                          double* out, const int* err, double* d_energy, double* d_virial, cudaStream_t st) {
+  k_totals<<<kReduceBlocks, 256, 0, st>>>(natoms, site_energy, wown, partials, out, err, d_energy, d_virial);
   return cudaGetLastError();
 }
 

@@ -20,21 +20,24 @@ cudaError_t launch_eval(const DevModel& md, const DevIO& io, int threads, int bl
                         cudaStream_t st);
 
 // Incoming-slot lists: for every atom k, the slots (i, s) whose neighbour is k,
-// sorted by slot id.  in_ptr [natoms + 1].
+// in any order (launch_force_gather sorts them).  in_ptr [natoms + 1].
 cudaError_t launch_incoming(int natoms, int stride, const int* js, const int* jtypes, const int* counts,
-                            int* in_cnt, int* in_ptr, int* in_cursor, int* in_slot, int* block_tmp,
-                            cudaStream_t st);
+                            int* in_cnt, int* in_ptr, int* in_slot, int* block_tmp, cudaStream_t st);
 
 // forces[i] = own slot gradients - incoming slot gradients; wown [natoms][6]
 // = -sym(sum_s r_is (x) g_is) (LAMMPS order xx,yy,zz,xy,xz,yz); when vatom
-// is non-null it receives the half/half split of every pair's virial.
+// is non-null it receives the half/half split of every pair's virial.  `sort`:
+// the incoming lists are fresh and get sorted by slot id.
 cudaError_t launch_force_gather(int natoms, int stride, const double* rijs, const int* counts,
-                                const double* pair_grad, const int* in_ptr, const int* in_slot,
+                                const double* pair_grad, const int* in_ptr, int* in_slot, bool sort,
                                 double* forces, double* wown, double* vatom, cudaStream_t st);
 
 // out[0] = sum site_energy[0..natoms), out[1..6] = sum wown; fixed order.
+// out[7] = error flags; out [kTotals] holds a counter that is zero between
+// calls.  The totals also go to d_energy [1] and d_virial [6] where given.
+constexpr int kTotals = 9;
 cudaError_t launch_totals(int natoms, const double* site_energy, const double* wown, double* partials,
-                          double* out, cudaStream_t st);
+                          double* out, const int* err, double* d_energy, double* d_virial, cudaStream_t st);
 
 // Per-configuration energy [nconfig] and reference-convention stress [nconfig][6].
 cudaError_t launch_config_totals(int natoms, int nconfig, const int* cfg_ptr, const double* site_energy,

@@ -38,6 +38,25 @@ def test_sizes_at_the_edges_of_rounds(n):
         assert np.abs(out[key] - ref[key]).max() <= 1e-10 * np.abs(ref[key]).max(), key
 
 
+@pytest.mark.parametrize("n,stride,hub", [(1023, 4, False), (1025, 4, False), (8192, 3, False), (8193, 3, False),
+                                          (90, 12, True)])
+def test_incoming_lists(n, stride, hub):
+    """Sizes around the one-block scan's limits; with `hub` every slot points at
+    atom 0, a list too long to sort in registers."""
+    pot = read_mtp(potential_path(NAME))
+    it, r, js, jt, counts = _rows(n, stride)
+    if hub:
+        js[:] = 0
+    js[::7, 1] = n + 3                       # a neighbour without an owner: no reaction force
+    ref = CpuMTP(pot).compute(it, r, js, jt, counts)
+    with MTPEngine(potential_path(NAME), n, stride) as eng:
+        out = eng.compute(it, r, js, jt, counts)
+        again = eng.compute(it, r, js, jt, counts)
+    assert np.abs(out["forces"] - ref["forces"]).max() <= 1e-10 * np.abs(ref["forces"]).max()
+    assert np.array_equal(out["forces"], again["forces"])
+    assert abs(out["energy"] - ref["energy"]) <= 1e-10 * abs(ref["energy"])
+
+
 def test_capture_of_another_size():
     big, small = 2000, 100
     dev = torch.device("cuda")
