@@ -69,6 +69,7 @@ struct mtp_handle {
   int max_atoms = 0, max_nbr = 0, debug = 0, precision = 0;
   double cutoff = 0.0;
   int device = 0, sm_count = 0;
+  size_t l2_bytes = 0;
   cudaStream_t own_stream = nullptr, stream = nullptr;
   int threads = 0, blocks_per_sm = 0;   // requested launch (mtp_set_launch); 0 threads: automatic
   int last_threads = 0, last_blocks = 0, last_bps = 0;
@@ -371,7 +372,7 @@ double launch_estimate(const Potential& pot, bool fp64, int lanes, int A, int bp
 // Launch shape for the evaluation kernel on natoms: the (lanes, atoms per
 // block) within the handle's request with the least expected time
 // (launch_estimate) among those whose value space fits in shared memory; when
-// none fits, the value space moves to global memory (A = 1).
+// none fits, the value space moves to global memory (A = 1 or 2).
 // While the stream is being captured nothing can be uploaded, so a shape whose
 // programs are not on the device yet gives way to the best one whose are.
 int pick_launch(mtp_handle* h, long long natoms, int stride, const DeviceSchedule** ds_out, int* blocks_out, bool fp64,
@@ -395,14 +396,42 @@ int pick_launch(mtp_handle* h, long long natoms, int stride, const DeviceSchedul
   bool vglobal = false;
   if (best.lanes == 0) {
     // value space in global memory: 512 lanes give an SM 16 warps with one
-    // block, so the blocks' value spaces stay within L2
+    // block, so the blocks' value spaces stay within L2.  Two atoms share
+    // every program entry (4.5 MB an iteration at level 28, as much L2 traffic
+    // as the operands) and fill more of each 32-byte sector a gather touches:
+    // an iteration takes 1.78x (FP64, 2.20 -> 1.96 ms for 2,048 atoms) or
+    // 1.09x (FP32) one atom's time, so they win where that saves a round, as
+    // long as the value spaces stay in L2 (four atoms' do not: 3.47 ms).
     vglobal = true;
     best.lanes = 512;
-    const int st = launch_occupancy(h, best.lanes, stride, fp64, true, 1, &best.bps);
+    const DeviceSchedule* sz = nullptr;
+    int st = get_sizes(h, best.lanes, &sz);
     if (st != MTP_OK) return st;
+    double least = 0.0;
+    for (int A : {1, 2}) {
+      if (h->apb > 0 && A > h->apb) continue;
+      const size_t spaces = static_cast<size_t>(h->sm_count) * sz->sched.v_size * A * (fp64 ? sizeof(double) : sizeof(float));
+      if (A > 1 && spaces > h->l2_bytes / 4 * 3) continue;
+      int bps = 0;
+      st = launch_occupancy(h, best.lanes, stride, fp64, true, A, &bps);
+      if (st != MTP_OK) return st;
+      if (bps <= 0) continue;
+      const long long per = static_cast<long long>(A) * h->sm_count;
+      const double cost = static_cast<double>((natoms + per - 1) / per) * (A == 1 ? 1.0 : fp64 ? 1.78 : 1.09);
+      if (best.bps == 0 || cost < least) {
+        least = cost;
+        best.A = A;
+        best.bps = 1;
+      }
+    }
     if (best.bps <= 0)
       return fail(h, MTP_E_CAPACITY, "the evaluation block does not fit in shared memory for this basis and max_nbr");
-    best.bps = 1;
+    if (best.A > 1 && !schedule_uploaded(h, best.lanes, access_width(fp64, best.A)) &&
+        schedule_uploaded(h, best.lanes, access_width(fp64, 1))) {
+      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+      if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) cudaGetLastError();
+      if (cs != cudaStreamCaptureStatusNone) best.A = 1;
+    }
   } else if (ready.lanes > 0 && !schedule_uploaded(h, best.lanes, access_width(fp64, best.A))) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) cudaGetLastError();
@@ -414,7 +443,7 @@ int pick_launch(mtp_handle* h, long long natoms, int stride, const DeviceSchedul
   const long long groups = (natoms + best.A - 1) / best.A;
   const long long blocks = std::max(1LL, std::min<long long>(static_cast<long long>(best.bps) * h->sm_count, groups));
   if (vglobal) {
-    const size_t need = static_cast<size_t>(blocks) * ds->sched.v_size * (fp64 ? sizeof(double) : sizeof(float));
+    const size_t need = static_cast<size_t>(blocks) * ds->sched.v_size * best.A * (fp64 ? sizeof(double) : sizeof(float));
     if (need > h->vscratch_bytes) {
       if (h->d_vscratch) cudaFree(h->d_vscratch);
       h->d_vscratch = nullptr;
@@ -816,6 +845,9 @@ int mtp_create(const char* mtp_path, int max_atoms, int max_nbr, double cutoff, 
   };
   if (cudaGetDevice(&h->device) != cudaSuccess) return bail(cuda_fail(h, cudaGetLastError(), "cudaGetDevice"));
   cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, h->device);
+  int l2 = 0;
+  cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, h->device);
+  h->l2_bytes = static_cast<size_t>(l2);
   if (cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking) != cudaSuccess)
     return bail(cuda_fail(h, cudaGetLastError(), "cudaStreamCreate"));
   h->stream = h->own_stream;

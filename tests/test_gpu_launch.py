@@ -38,6 +38,22 @@ def test_sizes_at_the_edges_of_rounds(n):
         assert np.abs(out[key] - ref[key]).max() <= 1e-10 * np.abs(ref[key]).max(), key
 
 
+@pytest.mark.parametrize("n,apb", [(148, 1), (149, 2), (297, 1), (592, 2)])
+def test_value_space_in_global_memory(n, apb):
+    """Level 28 in FP64 does not fit in shared memory; one or two atoms share a
+    block by the number of rounds.  (148 SMs.)"""
+    name = "cfg4_L28_S4.mtp"
+    pot = read_mtp(potential_path(name))
+    rows = _rows(n)
+    ref = CpuMTP(pot).compute(*rows)
+    with MTPEngine(potential_path(name), n, 12) as eng:
+        out = eng.compute(*rows)
+        if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+            assert eng.launch()["atoms_per_block"] == apb
+    for key in ("site_energies", "forces", "virial"):
+        assert np.abs(out[key] - ref[key]).max() <= 1e-10 * np.abs(ref[key]).max(), key
+
+
 @pytest.mark.parametrize("n,stride,hub", [(1023, 4, False), (1025, 4, False), (8192, 3, False), (8193, 3, False),
                                           (90, 12, True)])
 def test_incoming_lists(n, stride, hub):
