@@ -1303,7 +1303,10 @@ int mtp_adjoint_batch_device(mtp_handle* h, int natoms, int stride, int nconfig,
   int st = get_sizes(h, lanes, &ds);
   if (st != MTP_OK) return st;
   if (lanes < 512 && !adjoint_fits_shared(make_model(h, *ds), stride, lanes)) lanes = 512;
-  st = get_schedule(h, lanes, access_width(true, 1), &ds);
+  // an operand is a value and its tangent, 16 bytes (also where the value space
+  // is in global memory: L1 serves a gather by the same banks; entries ordered
+  // for 8 bytes: level 28, 64 configurations 35.8 ms, for 16: 32.2 ms)
+  st = get_schedule(h, lanes, 2 * access_width(true, 1), &ds);
   if (st != MTP_OK) return st;
   DevModel md = make_model(h, *ds);
   TrainIO tio{};

@@ -143,7 +143,8 @@ __host__ __device__ inline int n3_group_warps(int NW, int A, int n_pad, int item
 template <typename T>
 __host__ __device__ inline int staging_stride(int n_pad) {
   // long rows are rounded less: their padding would cost more than the bank conflicts
-  return n_pad <= 256 ? ((n_pad + 31) & ~31) + kVec<T> : ((n_pad + 3) & ~3) + 4;
+  constexpr int line = 8 * kVec<T>;
+  return n_pad <= 256 ? (n_pad + line - 1 - kVec<T>) / line * line + kVec<T> : (n_pad + 3) & ~3;
 }
 
 template <typename T>

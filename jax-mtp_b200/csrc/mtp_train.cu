@@ -5,38 +5,56 @@
 
 namespace mtp {
 
+// Warps that share one chunk of neighbours in the last phase (one, with no
+// exchange, for long rows: their staging needs the room).
+__host__ __device__ inline int train_group_warps(int NW, int n_pad) {
+  return n_pad > 192 ? 1 : n3_group_warps(NW, 1, n_pad, 1);
+}
+
+// Shared-memory carve of the adjoint block (one atom).  Staging is rows over the
+// kept neighbours, as in the evaluation kernel: f_mu, f'_mu, phi_n, phi'_n, the
+// powers of u_x, u_y, u_z and the tangents of u and d; the radial sensitivities
+// of the last phase take the rows of f and f', which are dead by then.  The
+// exchange of that phase's partial sums takes the moment half of a value space
+// in shared memory (dead as well) where it fits there, and its adjoints are
+// read in place there (structured bases); otherwise they have their own
+// regions.
 struct TrainSmem {
-  int pws;
-  size_t v, rad, u, du, f, fp, phi, phip, pw, A, Bv, jt, gxi, grad, red, cnt, total;
+  int qs, rows;
+  int f, fp, phi, phip, pw, du, A, B;   // first row of each field (du: du_x, du_y, du_z, dd)
+  size_t v, rad, st, jt, mono, chain, part, gxi, grad, cnt, total;
 };
 
 template <typename T>
-__host__ __device__ inline TrainSmem train_layout(int v_size, int S, int R, int K, int P, int D, int Sa, int n_pad,
-                                                  int threads) {
+__host__ __device__ inline TrainSmem train_layout(const DevModel& md, bool vglobal, int n_pad, int threads) {
+  const int S = md.S, R = md.R, K = md.K, D = md.D;
   TrainSmem L;
-  L.pws = 3 * (D + 1);
-  if ((L.pws & 1) == 0) L.pws += 1;
+  L.qs = staging_stride<T>(n_pad);
+  L.f = 0;
+  L.fp = R;
+  L.phi = 2 * R;
+  L.phip = 2 * R + K;
+  L.pw = 2 * R + 2 * K;
+  L.du = L.pw + 3 * (D + 1);
+  L.rows = L.du + 4;
+  L.A = L.f;
+  L.B = L.fp;
   size_t o = 0;
   auto take = [&](size_t bytes) {
     size_t at = (o + 15) & ~size_t(15);
     o = at + bytes;
     return at;
   };
-  L.v = take(sizeof(T) * 2 * v_size);
+  L.v = take(vglobal ? 0 : sizeof(T) * 2 * md.v_size);
   L.rad = take(sizeof(T) * S * S * R * K);
-  L.u = take(sizeof(T) * 4 * n_pad);
-  L.du = take(sizeof(T) * 4 * n_pad);
-  L.f = take(sizeof(T) * R * n_pad);
-  L.fp = take(sizeof(T) * R * n_pad);
-  L.phi = take(sizeof(T) * K * n_pad);
-  L.phip = take(sizeof(T) * K * n_pad);
-  L.pw = take(sizeof(T) * L.pws * n_pad);
-  L.A = take(sizeof(T) * R * n_pad);
-  L.Bv = take(sizeof(T) * R * n_pad);
-  L.jt = take(sizeof(int) * n_pad);
+  L.st = take(sizeof(T) * L.rows * L.qs);
+  L.jt = take(sizeof(int) * L.qs);
+  L.mono = take(sizeof(int) * md.P + sizeof(uint16_t) * md.n_list);
+  L.chain = !vglobal && md.chain_mode >= 0 ? L.v + sizeof(T) * 2 * md.v_dm : take(2 * sizeof(T) * md.n3_len);
+  const size_t part = train_group_warps(threads / 32, n_pad) > 1 ? sizeof(T) * 2 * threads : 0;
+  L.part = !vglobal && part <= sizeof(T) * 2 * md.M ? L.v : take(part);
   L.gxi = take(sizeof(double) * S);
   L.grad = take(sizeof(double) * S * S * R * K);
-  L.red = take(sizeof(double) * (threads / 32));
   L.cnt = take(sizeof(int) * (threads / 32 + 1));
   L.total = (o + 15) & ~size_t(15);
   return L;
@@ -121,6 +139,120 @@ struct DualRevBody {
   }
 };
 
+// Basic moments and their tangents of one monomial for NM radial functions,
+// kVec neighbours per 16-byte load (rows are padded to that with f = f' = 0).
+template <int NM>
+__device__ __forceinline__ void dual_moments(const double* __restrict__ f, const double* __restrict__ fp, int qs,
+                                             const double* __restrict__ px, const double* __restrict__ py,
+                                             const double* __restrict__ pz, int ea, int eb, int ec,
+                                             const double* __restrict__ du, int nv, double (&acc)[kMaxR],
+                                             double (&tac)[kMaxR]) {
+  const double am = ea, bm = eb, cm = ec;
+  const double *px1 = px - (ea > 0 ? qs : 0), *py1 = py - (eb > 0 ? qs : 0), *pz1 = pz - (ec > 0 ? qs : 0);
+  auto two = [](const double* p) { return *reinterpret_cast<const double2*>(p); };
+  for (int q = 0; q < nv; q += 2) {
+    const double2 x = two(px + q), y = two(py + q), z = two(pz + q), x1 = two(px1 + q), y1 = two(py1 + q),
+                  z1 = two(pz1 + q);
+    const double2 dx = two(du + q), dy = two(du + qs + q), dz = two(du + 2 * qs + q), dd = two(du + 3 * qs + q);
+    const double xy0 = x.x * y.x, xy1 = x.y * y.y, m0 = xy0 * z.x, m1 = xy1 * z.y;
+    const double dm0 = fma(am * x1.x * dx.x, y.x * z.x, fma(bm * y1.x * dy.x, x.x * z.x, cm * z1.x * dz.x * xy0));
+    const double dm1 = fma(am * x1.y * dx.y, y.y * z.y, fma(bm * y1.y * dy.y, x.y * z.y, cm * z1.y * dz.y * xy1));
+    const double e0 = dd.x * m0, e1 = dd.y * m1;
+#pragma unroll
+    for (int mu = 0; mu < NM; ++mu) {
+      const double2 g = two(f + mu * qs + q), gp = two(fp + mu * qs + q);
+      acc[mu] = fma(g.x, m0, acc[mu]);
+      tac[mu] = fma(gp.x, e0, fma(g.x, dm0, tac[mu]));
+      acc[mu] = fma(g.y, m1, acc[mu]);
+      tac[mu] = fma(gp.y, e1, fma(g.y, dm1, tac[mu]));
+    }
+  }
+}
+
+// Radial sensitivities of the kept neighbours: with (lambda, tau) the dual
+// adjoints of the basic moments, GA_mu = sum_s lambda u^s + tau d(u^s) and
+// GB_mu = sum_s tau u^s over the monomials s of mu.  Lanes are neighbours and
+// the warps of a group split the monomial chains, as in the evaluation
+// kernel's force phase; a step reads its radial functions' (lambda, tau) one
+// after the other from the chain-ordered copy, 16 bytes each, the same for all
+// lanes.  (One thread per neighbour and share of the monomials, with the
+// tables and moment positions read from L2, took 30,000 of 76,000 cycles an
+// atom at level 20.)
+template <int R, int MODE>
+__device__ __forceinline__ void sensitivities(const DevModel& md, const TrainSmem& L, unsigned char* smem, int nv,
+                                              int n_pad, int tid, int NT) {
+  const int w = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, NW = NT >> 5;   // known to be warp-uniform
+  const int GW = train_group_warps(NW, n_pad), g = w / GW, wg = w - g * GW, NG = NW / GW;
+  const int lg = 31 - __clz(GW);
+  const int i0 = md.n3_off[GW - 1 + lg + wg], i1 = md.n3_off[GW + lg + wg];
+  const int D1 = md.D + 1, qs = L.qs;
+  double* part = reinterpret_cast<double*>(smem + L.part);
+  for (int r0 = 0; r0 < nv; r0 += 32 * NG) {
+    const int j = r0 + 32 * g + lane;
+    const bool act = j < nv;
+    double* st = reinterpret_cast<double*>(smem + L.st) + (act ? j : r0);
+    const double *px = st + L.pw * qs, *py = px + D1 * qs, *pz = py + D1 * qs, *du = st + L.du * qs;
+    const double dux = du[0], duy = du[qs], duz = du[2 * qs];
+    double GA[R], GB[R];
+#pragma unroll
+    for (int mu = 0; mu < R; ++mu) GA[mu] = GB[mu] = 0.0;
+    const int iend = r0 + 32 * g < nv ? i1 : i0;
+    for (int i = i0; i < iend; ++i) {
+      const int word = md.n3_words[i];
+      const int top = word & 15, ea = (word >> 4) & 15, eb = (word >> 8) & 15;
+      const double2* lt = reinterpret_cast<const double2*>(smem + L.chain) + (word >> 16) * 4;
+      const double xa = px[ea * qs], yb = py[eb * qs], xy = xa * yb;
+      const double dxy = ea * px[max(ea - 1, 0) * qs] * dux * yb + eb * py[max(eb - 1, 0) * qs] * duy * xa;
+      double cd = top;
+#pragma unroll
+      for (int k = 0; k <= kMaxDegree; ++k) {
+        if (k > top) break;
+        const double zc = pz[(top - k) * qs], zc1 = pz[max(top - k - 1, 0) * qs];
+        const double m = xy * zc, dm = fma(dxy, zc, xy * (cd * zc1) * duz);
+        cd -= 1.0;
+#pragma unroll
+        for (int mu = 0; mu < (MODE < 0 ? R : chain_nm<R, MODE < 0 ? 0 : MODE>(k)); ++mu) {
+          const double2 v = *lt++;
+          GA[mu] = fma(v.x, m, fma(v.y, dm, GA[mu]));
+          GB[mu] = fma(v.y, m, GB[mu]);
+        }
+      }
+    }
+    if (GW > 1) {
+      // one radial function at a time: with the value space in global memory,
+      // shared memory taken here is L1 taken from its gathers
+      double* mine = part + w * 32 + lane;
+#pragma unroll
+      for (int mu = 0; mu < R; ++mu) {
+        mine[0] = GA[mu];
+        mine[NT] = GB[mu];
+        __syncthreads();
+        if (wg == 0) {
+          for (int x = 1; x < GW; ++x) {
+            GA[mu] += mine[x * 32];
+            GB[mu] += mine[NT + x * 32];
+          }
+        }
+        __syncthreads();
+      }
+    }
+    if (wg == 0 && act) {
+      const double dd = du[3 * qs];
+#pragma unroll
+      for (int mu = 0; mu < R; ++mu) {
+        st[(L.A + mu) * qs] = GA[mu];
+        st[(L.B + mu) * qs] = dd * GB[mu];
+      }
+    }
+  }
+}
+
+// One thread's neighbour slot of an atom and the atom's own values.
+struct TrainSlot {
+  double x, y, z;
+  int jt, j, it, cfg, cnt;
+};
+
 template <typename T, bool kVGlobal>
 __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, int n_pad, void* vscratch,
                                                      double* partials) {
@@ -128,7 +260,7 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
   const int NT = blockDim.x, tid = threadIdx.x;
   const int my_wsteps = warp_steps_of_lane(md, tid, NT);
   const int S = md.S, R = md.R, K = md.K, P = md.P, D1 = md.D + 1;
-  const TrainSmem L = train_layout<T>(kVGlobal ? 0 : md.v_size, S, R, K, P, md.D, md.Sa, n_pad, NT);
+  const TrainSmem L = train_layout<T>(md, kVGlobal, n_pad, NT);
   using T2 = typename Dual2<T>::type;
   // program entries in flight per thread; with the value space in global
   // memory their operand gathers are issued before any of their flushes
@@ -138,34 +270,30 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
   T2* V = kVGlobal ? reinterpret_cast<T2*>(vscratch) + static_cast<size_t>(blockIdx.x) * md.v_size
                    : reinterpret_cast<T2*>(smem + L.v);
   T* sRad = reinterpret_cast<T*>(smem + L.rad);
-  T* sU = reinterpret_cast<T*>(smem + L.u);
-  T* sDu = reinterpret_cast<T*>(smem + L.du);
-  T* sF = reinterpret_cast<T*>(smem + L.f);
-  T* sFp = reinterpret_cast<T*>(smem + L.fp);
-  T* sPhi = reinterpret_cast<T*>(smem + L.phi);
-  T* sPhip = reinterpret_cast<T*>(smem + L.phip);
-  T* sPw = reinterpret_cast<T*>(smem + L.pw);
-  T* sA = reinterpret_cast<T*>(smem + L.A);
-  T* sB = reinterpret_cast<T*>(smem + L.Bv);
+  T* sSt = reinterpret_cast<T*>(smem + L.st);
   int* sJt = reinterpret_cast<int*>(smem + L.jt);
+  int* sMono = reinterpret_cast<int*>(smem + L.mono);
+  uint16_t* sList = reinterpret_cast<uint16_t*>(sMono + P);
+  T2* sChain = reinterpret_cast<T2*>(smem + L.chain);
   double* gXi = reinterpret_cast<double*>(smem + L.gxi);
   double* gRad = reinterpret_cast<double*>(smem + L.grad);
   int* sCnt = reinterpret_cast<int*>(smem + L.cnt);
-  const int pws = L.pws;
+  const int qs = L.qs;
   const int nrad = S * S * R * K;
   // this block's partial gradients [Sa | S | S*S*R*K]; the moment part is
   // accumulated here directly (each thread owns the same coefficients for
   // every atom), species and radial parts in shared memory
   double* out = partials + static_cast<size_t>(blockIdx.x) * (md.Sa + S + nrad);
-  const int4* mono_abc = reinterpret_cast<const int4*>(md.mono_abc);
 
   for (int x = tid; x < nrad; x += NT) {
     sRad[x] = static_cast<T>(md.radial[x]);
     gRad[x] = 0.0;
   }
+  for (int x = tid; x < P; x += NT) sMono[x] = md.mono_word[x];
+  for (int x = tid; x < md.n_list; x += NT) sList[x] = static_cast<uint16_t>(md.mono_list[x]);
   for (int x = tid; x < md.Sa; x += NT) out[x] = 0.0;
   for (int x = tid; x < S; x += NT) gXi[x] = 0.0;
-  for (int x = tid; x < md.nzero; x += NT) V[md.v_m + md.zero_list[x]] = Dual2<T>::make(T(0), T(0));
+  for (int x = tid; x < md.ndm_zero; x += NT) V[md.v_dm + md.dm_zero[x]] = Dual2<T>::make(T(0), T(0));
   if (tid == 0) {
     V[md.v_zero] = Dual2<T>::make(T(0), T(0));
     V[md.v_one] = Dual2<T>::make(T(1), T(0));
@@ -174,15 +302,34 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
   const T inv_range = static_cast<T>(1.0 / (md.rmax - md.rmin));
   const T rsum = static_cast<T>(md.rmin + md.rmax);
   const T scal = static_cast<T>(md.scaling);
+  auto load_slot = [&](int atom, int s) {
+    TrainSlot r{0.0, 0.0, 0.0, -1, -1, 0, 0, 0};
+    if (atom < io.natoms) {
+      r.it = __ldg(io.itypes + atom);
+      r.cfg = __ldg(io.cfg + atom);
+      r.cnt = io.counts ? __ldg(io.counts + atom) : io.nbr_stride;
+      if (s < io.nbr_stride) {
+        const size_t x = static_cast<size_t>(atom) * io.nbr_stride + s;
+        r.jt = __ldg(io.jtypes + x);
+        r.j = __ldg(io.js + x);
+        r.x = __ldg(io.rijs + 3 * x);
+        r.y = __ldg(io.rijs + 3 * x + 1);
+        r.z = __ldg(io.rijs + 3 * x + 2);
+      }
+    }
+    return r;
+  };
   __syncthreads();
 
+  // the next atom's slots are loaded before the last phases of this one
+  TrainSlot ahead = load_slot(blockIdx.x, tid);
   for (int atom = blockIdx.x; atom < io.natoms; atom += gridDim.x) {
-    int it = __ldg(io.itypes + atom);
+    int it = ahead.it;
     if (it < 0 || it >= S) {
       if (tid == 0) atomicOr(io.err, kErrSpecies);
       it = 0;
     }
-    int cfg = __ldg(io.cfg + atom);
+    int cfg = ahead.cfg;
     if (cfg < 0 || cfg >= io.nconfig) {
       if (tid == 0) atomicOr(io.err, kErrCapacity);
       cfg = 0;
@@ -196,26 +343,32 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
     const T c01 = static_cast<T>(0.5 * gs[5] * iv);
     const T gfx = static_cast<T>(__ldg(io.gF + 3 * atom)), gfy = static_cast<T>(__ldg(io.gF + 3 * atom + 1)),
             gfz = static_cast<T>(__ldg(io.gF + 3 * atom + 2));
-    int cnt = io.counts ? __ldg(io.counts + atom) : io.nbr_stride;
+    int cnt = ahead.cnt;
     if (cnt > n_pad || cnt < 0) {
       if (tid == 0) atomicOr(io.err, kErrCapacity);
       cnt = cnt < 0 ? 0 : n_pad;
     }
-    const size_t row = static_cast<size_t>(atom) * io.nbr_stride;
+    // (the exchange of the last phase may have used these slots)
+    for (int x = tid; x < md.nzero; x += NT) V[md.v_m + md.zero_list[x]] = Dual2<T>::make(T(0), T(0));
+    for (int x = tid; x < md.nseed; x += NT) {
+      const T sv = static_cast<T>(md.seed_val[x]);
+      V[md.v_dm + md.seed_idx[x]] = Dual2<T>::make(a_i * sv, sv);
+    }
 
     // ---- N1: stage neighbours with their tangents -------------------------
     int nv = 0;
     for (int s0 = 0; s0 < io.nbr_stride; s0 += NT) {
       const int s = s0 + tid;
+      const TrainSlot row = s0 == 0 ? ahead : load_slot(atom, s);
       bool valid = false;
       T rx = T(0), ry = T(0), rz = T(0), d = T(0);
       int jt = -1, j = -1;
-      if (s < cnt) {
-        jt = __ldg(io.jtypes + row + s);
-        j = __ldg(io.js + row + s);
-        rx = static_cast<T>(__ldg(io.rijs + 3 * (row + s)));
-        ry = static_cast<T>(__ldg(io.rijs + 3 * (row + s) + 1));
-        rz = static_cast<T>(__ldg(io.rijs + 3 * (row + s) + 2));
+      if (s < io.nbr_stride && s < cnt) {
+        jt = row.jt;
+        j = row.j;
+        rx = static_cast<T>(row.x);
+        ry = static_cast<T>(row.y);
+        rz = static_cast<T>(row.z);
         if (jt >= S) {
           atomicOr(io.err, kErrSpecies);
           jt = -1;
@@ -228,18 +381,12 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
       const int w = tid >> 5, l = tid & 31;
       if (l == 0) sCnt[w] = __popc(bal);
       __syncthreads();
-      if (tid == 0) {
-        int acc = 0;
-        for (int i = 0; i < (NT >> 5); ++i) {
-          int c = sCnt[i];
-          sCnt[i] = acc;
-          acc += c;
-        }
-        sCnt[NT >> 5] = acc;
-      }
-      __syncthreads();
+      const int wc = l < (NT >> 5) ? sCnt[l] : 0;
+      const int before = __reduce_add_sync(0xffffffffu, l < w ? wc : 0);
+      const int all = __reduce_add_sync(0xffffffffu, wc);
       if (valid) {
-        const int q = nv + sCnt[w] + __popc(bal & ((1u << l) - 1u));
+        const int q = nv + before + __popc(bal & ((1u << l) - 1u));
+        T* st = sSt + q;
         const T inv_d = T(1) / d;
         const T ux = rx * inv_d, uy = ry * inv_d, uz = rz * inv_d;
         // direction of the neighbour vector: force part + stress part
@@ -253,14 +400,10 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
         dry += c01 * rx + c11 * ry + c12 * rz;
         drz += c02 * rx + c12 * ry + c22 * rz;
         const T dd = ux * drx + uy * dry + uz * drz;
-        sU[4 * q] = ux;
-        sU[4 * q + 1] = uy;
-        sU[4 * q + 2] = uz;
-        sU[4 * q + 3] = d;
-        sDu[4 * q] = (drx - ux * dd) * inv_d;
-        sDu[4 * q + 1] = (dry - uy * dd) * inv_d;
-        sDu[4 * q + 2] = (drz - uz * dd) * inv_d;
-        sDu[4 * q + 3] = dd;
+        st[L.du * qs] = (drx - ux * dd) * inv_d;
+        st[(L.du + 1) * qs] = (dry - uy * dd) * inv_d;
+        st[(L.du + 2) * qs] = (drz - uz * dd) * inv_d;
+        st[(L.du + 3) * qs] = dd;
         sJt[q] = jt;
         const T x = (T(2) * d - rsum) * inv_range;
         const T dxdd = T(2) * inv_range;
@@ -275,8 +418,8 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
         }
         T t_prev = T(0), t_cur = T(1), dt_prev = T(0), dt_cur = T(0);
         for (int n = 0; n < K; ++n) {
-          sPhi[q * K + n] = scal * smooth * t_cur;
-          sPhip[q * K + n] = scal * (T(-2) * gap * t_cur + smooth * dt_cur * dxdd);
+          st[(L.phi + n) * qs] = scal * smooth * t_cur;
+          st[(L.phip + n) * qs] = scal * (T(-2) * gap * t_cur + smooth * dt_cur * dxdd);
 #pragma unroll
           for (int mu = 0; mu < kMaxR; ++mu) {
             if (mu < R) {
@@ -300,68 +443,61 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
 #pragma unroll
         for (int mu = 0; mu < kMaxR; ++mu) {
           if (mu < R) {
-            sF[q * R + mu] = scal * smooth * base[mu];
-            sFp[q * R + mu] = scal * (T(-2) * gap * base[mu] + smooth * dbase[mu] * dxdd);
+            st[(L.f + mu) * qs] = scal * smooth * base[mu];
+            st[(L.fp + mu) * qs] = scal * (T(-2) * gap * base[mu] + smooth * dbase[mu] * dxdd);
           }
         }
-        T* pw = sPw + q * pws;
+        T* pw = st + L.pw * qs;
         T px = T(1), py = T(1), pz = T(1);
         for (int e = 0; e < D1; ++e) {
-          pw[e] = px;
-          pw[D1 + e] = py;
-          pw[2 * D1 + e] = pz;
+          pw[e * qs] = px;
+          pw[(D1 + e) * qs] = py;
+          pw[(2 * D1 + e) * qs] = pz;
           px *= ux;
           py *= uy;
           pz *= uz;
         }
       }
-      nv += sCnt[NT >> 5];
-      __syncthreads();
+      nv += all;
+      if (s0 + NT < io.nbr_stride) __syncthreads();   // the next sweep overwrites the counts
     }
+    // rows end at a whole 16-byte word: the slot past an odd count adds nothing
+    // (all rows zero, the species one that no gradient matches)
+    if (nv & 1) {
+      for (int r = tid; r < L.rows; r += NT) sSt[r * qs + nv] = T(0);
+      if (tid == 0) sJt[nv] = -1;
+    }
+    __syncthreads();
 
     // ---- N2: basic moments and their tangents ------------------------------
-    for (int p = tid; p < P; p += NT) {
-      const int4 abc = __ldg(mono_abc + p);
-      const int a = abc.x, b = abc.y, cc = abc.z;
-      const T am = static_cast<T>(a), bm = static_cast<T>(b), cm = static_cast<T>(cc);
+    // most radial functions first, one count per warp (Schedule::mono_word)
+    for (int t0 = 0; t0 < P; t0 += NT) {
+      const bool act = t0 + tid < P;
+      const int word = sMono[act ? P - 1 - (t0 + tid) : 0];
+      const int nm = __reduce_max_sync(0xffffffffu, act ? word >> 12 & 15 : 0);
+      const int ea = word & 15, eb = word >> 4 & 15, ec = word >> 8 & 15;
+      const T* px = sSt + (L.pw + ea) * qs;
+      const T* py = sSt + (L.pw + D1 + eb) * qs;
+      const T* pz = sSt + (L.pw + 2 * D1 + ec) * qs;
       T acc[kMaxR], tac[kMaxR];
 #pragma unroll
-      for (int mu = 0; mu < kMaxR; ++mu) {
-        acc[mu] = T(0);
-        tac[mu] = T(0);
+      for (int mu = 0; mu < kMaxR; ++mu) acc[mu] = tac[mu] = T(0);
+      switch (nm) {
+        case 0: break;
+#define MTP_DUAL(NM) \
+  case NM: dual_moments<NM>(sSt + L.f * qs, sSt + L.fp * qs, qs, px, py, pz, ea, eb, ec, sSt + L.du * qs, nv, acc, tac); break;
+        MTP_DUAL(1) MTP_DUAL(2) MTP_DUAL(3) MTP_DUAL(4) MTP_DUAL(5) MTP_DUAL(6) MTP_DUAL(7) MTP_DUAL(8)
+#undef MTP_DUAL
+        default: break;
       }
-      for (int q = 0; q < nv; ++q) {
-        const T* pw = sPw + q * pws;
-        const T px = pw[a], py = pw[D1 + b], pz = pw[2 * D1 + cc];
-        const T mono = px * py * pz;
-        const T* du = sDu + 4 * q;
-        const T dmono = am * pw[a > 0 ? a - 1 : 0] * py * pz * du[0] +
-                        bm * px * pw[D1 + (b > 0 ? b - 1 : 0)] * pz * du[1] +
-                        cm * px * py * pw[2 * D1 + (cc > 0 ? cc - 1 : 0)] * du[2];
-        const T dmd = du[3] * mono;
+      if (act) {
+        const uint16_t* k = sList + (static_cast<unsigned>(word) >> 16);
 #pragma unroll
-        for (int mu = 0; mu < kMaxR; ++mu) {
-          if (mu < R) {
-            const T f = sF[q * R + mu];
-            acc[mu] = dev_fma(f, mono, acc[mu]);
-            tac[mu] = dev_fma(sFp[q * R + mu], dmd, dev_fma(f, dmono, tac[mu]));
-          }
-        }
-      }
-#pragma unroll
-      for (int mu = 0; mu < kMaxR; ++mu) {
-        if (mu < R) {
-          const int k = __ldg(md.mono_k + kMaxR * p + mu);
-          if (k >= 0) V[md.v_m + k] = Dual2<T>::make(acc[mu], tac[mu]);
-        }
+        for (int mu = 0; mu < kMaxR; ++mu)
+          if (mu < (word >> 12 & 15) && k[mu] != 0xFFFFu) V[md.v_m + k[mu]] = Dual2<T>::make(acc[mu], tac[mu]);
       }
     }
-    for (int x = tid; x < md.n_dm; x += NT) V[md.v_dm + x] = Dual2<T>::make(T(0), T(0));
     __syncthreads();
-    for (int x = tid; x < md.nseed; x += NT) {
-      const T sv = static_cast<T>(md.seed_val[x]);
-      V[md.v_dm + md.seed_idx[x]] = Dual2<T>::make(a_i * sv, sv);
-    }
 
     // ---- dual forward tree --------------------------------------------------
     for (int ps = 0; ps < md.nfwd; ++ps) {
@@ -370,9 +506,20 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
                                                __shfl_sync(0xFFFFFFFFu, my_wsteps, ps), NT, tid, body);
       __syncthreads();
     }
-    for (int a = tid; a < md.Sa; a += NT) {
-      const T2 v = V[md.v_m + __ldg(md.mapping + a)];
-      out[a] += static_cast<double>(a_i) * static_cast<double>(v.x) + static_cast<double>(v.y);
+    // four coefficients at a time, so that their loads overlap
+    for (int a0 = tid; a0 < md.Sa; a0 += 4 * NT) {
+      T2 v[4];
+      double o[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (a0 + k * NT < md.Sa) {
+          v[k] = V[md.v_m + __ldg(md.mapping + a0 + k * NT)];
+          o[k] = out[a0 + k * NT];
+        }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (a0 + k * NT < md.Sa)
+          out[a0 + k * NT] = o[k] + (static_cast<double>(a_i) * static_cast<double>(v[k].x) + static_cast<double>(v[k].y));
     }
     if (tid == 0) gXi[it] += static_cast<double>(a_i);
 
@@ -385,73 +532,48 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
     }
 
     // ---- N3: per-neighbour radial sensitivities ------------------------------
-    {
-      int tpn = 32;
-      while (tpn > 1 && tpn * nv > NT) tpn >>= 1;
-      const int total = nv * tpn;
-      for (int base = 0; base < total; base += NT) {
-        const int idx = base + tid;
-        const bool active = idx < total;
-        const int q = active ? idx / tpn : 0;
-        const int sl = idx & (tpn - 1);
-        T GA[kMaxR], GB[kMaxR];
-#pragma unroll
-        for (int mu = 0; mu < kMaxR; ++mu) {
-          GA[mu] = T(0);
-          GB[mu] = T(0);
-        }
-        if (active) {
-          const T* pw = sPw + q * pws;
-          const T* du = sDu + 4 * q;
-          for (int p = sl; p < P; p += tpn) {
-            const int4 abc = __ldg(mono_abc + p);
-            const int a = abc.x, b = abc.y, cc = abc.z;
-            const T px = pw[a], py = pw[D1 + b], pz = pw[2 * D1 + cc];
-            const T mono = px * py * pz;
-            const T dmono = static_cast<T>(a) * pw[a > 0 ? a - 1 : 0] * py * pz * du[0] +
-                            static_cast<T>(b) * px * pw[D1 + (b > 0 ? b - 1 : 0)] * pz * du[1] +
-                            static_cast<T>(cc) * px * py * pw[2 * D1 + (cc > 0 ? cc - 1 : 0)] * du[2];
-#pragma unroll
-            for (int mu = 0; mu < kMaxR; ++mu) {
-              if (mu < R) {
-                const int k = __ldg(md.mono_k + kMaxR * p + mu);
-                if (k >= 0) {
-                  const T2 lt = V[md.v_dm + __ldg(md.dm_pos + k)];   // (lambda, tau)
-                  GA[mu] = dev_fma(lt.x, mono, dev_fma(lt.y, dmono, GA[mu]));
-                  GB[mu] = dev_fma(lt.y, mono, GB[mu]);
-                }
-              }
-            }
-          }
-        }
-        for (int o = tpn >> 1; o > 0; o >>= 1) {
-#pragma unroll
-          for (int mu = 0; mu < kMaxR; ++mu) {
-            GA[mu] += __shfl_xor_sync(0xffffffffu, GA[mu], o);
-            GB[mu] += __shfl_xor_sync(0xffffffffu, GB[mu], o);
-          }
-        }
-        if (active && sl == 0) {
-          const T dd = sDu[4 * q + 3];
-#pragma unroll
-          for (int mu = 0; mu < kMaxR; ++mu) {
-            if (mu < R) {
-              sA[q * R + mu] = GA[mu];
-              sB[q * R + mu] = dd * GB[mu];
-            }
-          }
-        }
+    const bool in_place = !kVGlobal && md.chain_mode >= 0;
+    for (int x = tid; x < (in_place ? 0 : md.n3_len); x += NT) {
+      const int k = md.chain_mode >= 0 ? x : __ldg(md.n3_src + x);   // structured: placed in chain order
+      sChain[x] = k >= 0 ? V[md.v_dm + k] : Dual2<T>::make(T(0), T(0));
+    }
+    ahead = load_slot(atom + gridDim.x, tid);
+    __syncthreads();
+#define MTP_SENS(RR, MODE) \
+  case RR: sensitivities<RR, MODE>(md, L, smem, nv, n_pad, tid, NT); break;
+    if (md.chain_mode == 0) {
+      switch (R) {
+        MTP_SENS(1, 0) MTP_SENS(2, 0) MTP_SENS(3, 0) MTP_SENS(4, 0) MTP_SENS(5, 0) MTP_SENS(6, 0) MTP_SENS(7, 0)
+        MTP_SENS(8, 0)
+        default: break;
+      }
+    } else if (md.chain_mode == 1) {
+      sensitivities<6, 1>(md, L, smem, nv, n_pad, tid, NT);
+    } else if (md.chain_mode == 2) {
+      sensitivities<6, 2>(md, L, smem, nv, n_pad, tid, NT);
+    } else {
+      switch (R) {
+        MTP_SENS(1, -1) MTP_SENS(2, -1) MTP_SENS(3, -1) MTP_SENS(4, -1) MTP_SENS(5, -1) MTP_SENS(6, -1)
+        MTP_SENS(7, -1) MTP_SENS(8, -1)
+        default: break;
       }
     }
+#undef MTP_SENS
     __syncthreads();
-    // ---- N4: radial coefficient gradient, one thread per (mu, n) -------------
-    for (int x = tid; x < R * K; x += NT) {
-      const int mu = x / K, n = x % K;
-      for (int q = 0; q < nv; ++q) {
-        const double g = static_cast<double>(sA[q * R + mu]) * static_cast<double>(sPhi[q * K + n]) +
-                         static_cast<double>(sB[q * R + mu]) * static_cast<double>(sPhip[q * K + n]);
-        gRad[((it * S + sJt[q]) * R + mu) * K + n] += g;
+    // ---- N4: radial coefficient gradient, one thread per (species, mu, n) ----
+    for (int x = tid; x < S * R * K; x += NT) {
+      const int jt = x / (R * K), mu = x / K % R, n = x % K;
+      const T *pa = sSt + (L.A + mu) * qs, *pb = sSt + (L.B + mu) * qs, *pf = sSt + (L.phi + n) * qs,
+              *pg = sSt + (L.phip + n) * qs;
+      double g = 0.0;
+      for (int q = 0; q < nv; q += 2) {
+        const double2 a = *reinterpret_cast<const double2*>(pa + q), b = *reinterpret_cast<const double2*>(pb + q),
+                      f = *reinterpret_cast<const double2*>(pf + q), h = *reinterpret_cast<const double2*>(pg + q);
+        const int2 t = *reinterpret_cast<const int2*>(sJt + q);
+        if (t.x == jt) g += a.x * f.x + b.x * h.x;
+        if (t.y == jt) g += a.y * f.y + b.y * h.y;
       }
+      gRad[((it * S + jt) * R + mu) * K + n] += g;
     }
     __syncthreads();
   }
@@ -460,14 +582,24 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
   for (int x = tid; x < nrad; x += NT) out[md.Sa + S + x] = gRad[x];
 }
 
+// Sum of the blocks' partials in a fixed order: a block takes 32 gradients,
+// its warp w adds the partials of blocks w, w + 8, .. and the eight sums are
+// added in warp order (one thread walking all blocks' partials was a chain of
+// a few hundred L2 loads).
 __global__ void k_adjoint_reduce(int nblocks, int Sa, int S, int nrad, const double* __restrict__ partials,
                                  double* __restrict__ gmoment, double* __restrict__ gspecies,
                                  double* __restrict__ gradial) {
-  const int np = Sa + S + nrad;
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= np) return;
+  __shared__ double sum[8][32];
+  const int np = Sa + S + nrad, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int x = blockIdx.x * 32 + lane;
   double s = 0.0;
-  for (int b = 0; b < nblocks; ++b) s += partials[static_cast<size_t>(b) * np + x];
+  if (x < np)
+#pragma unroll 8
+    for (int b = w; b < nblocks; b += 8) s += partials[static_cast<size_t>(b) * np + x];
+  sum[w][lane] = s;
+  __syncthreads();
+  if (w > 0 || x >= np) return;
+  for (int k = 1; k < 8; ++k) s += sum[k][lane];
   if (x < Sa) gmoment[x] = s;
   else if (x < Sa + S) gspecies[x - Sa] = s;
   else gradial[x - Sa - S] = s;
@@ -505,7 +637,7 @@ static int adjoint_occupancy(size_t bytes, int threads) {
 }
 
 bool adjoint_fits_shared(const DevModel& md, int n_pad, int threads) {
-  const TrainSmem L = train_layout<double>(md.v_size, md.S, md.R, md.K, md.P, md.D, md.Sa, n_pad, threads);
+  const TrainSmem L = train_layout<double>(md, false, n_pad, threads);
   return adjoint_occupancy<false>(L.total, threads) > 0;
 }
 
@@ -515,11 +647,11 @@ cudaError_t launch_adjoint(const DevModel& md, const TrainIO& io, int threads, i
   const int nrad = md.S * md.S * md.R * md.K;
   const int np = md.Sa + md.S + nrad;
   bool vglobal = false;
-  TrainSmem L = train_layout<double>(md.v_size, md.S, md.R, md.K, md.P, md.D, md.Sa, n_pad, threads);
+  TrainSmem L = train_layout<double>(md, false, n_pad, threads);
   int bps = adjoint_occupancy<false>(L.total, threads);
   if (bps <= 0) {
     vglobal = true;
-    L = train_layout<double>(0, md.S, md.R, md.K, md.P, md.D, md.Sa, n_pad, threads);
+    L = train_layout<double>(md, true, n_pad, threads);
     bps = adjoint_occupancy<true>(L.total, threads);
   }
   if (bps <= 0) {
@@ -562,7 +694,7 @@ cudaError_t launch_adjoint(const DevModel& md, const TrainIO& io, int threads, i
       k_mtp_adjoint<double, false><<<blocks, threads, L.total, st>>>(md, io, n_pad, ws.vscratch, ws.partials);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    k_adjoint_reduce<<<(np + 255) / 256, 256, 0, st>>>(blocks, md.Sa, md.S, nrad, ws.partials, gmoment, gspecies,
+    k_adjoint_reduce<<<(np + 31) / 32, 256, 0, st>>>(blocks, md.Sa, md.S, nrad, ws.partials, gmoment, gspecies,
                                                       gradial);
   } else {
     cudaMemsetAsync(gmoment, 0, md.Sa * sizeof(double), st);
