@@ -80,7 +80,11 @@ struct mtp_handle {
   std::map<int, DeviceSchedule> scheds;
   std::map<int, DeviceSchedule> sizes;   // by lanes: schedules without programs, to size launches
   // potential tables on the device
-  double *d_radial = nullptr, *d_species = nullptr, *d_theta = nullptr, *d_seed_val = nullptr;
+  // coefficients: radial, species, theta and the seeds' values in one buffer,
+  // sent by one copy from its page-locked image
+  double *d_coef = nullptr, *h_coef = nullptr;
+  double *d_radial = nullptr, *d_species = nullptr, *d_theta = nullptr, *d_seed_val = nullptr;   // parts of d_coef
+  std::vector<int> seed_of;    // [Sa] seed that each mapped moment adds to
   int *d_mapping = nullptr, *d_seed_idx = nullptr, *d_zero = nullptr, *d_abc = nullptr, *d_mk = nullptr;
   // tables that are the same for every schedule of the potential
   int *d_dm_pos = nullptr, *d_dm_zero = nullptr, *d_n3_src = nullptr;
@@ -283,21 +287,19 @@ int get_schedule(mtp_handle* h, int lanes, int width, const DeviceSchedule** out
   return MTP_OK;
 }
 
+// Send the coefficients after the work already on the handle's stream, and wait
+// for them: later work sees them on any stream, graph replays included.
 int upload_coeffs(mtp_handle* h) {
   const Potential& p = h->pot;
-  MTP_CUDA(h, cudaMemcpy(h->d_radial, p.radial.data(), p.radial.size() * sizeof(double), cudaMemcpyHostToDevice));
-  MTP_CUDA(h, cudaMemcpy(h->d_species, p.species.data(), p.species.size() * sizeof(double), cudaMemcpyHostToDevice));
-  MTP_CUDA(h, cudaMemcpy(h->d_theta, p.moment.data(), p.moment.size() * sizeof(double), cudaMemcpyHostToDevice));
-  std::vector<int> si;
-  std::vector<double> sv;
-  seed_list(p, si, sv);
-  // seeds go to the adjoint positions of their moments
-  std::vector<int> dm_pos;
-  adjoint_layout(p, dm_pos);
-  for (int& k : si) k = dm_pos[k];
-  h->nseed = static_cast<int>(si.size());
-  MTP_CUDA(h, cudaMemcpy(h->d_seed_idx, si.data(), si.size() * sizeof(int), cudaMemcpyHostToDevice));
-  MTP_CUDA(h, cudaMemcpy(h->d_seed_val, sv.data(), sv.size() * sizeof(double), cudaMemcpyHostToDevice));
+  double* o = h->h_coef;
+  o = std::copy(p.radial.begin(), p.radial.end(), o);
+  o = std::copy(p.species.begin(), p.species.end(), o);
+  o = std::copy(p.moment.begin(), p.moment.end(), o);
+  std::fill(o, o + h->nseed, 0.0);
+  for (int a = 0; a < p.Sa; ++a) o[h->seed_of[a]] += p.moment[a];
+  const size_t n = (o - h->h_coef) + h->nseed;
+  MTP_CUDA(h, cudaMemcpyAsync(h->d_coef, h->h_coef, n * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  MTP_CUDA(h, cudaStreamSynchronize(h->stream));
   return MTP_OK;
 }
 
@@ -308,7 +310,8 @@ void free_handle(mtp_handle* h) {
     F(kv.second.d_entries);
     F(kv.second.d_warp_steps);
   }
-  F(h->d_radial); F(h->d_species); F(h->d_theta); F(h->d_seed_val);
+  F(h->d_coef);
+  if (h->h_coef) cudaFreeHost(h->h_coef);
   F(h->d_mapping); F(h->d_seed_idx); F(h->d_zero); F(h->d_abc); F(h->d_mk); F(h->d_dm_pos);
   F(h->d_dm_zero); F(h->d_n3_src);
   F(h->d_mono_word); F(h->d_mono_list);
@@ -853,9 +856,9 @@ int mtp_create(const char* mtp_path, int max_atoms, int max_nbr, double cutoff, 
   h->stream = h->own_stream;
   const Potential& p = h->pot;
   const size_t N = static_cast<size_t>(max_atoms), NS = N * max_nbr;
-  bool ok = dalloc(&h->d_radial, p.radial.size()) == cudaSuccess && dalloc(&h->d_species, p.S) == cudaSuccess &&
-            dalloc(&h->d_theta, p.Sa) == cudaSuccess && dalloc(&h->d_mapping, p.Sa) == cudaSuccess &&
-            dalloc(&h->d_seed_idx, p.Sa) == cudaSuccess && dalloc(&h->d_seed_val, p.Sa) == cudaSuccess &&
+  const size_t ncoef = p.radial.size() + p.S + 2 * static_cast<size_t>(p.Sa);
+  bool ok = dalloc(&h->d_coef, ncoef) == cudaSuccess && dalloc(&h->d_mapping, p.Sa) == cudaSuccess &&
+            dalloc(&h->d_seed_idx, p.Sa) == cudaSuccess &&
             dalloc(&h->d_itypes, N) == cudaSuccess && dalloc(&h->d_js, NS) == cudaSuccess &&
             dalloc(&h->d_jtypes, NS) == cudaSuccess && dalloc(&h->d_counts, N) == cudaSuccess &&
             dalloc(&h->d_rijs, 3 * NS) == cudaSuccess && dalloc(&h->d_G, 3 * NS) == cudaSuccess &&
@@ -871,7 +874,8 @@ int mtp_create(const char* mtp_path, int max_atoms, int max_nbr, double cutoff, 
     h->err = "device allocation failed for the requested capacities";
     return bail(MTP_E_OOM);
   }
-  if (cudaMallocHost(&h->h_tot, 8 * sizeof(double)) != cudaSuccess) {
+  if (cudaMallocHost(&h->h_tot, 8 * sizeof(double)) != cudaSuccess ||
+      cudaMallocHost(&h->h_coef, std::max<size_t>(ncoef, 1) * sizeof(double)) != cudaSuccess) {
     h->err = "pinned host allocation failed";
     return bail(MTP_E_OOM);
   }
@@ -880,6 +884,24 @@ int mtp_create(const char* mtp_path, int max_atoms, int max_nbr, double cutoff, 
   cudaMemset(h->d_tot, 0, kTotals * sizeof(double));
   if (cudaMemcpy(h->d_mapping, p.mapping.data(), p.Sa * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
     return bail(cuda_fail(h, cudaGetLastError(), "upload mapping"));
+  h->d_radial = h->d_coef;
+  h->d_species = h->d_radial + p.radial.size();
+  h->d_theta = h->d_species + p.S;
+  h->d_seed_val = h->d_theta + p.Sa;
+  {
+    // seeds of the reverse pass: the mapped moments, at their adjoint positions
+    std::vector<int> si, dm_pos;
+    std::vector<double> sv;
+    seed_list(p, si, sv);
+    adjoint_layout(p, dm_pos);
+    h->nseed = static_cast<int>(si.size());
+    std::map<int, int> seed;
+    for (int k = 0; k < h->nseed; ++k) seed[si[k]] = k;
+    for (int m : p.mapping) h->seed_of.push_back(seed[m]);
+    for (int& k : si) k = dm_pos[k];
+    if (cudaMemcpy(h->d_seed_idx, si.data(), si.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
+      return bail(cuda_fail(h, cudaGetLastError(), "upload seeds"));
+  }
   int st = upload_coeffs(h);
   if (st != MTP_OK) return bail(st);
   const DeviceSchedule* ds = nullptr;
@@ -938,11 +960,15 @@ int mtp_get_stats(const mtp_handle* h, double* out4) {
 
 int mtp_set_coeffs(mtp_handle* h, const double* species, const double* moment, const double* radial) {
   if (!h) return MTP_E_INVALID;
+  // inside a stream capture the copy would only be recorded (and read the
+  // image at every replay): refused, as the synchronisation is there
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  MTP_CUDA(h, cudaStreamIsCapturing(h->stream, &cs));
+  if (cs != cudaStreamCaptureStatusNone) MTP_CUDA(h, cudaStreamSynchronize(h->stream));
   Potential& p = h->pot;
   if (species) std::copy(species, species + p.S, p.species.begin());
   if (moment) std::copy(moment, moment + p.Sa, p.moment.begin());
   if (radial) std::copy(radial, radial + p.radial.size(), p.radial.begin());
-  MTP_CUDA(h, cudaStreamSynchronize(h->stream));
   ++h->gen;
   return upload_coeffs(h);
 }

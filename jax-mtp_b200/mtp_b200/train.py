@@ -77,18 +77,30 @@ class DeviceBatch:
             jtypes=torch.cat([self.jtypes, torch.full((N, pad), -1, dtype=self.jtypes.dtype, device=dev)], 1))
 
 
+def _host_coeffs(*tensors):
+    """The tensors as FP64 host arrays, by one copy where they share a device
+    (each copy from the GPU waits for it)."""
+    flat = [t.detach().double().reshape(-1) for t in tensors]
+    if all(t.device == flat[0].device for t in flat):
+        host = torch.cat(flat).cpu().numpy()
+    else:
+        host = np.concatenate([t.cpu().numpy() for t in flat])
+    ends = np.cumsum([t.numel() for t in flat])
+    return [a.reshape(t.shape) for a, t in zip(np.split(host, ends[:-1]), tensors)]
+
+
 class MTPFunction(torch.autograd.Function):
     """(species, moment, radial) -> (E [C], F [N,3], sigma [C,6])."""
 
     @staticmethod
     def forward(ctx, species, moment, radial, engine: MTPEngine, batch: DeviceBatch):
-        engine.set_coeffs(species.detach().double().cpu().numpy(), moment.detach().double().cpu().numpy(),
-                          radial.detach().double().cpu().numpy())
+        host = _host_coeffs(species, moment, radial)
+        engine.set_coeffs(*host)
         b = batch
         E, F, S = engine.batch_device(b.itypes, b.rijs, b.js, b.jtypes, b.counts, b.cfg, b.volumes, b.nconfig)
         ctx.engine = engine
         ctx.batch = batch
-        ctx.coeffs = (species.detach(), moment.detach(), radial.detach())
+        ctx.coeffs = host
         ctx.devices = (species.device, moment.device, radial.device)
         return E, F, S
 
@@ -96,9 +108,8 @@ class MTPFunction(torch.autograd.Function):
     def backward(ctx, gE, gF, gS):
         b = ctx.batch
         eng = ctx.engine
-        sp, mo, ra = ctx.coeffs
         # the handle may have seen other coefficients since the forward
-        eng.set_coeffs(sp.double().cpu().numpy(), mo.double().cpu().numpy(), ra.double().cpu().numpy())
+        eng.set_coeffs(*ctx.coeffs)
         dev = b.rijs.device
         z = lambda shape: torch.zeros(shape, dtype=torch.float64, device=dev)
         gE = z(b.nconfig) if gE is None else gE.to(dev, torch.float64).contiguous()
