@@ -571,7 +571,10 @@ int run_host_pipelined_body(mtp_handle* h, int natoms, int stride, const int* it
                             const int* js, const int* jtypes, const int* counts, double* vatom) {
   const cudaStream_t s = h->stream;
   if (!h->copy_stream) MTP_CUDA(h, cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
-  const int nch = std::max(1, std::min(kPipelineChunks, natoms / (kPipelineMinAtoms / 2)));
+  // About 8 chunks of at least 8,192 atoms, 16 on large systems: what follows
+  // the last copy is one chunk's evaluation (level 16 FP64, 107,550 atoms, three
+  // chunks: 4.99 ms, eight: 4.67; level 20, 91,446 atoms, two: 6.37, eight: 5.25)
+  const int nch = std::max({1, std::min(kPipelineChunks / 2, natoms / 8192), std::min(kPipelineChunks, natoms / 32768)});
   while (static_cast<int>(h->chunk_events.size()) < nch + 1) {
     cudaEvent_t ev;
     MTP_CUDA(h, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
