@@ -115,6 +115,9 @@ struct mtp_handle {
   // host-buffer calls (mtp_compute) on large systems copy the inputs in atom
   // chunks on copy_stream while the evaluation kernel runs on earlier chunks
   cudaStream_t copy_stream = nullptr;
+  // set while a host call is captured: its graph forks (run_device)
+  bool fork = false;
+  cudaEvent_t fork_event = nullptr, join_event = nullptr;
   std::vector<cudaEvent_t> chunk_events;
   int prof_used = 0;
   // mtp_execute_potential: page-locked staging of the per-atom rows
@@ -330,6 +333,8 @@ void free_handle(mtp_handle* h) {
   if (h->h_tot) cudaFreeHost(h->h_tot);
   for (auto ev : h->chunk_events) cudaEventDestroy(ev);
   if (h->copy_stream) cudaStreamDestroy(h->copy_stream);
+  if (h->fork_event) cudaEventDestroy(h->fork_event);
+  if (h->join_event) cudaEventDestroy(h->join_event);
   if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
   for (void* q : {static_cast<void*>(h->hp_rij), static_cast<void*>(h->hp_F), static_cast<void*>(h->hp_js),
                   static_cast<void*>(h->hp_jt), static_cast<void*>(h->hp_cnt), static_cast<void*>(h->hp_types)})
@@ -516,11 +521,22 @@ int prof_begin(mtp_handle* h, cudaEvent_t* e1) {
 }
 
 // Evaluate site energies and per-slot gradients, then forces and virials.
+// `counted`: the incoming slots were counted with the rows.  While a call is
+// captured (h->fork) the incoming lists, which only the force gather needs,
+// become a branch of the graph beside the evaluation.
 int run_device(mtp_handle* h, int natoms, int stride, const int* itypes, const double* rijs, const int* js,
-               const int* jtypes, const int* counts, bool rebuild_incoming, double* forces, double* vatom) {
+               const int* jtypes, const int* counts, bool rebuild_incoming, bool counted, double* forces,
+               double* vatom) {
+  const bool fork = rebuild_incoming && h->fork;
   if (rebuild_incoming) {
+    const cudaStream_t s = fork ? h->copy_stream : h->stream;
+    if (fork) {
+      MTP_CUDA(h, cudaEventRecord(h->fork_event, h->stream));
+      MTP_CUDA(h, cudaStreamWaitEvent(s, h->fork_event, 0));
+    }
     MTP_CUDA(h, launch_incoming(natoms, stride, js, jtypes, counts, h->d_in_cnt, h->d_in_ptr, h->d_in_slot,
-                                h->d_blk, h->stream));
+                                h->d_blk, counted, s));
+    if (fork) MTP_CUDA(h, cudaEventRecord(h->join_event, s));
   }
   cudaEvent_t e1 = nullptr;
   int st = prof_begin(h, &e1);
@@ -528,6 +544,7 @@ int run_device(mtp_handle* h, int natoms, int stride, const int* itypes, const d
   st = eval_range(h, natoms, 0, natoms, stride, itypes, rijs, jtypes, counts);
   if (st != MTP_OK) return st;
   if (e1) MTP_CUDA(h, cudaEventRecord(e1, h->stream));
+  if (fork) MTP_CUDA(h, cudaStreamWaitEvent(h->stream, h->join_event, 0));
   MTP_CUDA(h, launch_force_gather(natoms, stride, rijs, counts, h->d_G, h->d_in_ptr, h->d_in_slot,
                                   rebuild_incoming, forces, h->d_wown, vatom, h->stream));
   return MTP_OK;
@@ -609,7 +626,7 @@ int run_host_pipelined_body(mtp_handle* h, int natoms, int stride, const int* it
   }
   if (e1) MTP_CUDA(h, cudaEventRecord(e1, s));
   MTP_CUDA(h, launch_incoming(natoms, stride, h->d_js, h->d_jtypes, counts ? h->d_counts : nullptr, h->d_in_cnt,
-                              h->d_in_ptr, h->d_in_slot, h->d_blk, s));
+                              h->d_in_ptr, h->d_in_slot, h->d_blk, false, s));
   MTP_CUDA(h, launch_force_gather(natoms, stride, h->d_rijs, counts ? h->d_counts : nullptr, h->d_G, h->d_in_ptr,
                                   h->d_in_slot, true, h->d_F, h->d_wown, vatom, s));
   return MTP_OK;
@@ -675,7 +692,7 @@ int enqueue_small_call(mtp_handle* h, int natoms, int stride, const int* itypes,
     if (counts) MTP_CUDA(h, cudaMemcpyAsync(h->d_counts, counts, N * sizeof(int), cudaMemcpyHostToDevice, s));
   }
   int st = run_device(h, natoms, stride, h->d_itypes, h->d_rijs, h->d_js, h->d_jtypes, counts ? h->d_counts : nullptr,
-                      true, h->d_F, (flags & MTP_VATOM) ? h->d_vatom : nullptr);
+                      true, false, h->d_F, (flags & MTP_VATOM) ? h->d_vatom : nullptr);
   if (st != MTP_OK) return st;
   MTP_CUDA(h, launch_totals(natoms, h->d_E, h->d_wown, h->d_partials, h->d_tot, h->d_err, nullptr, nullptr, s));
   if (natoms > 0) {
@@ -704,9 +721,14 @@ int run_graphable(mtp_handle* h, const HostCallKey& key, bool pinned, Enqueue&& 
   } else if (pinned && key == h->seen_key && !h->seen_uncapturable) {
     cudaGraph_t g = nullptr;
     cudaGraphExec_t ex = nullptr;
+    if (!h->copy_stream) MTP_CUDA(h, cudaStreamCreateWithFlags(&h->copy_stream, cudaStreamNonBlocking));
+    if (!h->fork_event) MTP_CUDA(h, cudaEventCreateWithFlags(&h->fork_event, cudaEventDisableTiming));
+    if (!h->join_event) MTP_CUDA(h, cudaEventCreateWithFlags(&h->join_event, cudaEventDisableTiming));
     bool ok = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
     if (ok) {
+      h->fork = true;
       const int cst = enqueue();
+      h->fork = false;
       const cudaError_t ce = cudaStreamEndCapture(s, &g);
       ok = cst == MTP_OK && ce == cudaSuccess && g != nullptr;
     }
@@ -1018,7 +1040,7 @@ int mtp_compute_device(mtp_handle* h, int natoms, int stride, const int* d_itype
   if ((flags & MTP_EATOM) && !d_eatom) return fail(h, MTP_E_INVALID, "MTP_EATOM without an eatom pointer");
   if ((flags & MTP_VATOM) && !d_vatom) return fail(h, MTP_E_INVALID, "MTP_VATOM without a vatom pointer");
   const bool rebuild = !(flags & MTP_REUSE_NEIGHBORS);
-  int st = run_device(h, natoms, stride, d_itypes, d_rijs, d_js, d_jtypes, d_counts, rebuild, d_forces,
+  int st = run_device(h, natoms, stride, d_itypes, d_rijs, d_js, d_jtypes, d_counts, rebuild, false, d_forces,
                       (flags & MTP_VATOM) ? d_vatom : nullptr);
   if (st != MTP_OK) return st;
   if (flags & (MTP_EFLAG | MTP_VFLAG)) {
@@ -1050,9 +1072,9 @@ int mtp_compute_positions_device(mtp_handle* h, int nlocal, int nall, const doub
   if (nlocal > 0)
     MTP_CUDA(h, launch_rows_from_positions(nlocal, nall, d_x, d_species, d_owner, list_stride, d_neigh, d_numneigh,
                                            h->cutoff, stride, h->d_rijs, h->d_js, h->d_jtypes, h->d_counts,
-                                           h->d_err, h->stream));
+                                           h->d_in_cnt, h->d_err, h->stream));
   int st = run_device(h, nlocal, stride, nlocal > 0 ? d_species : h->d_itypes, h->d_rijs, h->d_js, h->d_jtypes,
-                      h->d_counts, true, d_forces, (flags & MTP_VATOM) ? d_vatom : nullptr);
+                      h->d_counts, true, true, d_forces, (flags & MTP_VATOM) ? d_vatom : nullptr);
   if (st != MTP_OK) return st;
   if (flags & (MTP_EFLAG | MTP_VFLAG)) {
     st = write_totals(h, nlocal, h->d_E, h->d_wown, h->d_partials, h->d_tot, (flags & MTP_EFLAG) ? d_energy : nullptr,
@@ -1172,10 +1194,10 @@ int mtp_compute_positions(mtp_handle* h, int nlocal, int nall, const double* x, 
       MTP_CUDA(h, cudaMemcpyAsync(h->d_numneigh, numneigh, N * sizeof(int), cudaMemcpyHostToDevice, s));
       MTP_CUDA(h, launch_rows_from_positions(nlocal, nall, h->d_xall, h->d_spall, h->d_owner, list_stride,
                                              h->d_neigh, h->d_numneigh, h->cutoff, stride, h->d_rijs, h->d_js,
-                                             h->d_jtypes, h->d_counts, h->d_err, s));
+                                             h->d_jtypes, h->d_counts, h->d_in_cnt, h->d_err, s));
     }
     int st = run_device(h, nlocal, stride, nlocal > 0 ? h->d_spall : h->d_itypes, h->d_rijs, h->d_js, h->d_jtypes,
-                        h->d_counts, true, h->d_F, (flags & MTP_VATOM) ? h->d_vatom : nullptr);
+                        h->d_counts, true, true, h->d_F, (flags & MTP_VATOM) ? h->d_vatom : nullptr);
     if (st != MTP_OK) return st;
     MTP_CUDA(h, launch_totals(nlocal, h->d_E, h->d_wown, h->d_partials, h->d_tot, h->d_err, nullptr, nullptr, s));
     if (nlocal > 0) {
@@ -1306,7 +1328,7 @@ int mtp_compute_batch_device(mtp_handle* h, int natoms, int stride, int nconfig,
     h->cfg_cap = nconfig + 1;
   }
   MTP_CUDA(h, launch_config_ptr(natoms, nconfig, d_cfg, h->d_cfg_ptr, h->d_err, h->stream));
-  int st = run_device(h, natoms, stride, d_itypes, d_rijs, d_js, d_jtypes, d_counts, true, d_forces, nullptr);
+  int st = run_device(h, natoms, stride, d_itypes, d_rijs, d_js, d_jtypes, d_counts, true, false, d_forces, nullptr);
   if (st != MTP_OK) return st;
   MTP_CUDA(h, launch_config_totals(natoms, nconfig, h->d_cfg_ptr, h->d_E, h->d_wown, d_volumes, d_energy, d_stress,
                                    h->stream));
@@ -1646,7 +1668,7 @@ int mtp_compute_device_noalloc(mtp_handle* h, int natoms, int stride, const int*
   const long long groups = (static_cast<long long>(natoms) + A - 1) / A;
   const int blocks = static_cast<int>(std::max(1LL, std::min<long long>(static_cast<long long>(bps) * h->sm_count,
                                                                          groups)));
-  MTP_CUDA(h, launch_incoming(natoms, stride, d_js, d_jtypes, d_counts, in_cnt, in_ptr, in_slot, blk, h->stream));
+  MTP_CUDA(h, launch_incoming(natoms, stride, d_js, d_jtypes, d_counts, in_cnt, in_ptr, in_slot, blk, false, h->stream));
   MTP_CUDA(h, launch_eval(md, io, lanes, blocks, fp64, false, A, h->stream));
   MTP_CUDA(h, launch_force_gather(natoms, stride, d_rijs, d_counts, grad, in_ptr, in_slot, true, d_forces, wown, nullptr,
                                   h->stream));

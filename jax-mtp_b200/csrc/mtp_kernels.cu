@@ -284,14 +284,17 @@ __device__ __forceinline__ void sort_incoming(int b, int n, int lane, int* in_sl
 }
 
 cudaError_t launch_incoming(int natoms, int stride, const int* js, const int* jtypes, const int* counts,
-                            int* in_cnt, int* in_ptr, int* in_slot, int* block_tmp, cudaStream_t st) {
+                            int* in_cnt, int* in_ptr, int* in_slot, int* block_tmp, bool counted, cudaStream_t st) {
   if (natoms <= 0) return cudaSuccess;
-  // the counts start at zero (the allocation-free path reuses a shared array)
-  cudaError_t e = cudaMemsetAsync(in_cnt, 0, sizeof(int) * natoms, st);
-  if (e != cudaSuccess) return e;
   const size_t n = static_cast<size_t>(natoms) * stride;
   const int gb = static_cast<int>(std::min<size_t>((n + 255) / 256, 148 * 32));
-  k_count_incoming<<<gb, 256, 0, st>>>(natoms, stride, js, jtypes, counts, in_cnt);
+  cudaError_t e = cudaSuccess;
+  if (!counted) {
+    // the counts start at zero (the allocation-free path reuses a shared array)
+    e = cudaMemsetAsync(in_cnt, 0, sizeof(int) * natoms, st);
+    if (e != cudaSuccess) return e;
+    k_count_incoming<<<gb, 256, 0, st>>>(natoms, stride, js, jtypes, counts, in_cnt);
+  }
   e = scan_exclusive(natoms, in_cnt, in_ptr, block_tmp, st);
   if (e != cudaSuccess) return e;
   k_fill_incoming<<<gb, 256, 0, st>>>(natoms, stride, js, jtypes, counts, in_ptr, in_cnt, in_slot);
@@ -452,7 +455,8 @@ __global__ void k_totals(int natoms, const double* __restrict__ e, const double*
 // Neighbour rows from positions, one warp per local atom: the candidates of
 // the atom's list closer than the cutoff are kept in list order (a ballot and
 // a prefix count give each kept candidate its slot), with r_ij = x_j - x_i,
-// the owner index of j and its species (-1 for a ghost without an owner).
+// the owner index of j and its species (-1 for a ghost without an owner).  It
+// also counts the incoming slots of each owner (in_cnt, zero before).
 // This is the host packing loop of the pair style (pair_jax_mtp.cpp:110-167)
 // on the device: r^2 is formed with separately rounded products and sums, as
 // that loop does, so the same candidates are kept.
@@ -461,7 +465,7 @@ __global__ void k_rows_from_positions(int nlocal, int nall, const double* __rest
                                       int list_stride, const int* __restrict__ neigh,
                                       const int* __restrict__ numneigh, double cut2, int stride,
                                       double* __restrict__ rijs, int* __restrict__ js, int* __restrict__ jtypes,
-                                      int* __restrict__ counts, int* __restrict__ err) {
+                                      int* __restrict__ counts, int* __restrict__ in_cnt, int* __restrict__ err) {
   const int i = static_cast<int>((static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= nlocal) return;   // the warp leaves together
@@ -493,8 +497,10 @@ __global__ void k_rows_from_positions(int nlocal, int nall, const double* __rest
         rijs[3 * o + 1] = dy;
         rijs[3 * o + 2] = dz;
         const int own = owner[j];
+        const int t = own >= 0 ? species[j] : -1;
         js[o] = own;
-        jtypes[o] = own >= 0 ? species[j] : -1;
+        jtypes[o] = t;
+        if (t >= 0 && own < nlocal) atomicAdd(in_cnt + own, 1);   // as k_count_incoming
       }
     }
     kept += __popc(m);
@@ -507,13 +513,15 @@ __global__ void k_rows_from_positions(int nlocal, int nall, const double* __rest
 
 cudaError_t launch_rows_from_positions(int nlocal, int nall, const double* x, const int* species, const int* owner,
                                        int list_stride, const int* neigh, const int* numneigh, double cutoff,
-                                       int stride, double* rijs, int* js, int* jtypes, int* counts, int* err,
-                                       cudaStream_t st) {
+                                       int stride, double* rijs, int* js, int* jtypes, int* counts, int* in_cnt,
+                                       int* err, cudaStream_t st) {
   if (nlocal <= 0) return cudaSuccess;
+  const cudaError_t e = cudaMemsetAsync(in_cnt, 0, sizeof(int) * nlocal, st);
+  if (e != cudaSuccess) return e;
   const size_t threads = static_cast<size_t>(nlocal) * 32;
   k_rows_from_positions<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, st>>>(
       nlocal, nall, x, species, owner, list_stride, neigh, numneigh, cutoff * cutoff, stride, rijs, js, jtypes,
-      counts, err);
+      counts, in_cnt, err);
   return cudaGetLastError();
 }
 

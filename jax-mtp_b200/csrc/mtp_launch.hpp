@@ -21,8 +21,9 @@ cudaError_t launch_eval(const DevModel& md, const DevIO& io, int threads, int bl
 
 // Incoming-slot lists: for every atom k, the slots (i, s) whose neighbour is k,
 // in any order (launch_force_gather sorts them).  in_ptr [natoms + 1].
+// `counted`: in_cnt already holds each atom's number of slots.
 cudaError_t launch_incoming(int natoms, int stride, const int* js, const int* jtypes, const int* counts,
-                            int* in_cnt, int* in_ptr, int* in_slot, int* block_tmp, cudaStream_t st);
+                            int* in_cnt, int* in_ptr, int* in_slot, int* block_tmp, bool counted, cudaStream_t st);
 
 // forces[i] = own slot gradients - incoming slot gradients; wown [natoms][6]
 // = -sym(sum_s r_is (x) g_is) (LAMMPS order xx,yy,zz,xy,xz,yz); when vatom
@@ -50,10 +51,11 @@ cudaError_t launch_config_ptr(int natoms, int nconfig, const int* cfg_of_atom, i
 // Rows [nlocal][stride] (r_ij, owner index, species, count) from positions
 // x [nall][3] and candidate lists neigh [nlocal][list_stride]: candidates
 // closer than cutoff, in list order; more than stride sets kErrCapacity.
+// in_cnt [nlocal] gets the number of slots that point at each atom.
 cudaError_t launch_rows_from_positions(int nlocal, int nall, const double* x, const int* species, const int* owner,
                                        int list_stride, const int* neigh, const int* numneigh, double cutoff,
-                                       int stride, double* rijs, int* js, int* jtypes, int* counts, int* err,
-                                       cudaStream_t st);
+                                       int stride, double* rijs, int* js, int* jtypes, int* counts, int* in_cnt,
+                                       int* err, cudaStream_t st);
 
 // FMA-chain peak probe.
 cudaError_t measure_fma_peak(double* fp64_tflops, double* fp32_tflops);
