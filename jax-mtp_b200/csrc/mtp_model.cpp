@@ -633,14 +633,26 @@ bool build_schedule(const Potential& pot, int lanes, Schedule& s, std::string& e
     jobs[it->second].sides.push_back(Side{static_cast<uint32_t>(s.v_dm + s.dm_pos[tgt]),
                                           static_cast<uint32_t>(s.v_m + other), static_cast<uint32_t>(mult)});
   };
+  // both sides of a product; a square's are the same, so one entry with twice
+  // the multiplicity does for both: 8, 4, 1.8 and 0.8 % of the reverse entries
+  // at levels 16, 20, 24 and 28.  L24 FP32 4646 -> 4608 us (55,296 atoms, four
+  // per block: 4149 -> 4134), L20 FP64 773 -> 767, L16 FP64 563 -> 558,
+  // L28 FP64 1894 -> 1882, its adjoint 31.09 -> 30.95 ms
+  auto add_sides = [&](std::vector<Job>& jobs, std::map<int, int>& job_of, const int* r, bool first, bool second) {
+    if (first && second && r[0] == r[1] && 2 * r[2] <= static_cast<int>(kMultMask)) {
+      add_side(jobs, job_of, r[0], r[3], r[1], 2 * r[2]);
+      return;
+    }
+    if (first) add_side(jobs, job_of, r[0], r[3], r[1], r[2]);
+    if (second) add_side(jobs, job_of, r[1], r[3], r[0], r[2]);
+  };
   for (int L = maxd; L >= 1; --L) {
     std::vector<Job> jobs;
     std::map<int, int> job_of;
     for (int e = 0; e < T; ++e) {
       const int* r = &pot.times[4 * e];
       if (depth[r[3]] != L) continue;
-      if (depth[r[0]] >= 1) add_side(jobs, job_of, r[0], r[3], r[1], r[2]);
-      if (depth[r[1]] >= 1) add_side(jobs, job_of, r[1], r[3], r[0], r[2]);
+      add_sides(jobs, job_of, r, depth[r[0]] >= 1, depth[r[1]] >= 1);
     }
     emit_jobs(jobs, lanes, width, false, programs, rev, parts);
     for (const auto& kv : job_of) written[kv.first] = 1;
@@ -652,8 +664,7 @@ bool build_schedule(const Potential& pot, int lanes, Schedule& s, std::string& e
       for (int e = 0; e < T; ++e) {
         const int* r = &pot.times[4 * e];
         if (depth[r[3]] != L) continue;
-        if (depth[r[0]] == 0) add_side(jobs, job_of, r[0], r[3], r[1], r[2]);
-        if (depth[r[1]] == 0) add_side(jobs, job_of, r[1], r[3], r[0], r[2]);
+        add_sides(jobs, job_of, r, depth[r[0]] == 0, depth[r[1]] == 0);
       }
     }
     emit_jobs(jobs, lanes, width, false, programs, rev, parts);
