@@ -453,6 +453,9 @@ __device__ __forceinline__ void chain_dense(int top, const typename Force<T>::P*
 // segment stopped.  With W_s = sum_mu Dm[s][mu] f_mu(d) over monomials s and
 // W'_s the same with f': G = grad_u sum_s W_s u^s and S = sum_s W'_s u^s.
 // Partial sums of a group's warps are added in warp order (deterministic).
+// Bound by the latency of the chains (two dependent multiply-adds a step): level
+// 24 mixed at 512 lanes x 4 atoms, 15,800 cycles an iteration, 18,400 with lanes
+// on neighbours but the adjoints read one value per load from the value space.
 template <typename T, int A, int R, int MODE>
 __device__ __forceinline__ void force_phase(const DevModel& md, const DevIO& io, const SmemLayout& L,
                                             unsigned char* smem, const int (&nv_a)[A], int base, int tid, int NT) {
@@ -628,6 +631,18 @@ __device__ __forceinline__ void warp_partials(double (&v)[A], double* red) {
 // space (moments, adjoints, partials) is a private slice of global memory
 // (L1/L2-resident) instead of shared memory; used when it does not fit in
 // shared memory (level 28 in FP64).
+//
+// What bounds it: shared-memory wavefronts.  Level 24 mixed at 512 lanes x 4
+// atoms keeps 16 warps and all of an SM's shared memory busy with one block; the
+// tree takes about three fifths of an iteration, most of it 16-byte gathers at
+// four cycles a warp, and the rest is the latency of N1 to N3 with 16 warps.
+// With the value space in global memory it is the L1 data pipe and the program
+// stream from L2.  Staging rows, 16-byte basic moments and neighbours on lanes
+// in the force phase, one launch, before -> after: level 24 mixed 512 x 4,
+// 55,296 atoms 4.74 -> 4.15 ms; level 20 mixed 256 x 4, 16,000 atoms 0.553 ->
+// 0.450; level 16 mixed 128 x 4, 27,648 atoms 0.435 -> 0.356, FP64 128 x 2 0.672
+// -> 0.565; level 24 FP64 512 x 2, 16,384 atoms 2.41 -> 2.32.
+//
 // One block's rows of a staging task (atom, slot), as they lie in memory.
 struct RowSlot {
   double x, y, z;

@@ -253,6 +253,11 @@ struct TrainSlot {
   int jt, j, it, cfg, cnt;
 };
 
+// Training gradient of one atom per block iteration.  The dual trees bound it: 16
+// bytes per operand through the L1 data pipe, from shared memory (level 20) or
+// from the block's slice of global memory (level 28).  Adjoint and reduction,
+// FP64, with the layout of the evaluation's phases: level 20, 4,968 atoms 0.77
+// -> 0.51 ms; level 28, 18,515 atoms 35.8 -> 31.0 ms.
 template <typename T, bool kVGlobal>
 __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, int n_pad, void* vscratch,
                                                      double* partials) {
