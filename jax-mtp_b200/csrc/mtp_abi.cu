@@ -74,8 +74,7 @@ struct mtp_handle {
   int threads = 0, blocks_per_sm = 0;   // requested launch (mtp_set_launch); 0 threads: automatic
   int last_threads = 0, last_blocks = 0, last_bps = 0;
   bool last_vglobal = false;
-  void* d_vscratch = nullptr;
-  size_t vscratch_bytes = 0;
+  void* d_vscratch = nullptr;   // value spaces in global memory, allocated once (pick_launch)
   size_t last_smem = 0;
   std::map<int, DeviceSchedule> scheds;
   std::map<int, DeviceSchedule> sizes;   // by lanes: schedules without programs, to size launches
@@ -377,6 +376,16 @@ double launch_estimate(const Potential& pot, bool fp64, int lanes, int A, int bp
   return rounds * (20.0 + 0.15 * pot.T / lanes + atom * A * resident);
 }
 
+// Value spaces in global memory, one slice of A atoms per SM, and the most atoms
+// that may share a block there: two as long as the slices stay in L2.
+size_t global_space_bytes(const mtp_handle* h, const DeviceSchedule& ds, int A, bool fp64) {
+  return static_cast<size_t>(h->sm_count) * ds.sched.v_size * A * (fp64 ? sizeof(double) : sizeof(float));
+}
+
+int global_atoms(const mtp_handle* h, const DeviceSchedule& ds, bool fp64) {
+  return global_space_bytes(h, ds, 2, fp64) <= h->l2_bytes / 4 * 3 ? 2 : 1;
+}
+
 // Launch shape for the evaluation kernel on natoms: the (lanes, atoms per
 // block) within the handle's request with the least expected time
 // (launch_estimate) among those whose value space fits in shared memory; when
@@ -418,8 +427,7 @@ int pick_launch(mtp_handle* h, long long natoms, int stride, const DeviceSchedul
     double least = 0.0;
     for (int A : {1, 2}) {
       if (h->apb > 0 && A > h->apb) continue;
-      const size_t spaces = static_cast<size_t>(h->sm_count) * sz->sched.v_size * A * (fp64 ? sizeof(double) : sizeof(float));
-      if (A > 1 && spaces > h->l2_bytes / 4 * 3) continue;
+      if (A > 1 && A > global_atoms(h, *sz, fp64)) continue;
       int bps = 0;
       st = launch_occupancy(h, best.lanes, stride, fp64, true, A, &bps);
       if (st != MTP_OK) return st;
@@ -450,16 +458,13 @@ int pick_launch(mtp_handle* h, long long natoms, int stride, const DeviceSchedul
   if (st != MTP_OK) return st;
   const long long groups = (natoms + best.A - 1) / best.A;
   const long long blocks = std::max(1LL, std::min<long long>(static_cast<long long>(best.bps) * h->sm_count, groups));
-  if (vglobal) {
-    const size_t need = static_cast<size_t>(blocks) * ds->sched.v_size * best.A * (fp64 ? sizeof(double) : sizeof(float));
-    if (need > h->vscratch_bytes) {
-      if (h->d_vscratch) cudaFree(h->d_vscratch);
-      h->d_vscratch = nullptr;
-      h->vscratch_bytes = 0;
-      MTP_CUDA(h, cudaMalloc(&h->d_vscratch, need));
-      h->vscratch_bytes = need;
-      ++h->gen;
-    }
+  if (vglobal && !h->d_vscratch) {
+    // for the largest launch any call of this handle can take (one block per SM
+    // with the most atoms), once: a graph that a caller captured holds the
+    // address, so the buffer must not move when a later call needs more of it
+    const size_t bytes = global_space_bytes(h, *ds, global_atoms(h, *ds, fp64), fp64);
+    MTP_CUDA(h, cudaMalloc(&h->d_vscratch, bytes));
+    ++h->gen;
   }
   *ds_out = ds;
   *blocks_out = static_cast<int>(blocks);

@@ -1,0 +1,111 @@
+"""Host code of the library on a CUDA runtime without a GPU.
+
+The library's objects are linked with tests/host/fake_cudart.cpp: device memory
+is host memory, kernels do not run, and the runtime calls are logged.  What is
+checked here is what the host does: which allocations, copies and launches it
+makes, in which order, and what it refuses while a stream is being captured."""
+
+import ctypes
+import os
+import re
+import subprocess
+
+import pytest
+
+from conftest import REPO, potential_path
+from mtp_b200._lib import EFLAG, REUSE_NEIGHBORS, SIGNATURES, VFLAG
+
+CSRC = os.path.join(REPO, "jax-mtp_b200", "csrc")
+FP64, MIXED = 0, 1
+L16, L20, L24, L28 = "cfg1_L16_S2.mtp", "cfg3_L20_S2.mtp", "cfg2_L24_S3.mtp", "cfg4_L28_S4.mtp"
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    subprocess.run(["make", "-C", CSRC, "-j", "4"], check=True, capture_output=True)
+    out = str(tmp_path_factory.mktemp("host") / "libmtp_host.so")
+    objs = [os.path.join(CSRC, "_build", f"mtp_{n}.o") for n in ("model", "kernels", "train", "md", "abi")]
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I/usr/local/cuda/include",
+                    os.path.join(REPO, "tests", "host", "fake_cudart.cpp"), *objs, "-o", out], check=True)
+    L = ctypes.CDLL(out)
+    for name, (res, args) in SIGNATURES.items():
+        getattr(L, name).restype, getattr(L, name).argtypes = res, args
+    L.fake_log.restype, L.fake_stream.restype = ctypes.c_char_p, ctypes.c_void_p
+    L.fake_capture.argtypes = [ctypes.c_void_p, ctypes.c_int]
+    L.fake_set_device.argtypes = [ctypes.c_void_p, ctypes.c_int]
+    L.cudaMalloc.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.c_size_t]
+    return L
+
+
+class Handle:
+    """One handle with device buffers for its capacities, on a stream of the caller."""
+
+    def __init__(self, lib, name, atoms, stride, precision=FP64):
+        self.L, self.stride, self.h = lib, stride, ctypes.c_void_p()
+        assert lib.mtp_create(potential_path(name).encode(), atoms, stride, 5.0, 0, precision,
+                              ctypes.byref(self.h)) == 0
+        self.stream = lib.fake_stream()
+        lib.mtp_set_stream(self.h, self.stream)
+        sizes = dict(itypes=4 * atoms, rijs=24 * atoms * stride, js=4 * atoms * stride, jtypes=4 * atoms * stride,
+                     counts=4 * atoms, forces=24 * atoms, energy=8, virial=48)
+        self.buf = {k: self.alloc(n) for k, n in sizes.items()}
+        lib.fake_clear()
+
+    def alloc(self, n):
+        p = ctypes.c_void_p()
+        assert self.L.cudaMalloc(ctypes.byref(p), n) == 0
+        return p.value
+
+    def compute(self, n, flags=EFLAG | VFLAG, stride=None, energy=None, virial=None):
+        """Status and log of one device call."""
+        b = self.buf
+        self.L.fake_clear()
+        st = self.L.mtp_compute_device(self.h, n, stride or self.stride, b["itypes"], b["rijs"], b["js"], b["jtypes"],
+                                       b["counts"], flags, energy or b["energy"], b["forces"],
+                                       virial or b["virial"], None, None)
+        return st, self.log()
+
+    def captured(self, n, **kw):
+        """The same call while its stream is captured."""
+        self.L.fake_capture(self.stream, 1)
+        try:
+            return self.compute(n, **kw)
+        finally:
+            self.L.fake_capture(self.stream, 0)
+
+    def log(self):
+        return self.L.fake_log().decode()
+
+    def launch(self):
+        out = (ctypes.c_int * 5)()
+        assert self.L.mtp_get_launch(self.h, out) == 0
+        return dict(zip(("threads", "blocks", "smem", "per_sm", "atoms"), out))
+
+    def error(self):
+        return self.L.mtp_last_error(self.h).decode()
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        self.L.mtp_destroy(self.h)
+
+
+@pytest.mark.parametrize("precision,stride", [(FP64, 12), (MIXED, 600)])
+def test_global_value_space_never_moves(lib, precision, stride):
+    """A captured graph keeps the address of the value space in global memory:
+    no later call of the handle may free it, whatever its number of atoms."""
+    with Handle(lib, L28, 700, stride, precision) as h:
+        assert h.compute(100)[0] == 0
+        for n in (400, 256, 149, 700, 297, 1):
+            st, log = h.compute(n)
+            assert st == 0
+            assert "free" not in log, f"{n} atoms"
+
+
+def test_global_value_space_is_there_for_a_captured_size(lib):
+    """A size whose value spaces are more than those of the calls before it."""
+    with Handle(lib, L28, 4000, 12) as h:
+        assert h.compute(200)[0] == 0 and h.launch()["atoms"] == 2
+        st, log = h.captured(4000)
+        assert st == 0 and "in-capture" not in log, h.error()
