@@ -386,16 +386,16 @@ int global_atoms(const mtp_handle* h, const DeviceSchedule& ds, bool fp64) {
   return global_space_bytes(h, ds, 2, fp64) <= h->l2_bytes / 4 * 3 ? 2 : 1;
 }
 
-// Launch shape for the evaluation kernel on natoms: the (lanes, atoms per
-// block) within the handle's request with the least expected time
-// (launch_estimate) among those whose value space fits in shared memory; when
-// none fits, the value space moves to global memory (A = 1 or 2).
-// While the stream is being captured nothing can be uploaded, so a shape whose
-// programs are not on the device yet gives way to the best one whose are.
-int pick_launch(mtp_handle* h, long long natoms, int stride, const DeviceSchedule** ds_out, int* blocks_out, bool fp64,
-                bool* vglobal_out) {
-  struct Choice { int lanes = 0, A = 1, bps = 0; double est = 0.0; };
-  Choice best, ready;
+// One launch shape that fits and its expected time (or, with the value space in
+// global memory, its expected number of one-atom rounds).
+struct Shape {
+  int lanes = 0, A = 1, bps = 0;
+  double est = 0.0;
+};
+
+// The shapes of the handle's request that fit for natoms, with the value space
+// in shared memory.
+int shared_shapes(mtp_handle* h, long long natoms, int stride, bool fp64, std::vector<Shape>* out) {
   for (int lanes : {512, 256, 128}) {
     if (h->threads > 0 && lanes > h->threads) continue;
     for (int A : {4, 2, 1}) {
@@ -404,57 +404,68 @@ int pick_launch(mtp_handle* h, long long natoms, int stride, const DeviceSchedul
       int bps = 0;
       const int st = launch_occupancy(h, lanes, stride, fp64, false, A, &bps);
       if (st != MTP_OK) return st;
-      if (bps <= 0) continue;
-      const Choice c{lanes, A, bps, launch_estimate(h->pot, fp64, lanes, A, bps, h->sm_count, natoms)};
-      if (best.lanes == 0 || c.est < best.est) best = c;
-      if (schedule_uploaded(h, lanes, access_width(fp64, A)) && (ready.lanes == 0 || c.est < ready.est)) ready = c;
+      if (bps > 0) out->push_back({lanes, A, bps, launch_estimate(h->pot, fp64, lanes, A, bps, h->sm_count, natoms)});
     }
   }
-  bool vglobal = false;
-  if (best.lanes == 0) {
-    // value space in global memory: 512 lanes give an SM 16 warps with one
-    // block, so the blocks' value spaces stay within L2.  Two atoms share
-    // every program entry (4.5 MB an iteration at level 28, as much L2 traffic
-    // as the operands) and fill more of each 32-byte sector a gather touches:
-    // an iteration takes 1.78x (FP64, 2.20 -> 1.96 ms for 2,048 atoms) or
-    // 1.09x (FP32) one atom's time, so they win where that saves a round, as
-    // long as the value spaces stay in L2 (four atoms' do not: 3.47 ms).
-    vglobal = true;
-    best.lanes = 512;
-    const DeviceSchedule* sz = nullptr;
-    int st = get_sizes(h, best.lanes, &sz);
+  return MTP_OK;
+}
+
+// The same with the value space in global memory: 512 lanes give an SM 16 warps
+// with one block, so the blocks' value spaces stay within L2.  Two atoms share
+// every program entry (4.5 MB an iteration at level 28, as much L2 traffic as
+// the operands) and fill more of each 32-byte sector a gather touches: an
+// iteration takes 1.78x (FP64, 2.20 -> 1.96 ms for 2,048 atoms) or 1.09x (FP32)
+// one atom's time, so they win where that saves a round, as long as the value
+// spaces stay in L2 (four atoms' do not: 3.47 ms).
+int global_shapes(mtp_handle* h, long long natoms, int stride, bool fp64, std::vector<Shape>* out) {
+  const DeviceSchedule* sz = nullptr;
+  int st = get_sizes(h, 512, &sz);
+  if (st != MTP_OK) return st;
+  for (int A : {1, 2}) {
+    if (h->apb > 0 && A > h->apb) continue;
+    if (A > global_atoms(h, *sz, fp64)) continue;
+    int bps = 0;
+    st = launch_occupancy(h, 512, stride, fp64, true, A, &bps);
     if (st != MTP_OK) return st;
-    double least = 0.0;
-    for (int A : {1, 2}) {
-      if (h->apb > 0 && A > h->apb) continue;
-      if (A > 1 && A > global_atoms(h, *sz, fp64)) continue;
-      int bps = 0;
-      st = launch_occupancy(h, best.lanes, stride, fp64, true, A, &bps);
-      if (st != MTP_OK) return st;
-      if (bps <= 0) continue;
-      const long long per = static_cast<long long>(A) * h->sm_count;
-      const double cost = static_cast<double>((natoms + per - 1) / per) * (A == 1 ? 1.0 : fp64 ? 1.78 : 1.09);
-      if (best.bps == 0 || cost < least) {
-        least = cost;
-        best.A = A;
-        best.bps = 1;
-      }
-    }
-    if (best.bps <= 0)
-      return fail(h, MTP_E_CAPACITY, "the evaluation block does not fit in shared memory for this basis and max_nbr");
-    if (best.A > 1 && !schedule_uploaded(h, best.lanes, access_width(fp64, best.A)) &&
-        schedule_uploaded(h, best.lanes, access_width(fp64, 1))) {
-      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-      if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) cudaGetLastError();
-      if (cs != cudaStreamCaptureStatusNone) best.A = 1;
-    }
-  } else if (ready.lanes > 0 && !schedule_uploaded(h, best.lanes, access_width(fp64, best.A))) {
+    const long long per = static_cast<long long>(A) * h->sm_count;
+    if (bps > 0) out->push_back({512, A, 1, static_cast<double>((natoms + per - 1) / per) * (A == 1 ? 1.0 : fp64 ? 1.78 : 1.09)});
+  }
+  return MTP_OK;
+}
+
+// The shape with the least estimate (the first of equal ones), of those whose
+// programs are on the device when only these can be used; null if there is none.
+const Shape* best_shape(const mtp_handle* h, const std::vector<Shape>& shapes, bool fp64, bool uploaded) {
+  const Shape* best = nullptr;
+  for (const Shape& c : shapes)
+    if ((!uploaded || schedule_uploaded(h, c.lanes, access_width(fp64, c.A))) && (!best || c.est < best->est)) best = &c;
+  return best;
+}
+
+// Launch shape for the evaluation kernel on natoms: the (lanes, atoms per
+// block) within the handle's request with the least expected time among those
+// whose value space fits in shared memory; when none fits, the value space
+// moves to global memory.  While the stream is being captured nothing can be
+// uploaded, so a shape whose programs are not on the device yet gives way to
+// the best one whose are.
+int pick_launch(mtp_handle* h, long long natoms, int stride, const DeviceSchedule** ds_out, int* blocks_out, bool fp64,
+                bool* vglobal_out) {
+  std::vector<Shape> shapes;
+  int st = shared_shapes(h, natoms, stride, fp64, &shapes);
+  if (st != MTP_OK) return st;
+  const bool vglobal = shapes.empty();
+  if (vglobal && (st = global_shapes(h, natoms, stride, fp64, &shapes)) != MTP_OK) return st;
+  if (shapes.empty())
+    return fail(h, MTP_E_CAPACITY, "the evaluation block does not fit in shared memory for this basis and max_nbr");
+  Shape best = *best_shape(h, shapes, fp64, false);
+  if (!schedule_uploaded(h, best.lanes, access_width(fp64, best.A))) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) cudaGetLastError();
-    if (cs != cudaStreamCaptureStatusNone) best = ready;
+    if (cs != cudaStreamCaptureStatusNone)
+      if (const Shape* ready = best_shape(h, shapes, fp64, true)) best = *ready;
   }
   const DeviceSchedule* ds = nullptr;
-  const int st = get_schedule(h, best.lanes, access_width(fp64, best.A), &ds);
+  st = get_schedule(h, best.lanes, access_width(fp64, best.A), &ds);
   if (st != MTP_OK) return st;
   const long long groups = (natoms + best.A - 1) / best.A;
   const long long blocks = std::max(1LL, std::min<long long>(static_cast<long long>(best.bps) * h->sm_count, groups));

@@ -109,3 +109,22 @@ def test_global_value_space_is_there_for_a_captured_size(lib):
         assert h.compute(200)[0] == 0 and h.launch()["atoms"] == 2
         st, log = h.captured(4000)
         assert st == 0 and "in-capture" not in log, h.error()
+
+
+@pytest.mark.parametrize("first,second,atoms", [(4000, 100, 2), (100, 4000, 1)])
+def test_capture_in_global_memory_uses_the_programs_that_are_there(lib, first, second, atoms):
+    with Handle(lib, L28, 4000, 12) as h:
+        assert h.compute(first)[0] == 0
+        st, log = h.captured(second)
+        assert st == 0 and "in-capture" not in log, h.error()
+        assert h.launch()["atoms"] == atoms
+        assert h.compute(second)[0] == 0 and h.launch()["atoms"] == 3 - atoms
+
+
+def test_capture_in_shared_memory_uses_the_programs_that_are_there(lib):
+    with Handle(lib, L24, 20000, 12, MIXED) as h:
+        assert h.compute(20000)[0] == 0
+        ran = h.launch()
+        st, log = h.captured(100)
+        assert st == 0 and "in-capture" not in log, h.error()
+        assert (h.launch()["threads"], h.launch()["atoms"]) == (ran["threads"], ran["atoms"])
