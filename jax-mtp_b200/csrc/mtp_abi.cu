@@ -242,10 +242,6 @@ int get_sizes(mtp_handle* h, int lanes, const DeviceSchedule** out) {
   return MTP_OK;
 }
 
-bool schedule_uploaded(const mtp_handle* h, int lanes, int width) {
-  return h->scheds.count(lanes * 64 + width) > 0;
-}
-
 // Schedule for `lanes` threads and `width`-byte operand accesses, built and
 // uploaded on first use; refine_schedule runs where the value space can sit in
 // shared memory (bank order matters only there).
@@ -433,12 +429,38 @@ int global_shapes(mtp_handle* h, long long natoms, int stride, bool fp64, std::v
   return MTP_OK;
 }
 
-// The shape with the least estimate (the first of equal ones), of those whose
-// programs are on the device when only these can be used; null if there is none.
-const Shape* best_shape(const mtp_handle* h, const std::vector<Shape>& shapes, bool fp64, bool uploaded) {
-  const Shape* best = nullptr;
-  for (const Shape& c : shapes)
-    if ((!uploaded || schedule_uploaded(h, c.lanes, access_width(fp64, c.A))) && (!best || c.est < best->est)) best = &c;
+// Programs on the device for `lanes` threads: those whose entry order was tuned
+// for `width`-byte operands or, with `any_order`, others (every order computes
+// the same sums; the bank conflicts and the order of the terms differ).
+const DeviceSchedule* programs_on_device(const mtp_handle* h, int lanes, int width, bool any_order) {
+  const auto it = h->scheds.find(lanes * 64 + width);
+  if (it != h->scheds.end()) return &it->second;
+  if (any_order)
+    for (const auto& kv : h->scheds)
+      if (kv.second.sched.lanes == lanes) return &kv.second;
+  return nullptr;
+}
+
+// The shape with the least estimate (the first of equal ones).
+const Shape& best_shape(const std::vector<Shape>& shapes) {
+  return *std::min_element(shapes.begin(), shapes.end(), [](const Shape& a, const Shape& b) { return a.est < b.est; });
+}
+
+// The same for calls that can upload nothing: of the shapes whose programs are
+// on the device or, where there are none, of those that can run with programs
+// of another entry order.  Null *ds: there are none of these either.
+Shape best_uploaded_shape(const mtp_handle* h, const std::vector<Shape>& shapes, bool fp64, const DeviceSchedule** ds) {
+  Shape best;
+  *ds = nullptr;
+  for (const bool any_order : {false, true}) {
+    for (const Shape& c : shapes) {
+      const DeviceSchedule* p = programs_on_device(h, c.lanes, access_width(fp64, c.A), any_order);
+      if (!p || (*ds && c.est >= best.est)) continue;
+      best = c;
+      *ds = p;
+    }
+    if (*ds) break;
+  }
   return best;
 }
 
@@ -457,16 +479,17 @@ int pick_launch(mtp_handle* h, long long natoms, int stride, const DeviceSchedul
   if (vglobal && (st = global_shapes(h, natoms, stride, fp64, &shapes)) != MTP_OK) return st;
   if (shapes.empty())
     return fail(h, MTP_E_CAPACITY, "the evaluation block does not fit in shared memory for this basis and max_nbr");
-  Shape best = *best_shape(h, shapes, fp64, false);
-  if (!schedule_uploaded(h, best.lanes, access_width(fp64, best.A))) {
+  Shape best = best_shape(shapes);
+  const DeviceSchedule* ds = programs_on_device(h, best.lanes, access_width(fp64, best.A), false);
+  if (!ds) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) cudaGetLastError();
-    if (cs != cudaStreamCaptureStatusNone)
-      if (const Shape* ready = best_shape(h, shapes, fp64, true)) best = *ready;
+    if (cs != cudaStreamCaptureStatusNone) {
+      const Shape ready = best_uploaded_shape(h, shapes, fp64, &ds);
+      if (ds) best = ready;
+    }
   }
-  const DeviceSchedule* ds = nullptr;
-  st = get_schedule(h, best.lanes, access_width(fp64, best.A), &ds);
-  if (st != MTP_OK) return st;
+  if (!ds && (st = get_schedule(h, best.lanes, access_width(fp64, best.A), &ds)) != MTP_OK) return st;
   const long long groups = (natoms + best.A - 1) / best.A;
   const long long blocks = std::max(1LL, std::min<long long>(static_cast<long long>(best.bps) * h->sm_count, groups));
   if (vglobal && !h->d_vscratch) {
@@ -1618,34 +1641,14 @@ int mtp_compute_device_noalloc(mtp_handle* h, int natoms, int stride, const int*
   if (st != MTP_OK) return st;
   const bool fp64 = h->precision == MTP_PRECISION_FP64;
 
-  // launch shape from the schedules already on the device, each paired only
-  // with the atoms per block whose operand width its entry order was tuned
-  // for, within the handle's launch limits (mtp_set_launch); the value space
-  // must fit in shared memory (its global-memory form would need an allocation)
+  // launch shape within the handle's request whose programs are on the device;
+  // the value space must fit in shared memory (its global-memory form would need
+  // an allocation)
+  std::vector<Shape> shapes;
+  st = shared_shapes(h, natoms, stride, fp64, &shapes);
+  if (st != MTP_OK) return st;
   const DeviceSchedule* ds = nullptr;
-  int lanes = 0, A = 1, bps = 0;
-  double best = 0.0;
-  for (const auto& kv : h->scheds) {
-    const DevModel md = make_model(h, kv.second);
-    const int sl = kv.second.sched.lanes;
-    if (h->threads > 0 && sl > h->threads) continue;
-    for (int a : {4, 2, 1}) {
-      if (!eval_variant_exists(fp64, false, a)) continue;
-      if (h->apb > 0 && a != h->apb) continue;
-      if (kv.second.sched.width != access_width(fp64, a)) continue;
-      int b = eval_blocks_per_sm(md, stride, sl, fp64, false, a);
-      if (h->blocks_per_sm > 0) b = std::min(b, h->blocks_per_sm);
-      if (b <= 0) continue;
-      const double est = launch_estimate(h->pot, fp64, sl, a, b, h->sm_count, natoms);
-      if (!ds || est < best) {
-        best = est;
-        ds = &kv.second;
-        lanes = sl;
-        A = a;
-        bps = b;
-      }
-    }
-  }
+  const Shape shape = best_uploaded_shape(h, shapes, fp64, &ds);
   if (!ds)
     return fail(h, MTP_E_CAPACITY,
                 "no uploaded schedule gives a shared-memory launch within the handle's launch limits (either the "
@@ -1681,11 +1684,11 @@ int mtp_compute_device_noalloc(mtp_handle* h, int natoms, int stride, const int*
   io.pair_grad = grad;
   io.err = h->d_err;
   io.vscratch = nullptr;
-  const long long groups = (static_cast<long long>(natoms) + A - 1) / A;
-  const int blocks = static_cast<int>(std::max(1LL, std::min<long long>(static_cast<long long>(bps) * h->sm_count,
+  const long long groups = (static_cast<long long>(natoms) + shape.A - 1) / shape.A;
+  const int blocks = static_cast<int>(std::max(1LL, std::min<long long>(static_cast<long long>(shape.bps) * h->sm_count,
                                                                          groups)));
   MTP_CUDA(h, launch_incoming(natoms, stride, d_js, d_jtypes, d_counts, in_cnt, in_ptr, in_slot, blk, false, h->stream));
-  MTP_CUDA(h, launch_eval(md, io, lanes, blocks, fp64, false, A, h->stream));
+  MTP_CUDA(h, launch_eval(md, io, shape.lanes, blocks, fp64, false, shape.A, h->stream));
   MTP_CUDA(h, launch_force_gather(natoms, stride, d_rijs, d_counts, grad, in_ptr, in_slot, true, d_forces, wown, nullptr,
                                   h->stream));
   st = write_totals(h, natoms, energy, wown, partials, tot, d_energy, d_virial);

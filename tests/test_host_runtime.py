@@ -65,6 +65,23 @@ class Handle:
                                        virial or b["virial"], None, None)
         return st, self.log()
 
+    def adjoint(self, n):
+        b = self.buf
+        if "cfg" not in b:
+            b.update(cfg=self.alloc(4 * n), volumes=self.alloc(8), gE=self.alloc(8), gF=self.alloc(24 * n),
+                     gS=self.alloc(48), gspecies=self.alloc(1 << 16), gmoment=self.alloc(1 << 16),
+                     gradial=self.alloc(1 << 16))
+        return self.L.mtp_adjoint_batch_device(self.h, n, self.stride, 1, b["itypes"], b["rijs"], b["js"],
+                                               b["jtypes"], b["counts"], b["cfg"], b["volumes"], b["gE"], b["gF"],
+                                               b["gS"], b["gspecies"], b["gmoment"], b["gradial"])
+
+    def noalloc(self, n):
+        b = self.buf
+        self.L.fake_clear()
+        st = self.L.mtp_compute_device_noalloc(self.h, n, self.stride, b["itypes"], b["rijs"], b["js"], b["jtypes"],
+                                               b["counts"], b["energy"], b["forces"], b["virial"])
+        return st, self.log()
+
     def captured(self, n, **kw):
         """The same call while its stream is captured."""
         self.L.fake_capture(self.stream, 1)
@@ -128,3 +145,14 @@ def test_capture_in_shared_memory_uses_the_programs_that_are_there(lib):
         st, log = h.captured(100)
         assert st == 0 and "in-capture" not in log, h.error()
         assert (h.launch()["threads"], h.launch()["atoms"]) == (ran["threads"], ran["atoms"])
+
+
+def test_allocation_free_call_after_a_training_gradient(lib):
+    """The gradient's programs (ordered for 16-byte operands) serve rows that are
+    too long for four atoms per block, the width's own shape."""
+    with Handle(lib, L20, 100, 400, MIXED) as h:
+        assert h.noalloc(100)[0] != 0            # nothing uploaded
+        assert h.adjoint(100) == 0
+        st, log = h.noalloc(100)
+        assert st == 0, h.error()
+        assert "malloc" not in log and "k_mtp_eval" in log
