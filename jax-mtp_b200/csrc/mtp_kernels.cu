@@ -405,7 +405,10 @@ __device__ __forceinline__ double block_reduce_256(double v, double* red) {
 // over the lanes.  out[0..6] = totals, out[7] = the device error flags so far
 // (low 32 bits), so a host call reads both back with one copy; d_energy and
 // d_virial, where given, get theirs.  The ticket at out + 8 starts at zero and
-// ends at zero.  Two launches and two copies took 9 us of a 2,000-atom call.
+// wraps to zero after every grid's worth of blocks, also where launches on the
+// same scratch overlap (calls of the allocation-free path may race): such calls
+// spoil their own totals, not those of the calls after them.  Two launches and
+// two copies took 9 us of a 2,000-atom call.
 __global__ void k_totals(int natoms, const double* __restrict__ e, const double* __restrict__ w, double* partials,
                          double* out, const int* err, double* d_energy, double* d_virial) {
   __shared__ double red[7][8];
@@ -431,8 +434,7 @@ __global__ void k_totals(int natoms, const double* __restrict__ e, const double*
     __threadfence();
   }
   __syncthreads();
-  int* ticket = reinterpret_cast<int*>(out + 8);
-  if (threadIdx.x == 0) last = atomicAdd(ticket, 1) == static_cast<int>(gridDim.x) - 1;
+  if (threadIdx.x == 0) last = atomicInc(reinterpret_cast<unsigned*>(out + 8), gridDim.x - 1) == gridDim.x - 1;
   __syncthreads();
   if (!last) return;
   __threadfence();
@@ -448,7 +450,6 @@ __global__ void k_totals(int natoms, const double* __restrict__ e, const double*
     }
   } else if (lane == 0) {
     out[7] = __hiloint2double(0, *reinterpret_cast<const volatile int*>(err));
-    *ticket = 0;
   }
 }
 
