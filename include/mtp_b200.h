@@ -113,7 +113,11 @@ int mtp_get_info(const mtp_handle* h, int* out8);
 int mtp_get_stats(const mtp_handle* h, double* out4);
 
 /* Replace the coefficients (training updates): species [S], moment [Sa], radial [S*S*R*K]
- * in .mtp order.  Any pointer may be NULL to keep the current values. */
+ * in .mtp order.  Any pointer may be NULL to keep the current values.  Waits for
+ * the work on the handle's stream (the last one set, which must still exist) and,
+ * as a copy on the legacy default stream, for that of every blocking stream; work
+ * enqueued on another, non-blocking stream before a change of stream must be
+ * finished.  The call returns when the device holds the new values. */
 int mtp_set_coeffs(mtp_handle* h, const double* species_coeffs, const double* moment_coeffs,
                    const double* radial_coeffs);
 

@@ -156,3 +156,29 @@ def test_allocation_free_call_after_a_training_gradient(lib):
         st, log = h.noalloc(100)
         assert st == 0, h.error()
         assert "malloc" not in log and "k_mtp_eval" in log
+
+
+def test_coefficients_wait_for_work_on_the_stream_before(lib):
+    """An evaluation on the legacy default stream may still read the old values
+    when the handle has moved to its own, non-blocking stream."""
+    with Handle(lib, L16, 100, 12) as h:
+        lib.mtp_set_stream(h.h, None)
+        assert h.compute(100)[0] == 0
+        lib.mtp_use_own_stream(h.h)
+        lib.fake_clear()
+        species = (ctypes.c_double * 2)(1.0, 2.0)
+        assert lib.mtp_set_coeffs(h.h, species, None, None) == 0
+        lines = h.log().splitlines()
+        copy = next(i for i, x in enumerate(lines) if x.startswith("memcpy"))
+        waits = any(x == "synchronize stream (nil)" for x in lines[:copy])
+        assert waits or not lines[copy].startswith("memcpy-async"), lines
+
+
+def test_coefficients_refused_in_a_capture(lib):
+    with Handle(lib, L16, 100, 12) as h:
+        species = (ctypes.c_double * 2)(1.0, 2.0)
+        lib.fake_capture(h.stream, 1)
+        lib.fake_clear()
+        st = lib.mtp_set_coeffs(h.h, species, None, None)
+        lib.fake_capture(h.stream, 0)
+        assert st != 0 and "memcpy" not in h.log()
