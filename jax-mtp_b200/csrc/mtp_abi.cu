@@ -590,22 +590,24 @@ int run_device(mtp_handle* h, int natoms, int stride, const int* itypes, const d
   return MTP_OK;
 }
 
-// True where a kernel can write through p (device, managed or page-locked
-// host memory).
-bool device_writable(const void* p) {
+// True where this device's kernels can store doubles at p: aligned, and memory
+// of this device, managed or page-locked host memory (a peer's memory may not be
+// mapped here; a copy reaches it all the same).
+bool device_writable(const mtp_handle* h, const void* p) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  return a.type != cudaMemoryTypeUnregistered && a.devicePointer == p;
+  if (reinterpret_cast<uintptr_t>(p) % alignof(double) != 0 || a.devicePointer != p) return false;
+  return a.type == cudaMemoryTypeDevice ? a.device == h->device : a.type != cudaMemoryTypeUnregistered;
 }
 
 // Totals into the caller's device buffers (null: not asked for), by the kernel
 // itself or, where it cannot write there, by copies that report the error.
 int write_totals(mtp_handle* h, int natoms, const double* site_energy, const double* wown, double* partials,
                  double* tot, double* d_energy, double* d_virial) {
-  const bool e = d_energy && device_writable(d_energy), v = d_virial && device_writable(d_virial);
+  const bool e = d_energy && device_writable(h, d_energy), v = d_virial && device_writable(h, d_virial);
   MTP_CUDA(h, launch_totals(natoms, site_energy, wown, partials, tot, h->d_err, e ? d_energy : nullptr,
                             v ? d_virial : nullptr, h->stream));
   if (d_energy && !e)

@@ -182,3 +182,25 @@ def test_coefficients_refused_in_a_capture(lib):
         st = lib.mtp_set_coeffs(h.h, species, None, None)
         lib.fake_capture(h.stream, 0)
         assert st != 0 and "memcpy" not in h.log()
+
+
+def _totals(log):
+    return re.search(r"totals energy (\S+) virial (\S+)", log).groups()
+
+
+def test_totals_of_another_device_are_copied(lib):
+    """Peer memory may not be mapped on this device: kernels do not store there."""
+    with Handle(lib, L16, 100, 12) as h:
+        e, v = h.alloc(8), h.alloc(48)
+        lib.fake_set_device(e, 1)
+        st, log = h.compute(100, energy=e, virial=v)
+        assert st == 0 and _totals(log) == ("(nil)", hex(v))
+        assert re.search(rf"memcpy-async {hex(e)} 8 ", log)
+
+
+def test_totals_at_odd_addresses_are_copied(lib):
+    with Handle(lib, L16, 100, 12) as h:
+        e, v = h.alloc(16) + 4, h.alloc(56) + 4
+        st, log = h.compute(100, energy=e, virial=v)
+        assert st == 0 and _totals(log) == ("(nil)", "(nil)")
+        assert re.search(rf"memcpy-async {hex(e)} 8 ", log) and re.search(rf"memcpy-async {hex(v)} 48 ", log)
