@@ -94,6 +94,7 @@ struct mtp_handle {
   double* d_rijs = nullptr;
   double *d_G = nullptr, *d_E = nullptr, *d_F = nullptr, *d_wown = nullptr, *d_vatom = nullptr;
   int *d_in_cnt = nullptr, *d_in_ptr = nullptr, *d_in_slot = nullptr, *d_blk = nullptr;
+  bool lists_sorted = true;   // false from building the incoming lists to the force gather that sorts them
   double *d_partials = nullptr, *d_tot = nullptr;
   int* d_err = nullptr;
   int* d_cfg_ptr = nullptr;
@@ -574,6 +575,7 @@ int run_device(mtp_handle* h, int natoms, int stride, const int* itypes, const d
       MTP_CUDA(h, cudaEventRecord(h->fork_event, h->stream));
       MTP_CUDA(h, cudaStreamWaitEvent(s, h->fork_event, 0));
     }
+    h->lists_sorted = false;
     MTP_CUDA(h, launch_incoming(natoms, stride, js, jtypes, counts, h->d_in_cnt, h->d_in_ptr, h->d_in_slot,
                                 h->d_blk, counted, s));
     if (fork) MTP_CUDA(h, cudaEventRecord(h->join_event, s));
@@ -586,7 +588,8 @@ int run_device(mtp_handle* h, int natoms, int stride, const int* itypes, const d
   if (e1) MTP_CUDA(h, cudaEventRecord(e1, h->stream));
   if (fork) MTP_CUDA(h, cudaStreamWaitEvent(h->stream, h->join_event, 0));
   MTP_CUDA(h, launch_force_gather(natoms, stride, rijs, counts, h->d_G, h->d_in_ptr, h->d_in_slot,
-                                  rebuild_incoming, forces, h->d_wown, vatom, h->stream));
+                                  !h->lists_sorted, forces, h->d_wown, vatom, h->stream));
+  h->lists_sorted = true;
   return MTP_OK;
 }
 
@@ -667,10 +670,12 @@ int run_host_pipelined_body(mtp_handle* h, int natoms, int stride, const int* it
     if (st != MTP_OK) return st;
   }
   if (e1) MTP_CUDA(h, cudaEventRecord(e1, s));
+  h->lists_sorted = false;
   MTP_CUDA(h, launch_incoming(natoms, stride, h->d_js, h->d_jtypes, counts ? h->d_counts : nullptr, h->d_in_cnt,
                               h->d_in_ptr, h->d_in_slot, h->d_blk, false, s));
   MTP_CUDA(h, launch_force_gather(natoms, stride, h->d_rijs, counts ? h->d_counts : nullptr, h->d_G, h->d_in_ptr,
                                   h->d_in_slot, true, h->d_F, h->d_wown, vatom, s));
+  h->lists_sorted = true;
   return MTP_OK;
 }
 

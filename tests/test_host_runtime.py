@@ -204,3 +204,16 @@ def test_totals_at_odd_addresses_are_copied(lib):
         st, log = h.compute(100, energy=e, virial=v)
         assert st == 0 and _totals(log) == ("(nil)", "(nil)")
         assert re.search(rf"memcpy-async {hex(e)} 8 ", log) and re.search(rf"memcpy-async {hex(v)} 48 ", log)
+
+
+def test_lists_of_a_call_that_failed_are_sorted_by_the_next(lib):
+    """The incoming lists are sorted by the force gather: a call that fails
+    between the two leaves that to the call that reuses them."""
+    with Handle(lib, L16, 2000, 12) as h:
+        lib.fake_fail_malloc(1)                  # the upload of the programs, after the lists
+        st, log = h.compute(2000)
+        assert st != 0 and "k_fill_incoming" in log and "k_force_gather" not in log
+        st, log = h.compute(2000, flags=EFLAG | VFLAG | REUSE_NEIGHBORS)
+        assert st == 0 and "k_fill_incoming" not in log and "k_force_gatherILb1E" in log
+        st, log = h.compute(2000, flags=EFLAG | VFLAG | REUSE_NEIGHBORS)
+        assert st == 0 and "k_force_gatherILb0E" in log
