@@ -243,11 +243,18 @@ int mtp_adjoint_batch_device(mtp_handle* h, int natoms, int nbr_stride, int ncon
                              const double* d_gS, double* d_gspecies, double* d_gmoment,
                              double* d_gradial);
 
-/* Launch shape of the evaluation kernel: at most this many threads per block
- * (128/256/512), blocks per SM (0 = as many as fit) and atoms evaluated
- * together per block (0 = any, or 1/2/4; FP64 supports 1/2).  Among the shapes
- * allowed, each call takes the one expected to be fastest for its number of
- * atoms; until this is called, all are.  Used by the autotuner. */
+/* Launch shape of the evaluation kernel: threads per block (128/256/512), blocks
+ * per SM (0 = as many as fit) and atoms evaluated together per block (0 = those
+ * that put the most atoms on an SM, or 1/2/4; FP64 supports 1/2).  Where the
+ * threads asked for do not fit, the next fewer that do are used; where no shape
+ * does, the value space moves to global memory (512 threads, one or two atoms).
+ * The shape then depends on nbr_stride but not on the number of atoms, and with
+ * it the rounding of an atom's energy and gradients: the same rows give the same
+ * bits in a system of any size.  Until this is called, each call takes the shape
+ * expected to be fastest for its number of atoms, and results of systems of
+ * different sizes agree to rounding.  Inside a stream capture a shape whose
+ * programs are not on the device yet gives way to one whose are.  The training
+ * gradient takes the threads from here as well. */
 int mtp_set_launch(mtp_handle* h, int threads_per_block, int blocks_per_sm, int atoms_per_block);
 
 /* Last evaluation kernel's launch: out5 = threads, blocks, dynamic shared bytes,

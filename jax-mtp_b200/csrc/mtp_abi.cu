@@ -384,11 +384,15 @@ int global_atoms(const mtp_handle* h, const DeviceSchedule& ds, bool fp64) {
   return global_space_bytes(h, ds, 2, fp64) <= h->l2_bytes / 4 * 3 ? 2 : 1;
 }
 
-// One launch shape that fits and its expected time (or, with the value space in
-// global memory, its expected number of one-atom rounds).
+// One launch shape that fits, and what the choice goes by: the least of the
+// expected times or, with the value space in global memory, of the expected
+// one-atom rounds.  A request (mtp_set_launch) goes by a rank that does not
+// depend on the number of atoms, so that an atom's rounding does not either: the
+// threads asked for, or else the next fewer that fit; of several atoms per block
+// the one with the most atoms in flight per SM, then the most warps.
 struct Shape {
   int lanes = 0, A = 1, bps = 0;
-  double est = 0.0;
+  double cost = 0.0;
 };
 
 // The shapes of the handle's request that fit for natoms, with the value space
@@ -402,7 +406,10 @@ int shared_shapes(mtp_handle* h, long long natoms, int stride, bool fp64, std::v
       int bps = 0;
       const int st = launch_occupancy(h, lanes, stride, fp64, false, A, &bps);
       if (st != MTP_OK) return st;
-      if (bps > 0) out->push_back({lanes, A, bps, launch_estimate(h->pot, fp64, lanes, A, bps, h->sm_count, natoms)});
+      if (bps <= 0) continue;
+      const double rank = 1e5 * (512 / lanes) - (1024 * A * bps + bps * lanes / 32);   // at most 16 atoms in flight
+      out->push_back({lanes, A, bps,
+                      h->threads > 0 ? rank : launch_estimate(h->pot, fp64, lanes, A, bps, h->sm_count, natoms)});
     }
   }
   return MTP_OK;
@@ -425,8 +432,11 @@ int global_shapes(mtp_handle* h, long long natoms, int stride, bool fp64, std::v
     int bps = 0;
     st = launch_occupancy(h, 512, stride, fp64, true, A, &bps);
     if (st != MTP_OK) return st;
+    if (bps <= 0) continue;
     const long long per = static_cast<long long>(A) * h->sm_count;
-    if (bps > 0) out->push_back({512, A, 1, static_cast<double>((natoms + per - 1) / per) * (A == 1 ? 1.0 : fp64 ? 1.78 : 1.09)});
+    const double rounds = static_cast<double>((natoms + per - 1) / per) * (A == 1 ? 1.0 : fp64 ? 1.78 : 1.09);
+    const double rank = A == (h->apb == 2 ? 2 : 1) ? 0.0 : 1.0;
+    out->push_back({512, A, 1, h->threads > 0 ? rank : rounds});
   }
   return MTP_OK;
 }
@@ -443,9 +453,9 @@ const DeviceSchedule* programs_on_device(const mtp_handle* h, int lanes, int wid
   return nullptr;
 }
 
-// The shape with the least estimate (the first of equal ones).
+// The shape of the least cost (the first of equal ones).
 const Shape& best_shape(const std::vector<Shape>& shapes) {
-  return *std::min_element(shapes.begin(), shapes.end(), [](const Shape& a, const Shape& b) { return a.est < b.est; });
+  return *std::min_element(shapes.begin(), shapes.end(), [](const Shape& a, const Shape& b) { return a.cost < b.cost; });
 }
 
 // The same for calls that can upload nothing: of the shapes whose programs are
@@ -457,7 +467,7 @@ Shape best_uploaded_shape(const mtp_handle* h, const std::vector<Shape>& shapes,
   for (const bool any_order : {false, true}) {
     for (const Shape& c : shapes) {
       const DeviceSchedule* p = programs_on_device(h, c.lanes, access_width(fp64, c.A), any_order);
-      if (!p || (*ds && c.est >= best.est)) continue;
+      if (!p || (*ds && c.cost >= best.cost)) continue;
       best = c;
       *ds = p;
     }
@@ -467,9 +477,8 @@ Shape best_uploaded_shape(const mtp_handle* h, const std::vector<Shape>& shapes,
 }
 
 // Launch shape for the evaluation kernel on natoms: the (lanes, atoms per
-// block) within the handle's request with the least expected time among those
-// whose value space fits in shared memory; when none fits, the value space
-// moves to global memory.  While the stream is being captured nothing can be
+// block) of the least cost (Shape) among those whose value space fits in shared
+// memory; when none fits, the value space moves to global memory.  While the stream is being captured nothing can be
 // uploaded, so a shape whose programs are not on the device yet gives way to
 // the best one whose are.
 int pick_launch(mtp_handle* h, long long natoms, int stride, const DeviceSchedule** ds_out, int* blocks_out, bool fp64,

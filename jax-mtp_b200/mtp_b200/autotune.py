@@ -39,7 +39,7 @@ from .engine import MTPEngine
 __all__ = ["tune", "tune_batch", "tune_adjoint", "tune_step", "apply_cached", "cache_key", "DEFAULT_CANDIDATES",
            "tile_candidates"]
 
-DEFAULT_CANDIDATES = ((128, 1), (256, 1), (512, 1), (128, 2), (256, 2), (512, 2), (256, 4), (512, 4))
+DEFAULT_CANDIDATES = ((128, 1), (256, 1), (512, 1), (128, 2), (256, 2), (512, 2), (128, 4), (256, 4), (512, 4))
 
 
 def _cache_path() -> str:

@@ -128,6 +128,10 @@ class MTPEngine:
         check(lib().mtp_use_own_stream(self._h), self._h)
 
     def set_launch(self, threads: int, blocks_per_sm: int = 0, atoms_per_block: int = 0) -> None:
+        """Pin the evaluation's launch shape (0 atoms: those that put the most on
+        an SM).  An atom's results are then the same bits in systems of any size;
+        without it each call takes the shape expected to be fastest for its
+        number of atoms."""
         check(lib().mtp_set_launch(self._h, int(threads), int(blocks_per_sm), int(atoms_per_block)), self._h)
 
     def launch(self) -> Dict[str, int]:

@@ -93,6 +93,9 @@ class Handle:
     def log(self):
         return self.L.fake_log().decode()
 
+    def set_launch(self, threads, atoms):
+        assert self.L.mtp_set_launch(self.h, threads, 0, atoms) == 0
+
     def launch(self):
         out = (ctypes.c_int * 5)()
         assert self.L.mtp_get_launch(self.h, out) == 0
@@ -217,3 +220,39 @@ def test_lists_of_a_call_that_failed_are_sorted_by_the_next(lib):
         assert st == 0 and "k_fill_incoming" not in log and "k_force_gatherILb1E" in log
         st, log = h.compute(2000, flags=EFLAG | VFLAG | REUSE_NEIGHBORS)
         assert st == 0 and "k_force_gatherILb0E" in log
+
+
+SIZES = (1, 100, 149, 593, 1185, 5000)
+
+
+@pytest.mark.parametrize("name,precision,threads,atoms", [(L20, MIXED, 512, 4), (L20, MIXED, 512, 1), (L20, FP64, 256, 2),
+                                                         (L24, MIXED, 512, 4), (L24, MIXED, 128, 2), (L16, MIXED, 128, 4),
+                                                         (L28, FP64, 512, 2), (L28, FP64, 512, 1)])
+def test_requested_shape_is_pinned(lib, name, precision, threads, atoms):
+    with Handle(lib, name, max(SIZES), 12, precision) as h:
+        h.set_launch(threads, atoms)
+        for n in SIZES:
+            assert h.compute(n)[0] == 0
+            assert (h.launch()["threads"], h.launch()["atoms"]) == (threads, atoms), n
+
+
+@pytest.mark.parametrize("name,precision", [(L16, FP64), (L20, MIXED), (L24, MIXED), (L28, FP64)])
+def test_requested_threads_fix_the_shape_for_every_size(lib, name, precision):
+    with Handle(lib, name, max(SIZES), 12, precision) as h:
+        for threads in (128, 256, 512):
+            h.set_launch(threads, 0)
+            shapes = set()
+            for n in SIZES:
+                assert h.compute(n)[0] == 0
+                shapes.add((h.launch()["threads"], h.launch()["atoms"]))
+            assert len(shapes) == 1
+            if name != L28:                      # in global memory: always 512 threads
+                assert shapes.pop()[0] == threads
+
+
+def test_requested_threads_that_do_not_fit_give_way_to_fewer(lib):
+    with Handle(lib, L28, 1000, 450, MIXED) as h:   # 512 threads fit up to 444 slots, 256 up to 452
+        h.set_launch(512, 1)
+        for n in (1, 1000):
+            assert h.compute(n)[0] == 0
+            assert (h.launch()["threads"], h.launch()["atoms"]) == (256, 1)
