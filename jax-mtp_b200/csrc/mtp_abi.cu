@@ -227,9 +227,6 @@ DevModel make_model(mtp_handle* h, const DeviceSchedule& ds) {
 // the schedule's entry order is tuned for).
 inline int access_width(bool fp64, int atoms_per_block) { return (fp64 ? 8 : 4) * atoms_per_block; }
 
-// Dynamic shared memory one block of this part can opt in to.
-constexpr size_t kMaxSmemPerBlock = 227 * 1024;
-
 // Schedule without programs for `lanes` threads: what a launch needs to be sized.
 int get_sizes(mtp_handle* h, int lanes, const DeviceSchedule** out) {
   auto it = h->sizes.find(lanes);

@@ -33,6 +33,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "mtp_model.hpp"
@@ -88,7 +89,8 @@ struct DevModel {
 struct DevIO {
   int natoms;
   int nbr_stride;
-  int n_pad;                // staging rows (>= max count, <= nbr_stride rounded)
+  int n_pad;                // slots of a staging row (>= max count, <= nbr_stride rounded)
+  int qs;                   // its stride (row_stride; set by launch_eval)
   const int* itypes;        // [natoms]
   const double* rijs;       // [natoms][nbr_stride][3]
   const int* jtypes;        // [natoms][nbr_stride]
@@ -112,9 +114,9 @@ constexpr int kVec = 16 / static_cast<int>(sizeof(T));
 // (radial functions f_mu, their derivatives, 1/d, the powers of u_x, u_y and
 // u_z), so that the basic moments read several neighbours with one 16-byte
 // load and the force phase, whose lanes are neighbours, reads without bank
-// conflicts.  The row stride is one 16-byte word more than a multiple of 128
-// bytes: 8 lanes that read 8 different rows at the same neighbour hit 8
-// different bank groups.  The force phase's chain copy of dE/dm ([atom][n3_len])
+// conflicts.  The row stride is an odd number of 16-byte words: 8 lanes that read
+// 8 rows in turn at the same neighbour hit 8 different bank groups (row_stride).
+// The force phase's chain copy of dE/dm ([atom][n3_len])
 // and its partial sums take the moment half of the value space (dead once the
 // reverse passes are done) when they fit there.
 struct SmemLayout {
@@ -140,18 +142,29 @@ __host__ __device__ inline int n3_group_warps(int NW, int A, int n_pad, int item
   return gw;
 }
 
-template <typename T>
-__host__ __device__ inline int staging_stride(int n_pad) {
-  // long rows are rounded less: their padding would cost more than the bank conflicts
-  constexpr int line = 8 * kVec<T>;
-  return n_pad <= 256 ? (n_pad + line - 1 - kVec<T>) / line * line + kVec<T> : (n_pad + 3) & ~3;
+// Shared memory of an SM, what a block takes beside its own, and what one block
+// can have.
+constexpr size_t kSmemPerSM = 228 * 1024, kSmemReserved = 1024, kMaxSmemPerBlock = 227 * 1024;
+
+// Stride of a staging row of n_pad slots.  An odd number of 16-byte words (see
+// SmemLayout); where that is one word more than the slots need and without it
+// another block fits on an SM (`total` gives a block's bytes for a stride), the
+// slots' own words, whose bank conflicts in the basic moments cost less.
+template <typename T, typename Total>
+inline int row_stride(int n_pad, int threads, const Total& total) {
+  const int words = (n_pad + kVec<T> - 1) / kVec<T>;
+  auto blocks = [&](int w) {   // by shared memory and by registers (128 a thread)
+    const size_t bytes = total(w * kVec<T>);
+    return bytes > kMaxSmemPerBlock ? 0 : std::min<size_t>(512 / threads, kSmemPerSM / (bytes + kSmemReserved));
+  };
+  return (blocks(words) > blocks(words | 1) ? words : words | 1) * kVec<T>;
 }
 
 template <typename T>
 __host__ __device__ inline SmemLayout smem_layout(int v_size, int M, int S, int R, int K, int D, int P, int n_list,
-                                                  int n3_len, int n_pad, int threads, int A) {
+                                                  int n3_len, int n_pad, int qs, int threads, int A) {
   SmemLayout L;
-  L.qs = staging_stride<T>(n_pad);
+  L.qs = qs;
   L.rows = 2 * R + 1 + 3 * (D + 1);
   L.rp = (R + kVec<T> - 1) / kVec<T> * kVec<T>;
   // an atom's copy starts one 16-byte word further into the banks than the one before
@@ -503,8 +516,8 @@ __device__ __forceinline__ void force_phase(const DevModel& md, const DevIO& io,
       const int word = md.n3_words[i];
       const int top = word & 15;
       P h, hz, hs;
-      if (MODE < 0) chain_dense<T, R>(top, dmc + (word >> 16) * 4, f, fp, uz, h, hz, hs);
-      else chain<T, R, MODE < 0 ? 0 : MODE>(top, dmc + (word >> 16) * 4, f, fp, uz, h, hz, hs);
+      if (MODE < 0) chain_dense<T, R>(top, dmc + (word >> 16) * 2, f, fp, uz, h, hz, hs);
+      else chain<T, R, MODE < 0 ? 0 : MODE>(top, dmc + (word >> 16) * 2, f, fp, uz, h, hz, hs);
       Hx = F::fma(Hx, ux, H);
       H = F::fma(H, ux, h);
       Hz = F::fma(Hz, ux, hz);
@@ -708,7 +721,7 @@ __global__ void __launch_bounds__(512) k_mtp_eval(DevModel md, DevIO io) {
   // held by lane p and shuffled out at the pass: no load before a pass
   const int my_wsteps = warp_steps_of_lane(md, tid, NT);
   const SmemLayout L = smem_layout<T>(kVGlobal ? 0 : md.v_size, md.M, md.S, md.R, md.K, md.D, md.P, md.n_list, md.n3_len,
-                                      io.n_pad, NT, A);
+                                      io.n_pad, io.qs, NT, A);
   T* V = kVGlobal ? reinterpret_cast<T*>(io.vscratch) + static_cast<size_t>(blockIdx.x) * md.v_size * A
                   : reinterpret_cast<T*>(smem + L.v);
   T* sRad = reinterpret_cast<T*>(smem + L.rad);

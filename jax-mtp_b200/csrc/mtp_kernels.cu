@@ -11,11 +11,21 @@ namespace mtp {
 // ---------------------------------------------------------------------------
 // evaluation kernel launch
 // ---------------------------------------------------------------------------
+template <typename T>
+static SmemLayout eval_layout(const DevModel& md, int n_pad, int threads, bool vglobal, int A) {
+  auto layout = [&](int qs) {
+    return smem_layout<T>(vglobal ? 0 : md.v_size, md.M, md.S, md.R, md.K, md.D, md.P, md.n_list, md.n3_len, n_pad, qs,
+                          threads, A);
+  };
+  return layout(row_stride<T>(n_pad, threads, [&](int qs) { return layout(qs).total; }));
+}
+
+static SmemLayout eval_layout(const DevModel& md, int n_pad, int threads, bool fp64, bool vglobal, int A) {
+  return fp64 ? eval_layout<double>(md, n_pad, threads, vglobal, A) : eval_layout<float>(md, n_pad, threads, vglobal, A);
+}
+
 size_t eval_smem_bytes(const DevModel& md, int n_pad, int threads, bool fp64, bool vglobal, int A) {
-  const int vs = vglobal ? 0 : md.v_size;
-  SmemLayout L = fp64 ? smem_layout<double>(vs, md.M, md.S, md.R, md.K, md.D, md.P, md.n_list, md.n3_len, n_pad, threads, A)
-                      : smem_layout<float>(vs, md.M, md.S, md.R, md.K, md.D, md.P, md.n_list, md.n3_len, n_pad, threads, A);
-  return L.total;
+  return eval_layout(md, n_pad, threads, fp64, vglobal, A).total;
 }
 
 namespace {
@@ -36,7 +46,7 @@ cudaError_t ensure_smem_limit(size_t bytes) {
 template <typename T, bool G, int A>
 int occupancy_t(size_t bytes, int threads) {
   int nb = 0;
-  if (bytes > 227 * 1024) return 0;
+  if (bytes > kMaxSmemPerBlock) return 0;
   if (ensure_smem_limit<T, G, A>(bytes) != cudaSuccess) {
     cudaGetLastError();
     return 0;
@@ -83,10 +93,12 @@ int eval_blocks_per_sm(const DevModel& md, int n_pad, int threads, bool fp64, bo
 cudaError_t launch_eval(const DevModel& md, const DevIO& io, int threads, int blocks, bool fp64, bool vglobal, int A,
                         cudaStream_t st) {
   if (io.natoms <= 0) return cudaSuccess;
-  const size_t bytes = eval_smem_bytes(md, io.n_pad, threads, fp64, vglobal, A);
+  const SmemLayout L = eval_layout(md, io.n_pad, threads, fp64, vglobal, A);
+  DevIO rows = io;
+  rows.qs = L.qs;
 #define X(T, G, AA) \
   if ((fp64 == std::is_same<T, double>::value) && vglobal == G && A == AA) \
-    return launch_t<T, G, AA>(md, io, threads, blocks, bytes, st);
+    return launch_t<T, G, AA>(md, rows, threads, blocks, L.total, st);
   MTP_EVAL_VARIANTS(X)
 #undef X
   return cudaErrorInvalidValue;

@@ -448,7 +448,7 @@ int adjoint_layout(const Potential& pot, std::vector<int>& dm_pos) {
             if (it == basic_of.end()) ok = false;   // a hole: another structure
             else pos[it->second] = next++, ++found;
           }
-        next = (next + 3) & ~3;
+        next = (next + 1) & ~1;
       }
     if (!ok || found != B) continue;               // found < B: basic moments outside the pattern
     for (int k = 0; k < B; ++k) dm_pos[k] = pos[k];
@@ -569,9 +569,9 @@ bool build_schedule(const Potential& pot, int lanes, Schedule& s, std::string& e
         }
       }
       const int n = static_cast<int>(s.n3_src.size()) - first;
-      while (s.n3_src.size() % 4) s.n3_src.push_back(-1);
+      if (s.n3_src.size() % 2) s.n3_src.push_back(-1);
       // multiply-adds of the terms and Horner steps, 16-byte loads, the rest of a pair
-      chains.push_back({top | (a << 4) | (b << 8) | ((first / 4) << 16), 2 * n + 3 * (top + 1) + n / 4 + 12});
+      chains.push_back({top | (a << 4) | (b << 8) | ((first / 2) << 16), 2 * n + 3 * (top + 1) + n / 4 + 12});
     }
   s.n3_len = static_cast<int>(s.n3_src.size());
   long all = 0;

@@ -98,14 +98,14 @@ struct Schedule {
   // chain_mode >= 0: a level-structured basis (adjoint_layout) whose step k has
   // the radial functions mu < min(R, (k + chain_mode) / 2 + 1); -1: every step
   // has all R (adjoint 0 where the basis has no moment).  Chain slots are
-  // steps in order, radial functions within a step, each chain padded to a
-  // multiple of four; n3_src[slot] is the adjoint position it copies, or -1.
+  // steps in order, radial functions within a step, each chain padded to an
+  // even length (16 bytes of its copy); n3_src[slot] is the adjoint position it copies, or -1.
   int chain_mode = -1;
   int n3_len = 0;
   std::vector<int> n3_src;      // [n3_len]
   // dE/dm of moment k lives at v_dm + dm_pos[k]; the adjoint region ends at v_part
   std::vector<int> dm_pos;
-  // One word per chain, top | a << 4 | b << 8 | (first slot / 4) << 16, and the
+  // One word per chain, top | a << 4 | b << 8 | (first slot / 2) << 16, and the
   // list cut into W = 1, 2, 4, 8 and 16 runs of about equal cost (one per warp
   // of a group): run w of W is n3_words[n3_off[o + w] .. n3_off[o + w + 1])
   // with o = W - 1 + log2 W.
@@ -147,8 +147,8 @@ double emulate_schedule(const Potential& pot, const Schedule& s, std::vector<dou
 // are those with a + b + c <= D and mu < min(R, (D - a - b - c + o) / 2 + 1)
 // (the MLIP templates up to level 24: o = 0; 26 and 28: o = 1 and 2, with six
 // radial functions), else -1.  On such a basis the basic moments' adjoints
-// take their force-phase chain slots as positions (each chain padded to a
-// multiple of four) and the others follow, so the copy into chain slots is a
+// take their force-phase chain slots as positions (each chain padded to an even
+// length) and the others follow, so the copy into chain slots is a
 // copy in a row; otherwise dm_pos[k] = k.
 int adjoint_layout(const Potential& pot, std::vector<int>& dm_pos);
 

@@ -26,10 +26,10 @@ struct TrainSmem {
 };
 
 template <typename T>
-__host__ __device__ inline TrainSmem train_layout(const DevModel& md, bool vglobal, int n_pad, int threads) {
+__host__ __device__ inline TrainSmem train_layout(const DevModel& md, bool vglobal, int n_pad, int qs, int threads) {
   const int S = md.S, R = md.R, K = md.K, D = md.D;
   TrainSmem L;
-  L.qs = staging_stride<T>(n_pad);
+  L.qs = qs;
   L.f = 0;
   L.fp = R;
   L.phi = 2 * R;
@@ -200,7 +200,7 @@ __device__ __forceinline__ void sensitivities(const DevModel& md, const TrainSme
     for (int i = i0; i < iend; ++i) {
       const int word = md.n3_words[i];
       const int top = word & 15, ea = (word >> 4) & 15, eb = (word >> 8) & 15;
-      const double2* lt = reinterpret_cast<const double2*>(smem + L.chain) + (word >> 16) * 4;
+      const double2* lt = reinterpret_cast<const double2*>(smem + L.chain) + (word >> 16) * 2;
       const double xa = px[ea * qs], yb = py[eb * qs], xy = xa * yb;
       const double dxy = ea * px[max(ea - 1, 0) * qs] * dux * yb + eb * py[max(eb - 1, 0) * qs] * duy * xa;
       double cd = top;
@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
   const int NT = blockDim.x, tid = threadIdx.x;
   const int my_wsteps = warp_steps_of_lane(md, tid, NT);
   const int S = md.S, R = md.R, K = md.K, P = md.P, D1 = md.D + 1;
-  const TrainSmem L = train_layout<T>(md, kVGlobal, n_pad, NT);
+  const TrainSmem L = train_layout<T>(md, kVGlobal, n_pad, io.qs, NT);
   using T2 = typename Dual2<T>::type;
   // program entries in flight per thread; with the value space in global
   // memory their operand gathers are issued before any of their flushes
@@ -628,7 +628,7 @@ static cudaError_t adjoint_smem_limit(size_t bytes) {
 
 template <bool G>
 static int adjoint_occupancy(size_t bytes, int threads) {
-  if (bytes > 227 * 1024) return 0;
+  if (bytes > kMaxSmemPerBlock) return 0;
   int nb = 0;
   if (adjoint_smem_limit<G>(bytes) != cudaSuccess) {
     cudaGetLastError();
@@ -641,28 +641,36 @@ static int adjoint_occupancy(size_t bytes, int threads) {
   return nb;
 }
 
+static TrainSmem adjoint_layout_of(const DevModel& md, bool vglobal, int n_pad, int threads) {
+  const int qs = row_stride<double>(
+      n_pad, threads, [&](int q) { return train_layout<double>(md, vglobal, n_pad, q, threads).total; });
+  return train_layout<double>(md, vglobal, n_pad, qs, threads);
+}
+
 bool adjoint_fits_shared(const DevModel& md, int n_pad, int threads) {
-  const TrainSmem L = train_layout<double>(md, false, n_pad, threads);
+  const TrainSmem L = adjoint_layout_of(md, false, n_pad, threads);
   return adjoint_occupancy<false>(L.total, threads) > 0;
 }
 
-cudaError_t launch_adjoint(const DevModel& md, const TrainIO& io, int threads, int sm_count, TrainWorkspace& ws,
+cudaError_t launch_adjoint(const DevModel& md, const TrainIO& in, int threads, int sm_count, TrainWorkspace& ws,
                            double* gspecies, double* gmoment, double* gradial, cudaStream_t st, std::string& err) {
-  const int n_pad = io.nbr_stride;
+  const int n_pad = in.nbr_stride;
   const int nrad = md.S * md.S * md.R * md.K;
   const int np = md.Sa + md.S + nrad;
   bool vglobal = false;
-  TrainSmem L = train_layout<double>(md, false, n_pad, threads);
+  TrainSmem L = adjoint_layout_of(md, false, n_pad, threads);
   int bps = adjoint_occupancy<false>(L.total, threads);
   if (bps <= 0) {
     vglobal = true;
-    L = train_layout<double>(md, true, n_pad, threads);
+    L = adjoint_layout_of(md, true, n_pad, threads);
     bps = adjoint_occupancy<true>(L.total, threads);
   }
   if (bps <= 0) {
     err = "the adjoint block does not fit in shared memory for this basis and nbr_stride";
     return cudaSuccess;
   }
+  TrainIO io = in;
+  io.qs = L.qs;
   int blocks = std::max(1, std::min(io.natoms, bps * sm_count));
   if (vglobal) {
     // the blocks' global value spaces should stay resident in L2: cap their

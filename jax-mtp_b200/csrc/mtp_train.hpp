@@ -27,6 +27,7 @@ namespace mtp {
 
 struct TrainIO {
   int natoms, nbr_stride, nconfig;
+  int qs;                 // stride of a staging row (set by launch_adjoint)
   const int* itypes;
   const double* rijs;
   const int* js;
@@ -54,7 +55,7 @@ void train_free(TrainWorkspace& w);
 bool adjoint_fits_shared(const DevModel& md, int n_pad, int threads);
 
 // Runs the adjoint kernel (FP64) and the fixed-order reduction into the outputs.
-cudaError_t launch_adjoint(const DevModel& md, const TrainIO& io, int threads, int sm_count, TrainWorkspace& ws,
+cudaError_t launch_adjoint(const DevModel& md, const TrainIO& in, int threads, int sm_count, TrainWorkspace& ws,
                            double* gspecies, double* gmoment, double* gradial, cudaStream_t st, std::string& err);
 
 }  // namespace mtp

@@ -256,3 +256,21 @@ def test_requested_threads_that_do_not_fit_give_way_to_fewer(lib):
         for n in (1, 1000):
             assert h.compute(n)[0] == 0
             assert (h.launch()["threads"], h.launch()["atoms"]) == (256, 1)
+
+
+# Rows that each shape took, and blocks per SM, with neighbour-major staging rows:
+# (potential, precision, threads, atoms per block, slots, blocks per SM)
+ROWS = [(L16, MIXED, 128, 4, 80, 4), (L16, MIXED, 128, 4, 116, 3), (L16, MIXED, 256, 4, 183, 2), (L16, MIXED, 128, 2, 184, 4),
+        (L16, FP64, 128, 2, 80, 4), (L16, FP64, 256, 2, 170, 2), (L20, MIXED, 256, 4, 88, 2), (L20, MIXED, 128, 4, 40, 3),
+        (L20, FP64, 256, 2, 100, 2), (L20, FP64, 128, 2, 45, 3), (L24, MIXED, 512, 4, 72, 1), (L24, MIXED, 256, 4, 77, 1),
+        (L24, MIXED, 128, 4, 80, 1), (L24, MIXED, 256, 2, 74, 2), (L24, MIXED, 128, 2, 77, 2), (L24, FP64, 512, 2, 76, 1),
+        (L24, FP64, 256, 2, 82, 1), (L24, FP64, 128, 2, 85, 1), (L28, MIXED, 512, 1, 409, 1)]
+
+
+@pytest.mark.parametrize("name,precision,threads,atoms,slots,per_sm", ROWS)
+def test_row_lengths_that_fit(lib, name, precision, threads, atoms, slots, per_sm):
+    with Handle(lib, name, 2, slots, precision) as h:
+        h.set_launch(threads, atoms)
+        assert h.compute(2)[0] == 0
+        got = h.launch()
+        assert (got["threads"], got["atoms"]) == (threads, atoms) and got["per_sm"] >= per_sm
