@@ -121,7 +121,7 @@ constexpr int kVec = 16 / static_cast<int>(sizeof(T));
 // reverse passes are done) when they fit there.
 struct SmemLayout {
   int qs;         // stride of a staging row
-  int rows;       // staging rows per atom: R (f), R (f'), 1 (1/d), 3 (D + 1) (powers)
+  int rows;       // staging rows per atom: R (f), R (f'), 1 (1/d), 3 power_rows(D)
   int rp;         // radial functions per coefficient row (R rounded up to kVec)
   int n3s;        // stride of one atom's chain copy
   size_t v, rad, st, slot, mono, dmc, n3p, red, cnt, total;
@@ -129,6 +129,11 @@ struct SmemLayout {
 
 // Force-phase words: one FP64 value or a pair of FP32 ones (struct Force).
 constexpr int kForceBytes = 8;
+
+// Powers of a unit vector component in the staging: up to the degree, and the
+// first one always (levels 2 and 4 have scalar moments only, but their forces
+// point along the unit vector too).
+__host__ __device__ inline int power_rows(int D) { return D < 1 ? 2 : D + 1; }
 
 // Warps that share one chunk of neighbours (32 lanes of `items`) in the force
 // phase: as few as let every chunk of the block have a group (no partial sums
@@ -165,7 +170,7 @@ __host__ __device__ inline SmemLayout smem_layout(int v_size, int M, int S, int 
                                                   int n3_len, int n_pad, int qs, int threads, int A) {
   SmemLayout L;
   L.qs = qs;
-  L.rows = 2 * R + 1 + 3 * (D + 1);
+  L.rows = 2 * R + 1 + 3 * power_rows(D);
   L.rp = (R + kVec<T> - 1) / kVec<T> * kVec<T>;
   // an atom's copy starts one 16-byte word further into the banks than the one before
   L.n3s = ((n3_len + 15) & ~15) + 2;
@@ -480,7 +485,7 @@ __device__ __forceinline__ void force_phase(const DevModel& md, const DevIO& io,
   const int lg = 31 - __clz(GW);
   // offsets of the cut into 2^lg runs follow those of the cuts into fewer
   const int i0 = md.n3_off[GW - 1 + lg + wg], i1 = md.n3_off[GW + lg + wg];
-  const int D1 = md.D + 1, qs = L.qs, n_pad = io.n_pad;
+  const int D1 = power_rows(md.D), qs = L.qs, n_pad = io.n_pad;
   P* part = reinterpret_cast<P*>(smem + L.n3p);
   int J = 0;
 #pragma unroll
@@ -732,7 +737,7 @@ __global__ void __launch_bounds__(512) k_mtp_eval(DevModel md, DevIO io) {
   const int n_pad = io.n_pad, qs = L.qs;
   constexpr int VW = kVec<T>;
 
-  const int S = md.S, R = md.R, K = md.K, P = md.P, D1 = md.D + 1;
+  const int S = md.S, R = md.R, K = md.K, P = md.P, D1 = power_rows(md.D);
   // per-block constants; radial coefficients as [pair][n][mu], rows padded to whole 16-byte words
   for (int x = tid; x < S * S * K * L.rp; x += NT) {
     const int mu = x % L.rp, n = x / L.rp % K, st = x / (L.rp * K);
