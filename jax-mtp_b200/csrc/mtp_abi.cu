@@ -283,10 +283,11 @@ int get_schedule(mtp_handle* h, int lanes, int width, const DeviceSchedule** out
   return MTP_OK;
 }
 
-// Send the coefficients.  A blocking copy on the legacy default stream, after
-// the work on the handle's stream: it also waits for blocking streams that the
-// handle worked on before (kernels there may still read the old values), and
-// later work sees the new ones on any stream, graph replays included.
+// Send the coefficients, after the work on the handle's stream, by a copy on the
+// legacy default stream: it also comes after the work of blocking streams that
+// the handle used before (kernels there may still read the old values).  The
+// copy is waited for: later work sees the new values on any stream, graph
+// replays included.
 int upload_coeffs(mtp_handle* h) {
   const Potential& p = h->pot;
   double* o = h->h_coef;
@@ -296,7 +297,8 @@ int upload_coeffs(mtp_handle* h) {
   std::fill(o, o + h->nseed, 0.0);
   for (int a = 0; a < p.Sa; ++a) o[h->seed_of[a]] += p.moment[a];
   const size_t n = (o - h->h_coef) + h->nseed;
-  MTP_CUDA(h, cudaMemcpy(h->d_coef, h->h_coef, n * sizeof(double), cudaMemcpyHostToDevice));
+  MTP_CUDA(h, cudaMemcpyAsync(h->d_coef, h->h_coef, n * sizeof(double), cudaMemcpyHostToDevice, nullptr));
+  MTP_CUDA(h, cudaStreamSynchronize(nullptr));
   return MTP_OK;
 }
 
@@ -1038,8 +1040,9 @@ int mtp_get_stats(const mtp_handle* h, double* out4) {
 
 int mtp_set_coeffs(mtp_handle* h, const double* species, const double* moment, const double* radial) {
   if (!h) return MTP_E_INVALID;
-  // (refused inside a stream capture, before the host's values change)
-  MTP_CUDA(h, cudaStreamSynchronize(h->stream));
+  // (refused inside a stream capture, before the host's values change; the
+  // legacy default stream cannot be captured and is the copy's own)
+  if (h->stream) MTP_CUDA(h, cudaStreamSynchronize(h->stream));
   Potential& p = h->pot;
   if (species) std::copy(species, species + p.S, p.species.begin());
   if (moment) std::copy(moment, moment + p.Sa, p.moment.begin());

@@ -172,9 +172,8 @@ def test_coefficients_wait_for_work_on_the_stream_before(lib):
         species = (ctypes.c_double * 2)(1.0, 2.0)
         assert lib.mtp_set_coeffs(h.h, species, None, None) == 0
         lines = h.log().splitlines()
-        copy = next(i for i, x in enumerate(lines) if x.startswith("memcpy"))
-        waits = any(x == "synchronize stream (nil)" for x in lines[:copy])
-        assert waits or not lines[copy].startswith("memcpy-async"), lines
+        copy = next(x for x in lines if x.startswith("memcpy"))
+        assert copy.endswith("stream (nil)") and lines[-1] == "synchronize stream (nil)", lines
 
 
 def test_coefficients_refused_in_a_capture(lib):
