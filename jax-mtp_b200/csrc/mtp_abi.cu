@@ -84,8 +84,10 @@ struct mtp_handle {
   double *d_coef = nullptr, *h_coef = nullptr;
   double *d_radial = nullptr, *d_species = nullptr, *d_theta = nullptr, *d_seed_val = nullptr;   // parts of d_coef
   std::vector<int> seed_of;    // [Sa] seed that each mapped moment adds to
-  int *d_mapping = nullptr, *d_seed_idx = nullptr, *d_zero = nullptr, *d_abc = nullptr, *d_mk = nullptr;
-  // tables that are the same for every schedule of the potential
+  int *d_mapping = nullptr, *d_seed_idx = nullptr;
+  // tables that are the same for every schedule of the potential, and the buffer
+  // that holds them (upload_tables)
+  int *d_tables = nullptr, *d_zero = nullptr, *d_abc = nullptr, *d_mk = nullptr;
   int *d_dm_pos = nullptr, *d_dm_zero = nullptr, *d_n3_src = nullptr;
   int *d_mono_word = nullptr, *d_mono_list = nullptr;
   int nseed = 0;
@@ -240,6 +242,32 @@ int get_sizes(mtp_handle* h, int lanes, const DeviceSchedule** out) {
   return MTP_OK;
 }
 
+// The tables that are the same for every schedule of the potential, in one
+// buffer: on the device as a whole or, after a failure, not at all.
+int upload_tables(mtp_handle* h, const Schedule& t) {
+  const std::pair<int**, const std::vector<int>*> tables[] = {
+      {&h->d_abc, &t.mono_abc}, {&h->d_mk, &t.mono_k},   {&h->d_dm_pos, &t.dm_pos},     {&h->d_zero, &t.zero_list},
+      {&h->d_dm_zero, &t.dm_zero}, {&h->d_n3_src, &t.n3_src}, {&h->d_mono_word, &t.mono_word},
+      {&h->d_mono_list, &t.mono_list}};
+  std::vector<int> all;
+  std::vector<size_t> at;
+  for (const auto& x : tables) {
+    at.push_back(all.size());
+    all.insert(all.end(), x.second->begin(), x.second->end());
+    all.resize((all.size() + 63) / 64 * 64);   // each at a 256-byte boundary
+  }
+  int* d = nullptr;
+  MTP_CUDA(h, dalloc(&d, all.size()));
+  const cudaError_t e = cudaMemcpy(d, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    cudaFree(d);
+    return cuda_fail(h, e, "upload tables");
+  }
+  h->d_tables = d;
+  for (size_t k = 0; k < at.size(); ++k) *tables[k].first = d + at[k];
+  return MTP_OK;
+}
+
 // Schedule for `lanes` threads and `width`-byte operand accesses, built and
 // uploaded on first use; refine_schedule runs where the value space can sit in
 // shared memory (bank order matters only there).
@@ -251,17 +279,9 @@ int get_schedule(mtp_handle* h, int lanes, int width, const DeviceSchedule** out
     std::string err;
     if (!build_schedule(h->pot, lanes, ds.sched, err, width)) return fail(h, MTP_E_FORMAT, err);
     if (static_cast<size_t>(ds.sched.v_size) * width <= kMaxSmemPerBlock) refine_schedule(ds.sched);
-    if (h->d_abc == nullptr) {
-      const Schedule& t = ds.sched;
-      const std::pair<int**, const std::vector<int>*> tables[] = {
-          {&h->d_abc, &t.mono_abc}, {&h->d_mk, &t.mono_k},   {&h->d_dm_pos, &t.dm_pos},     {&h->d_zero, &t.zero_list},
-          {&h->d_dm_zero, &t.dm_zero}, {&h->d_n3_src, &t.n3_src}, {&h->d_mono_word, &t.mono_word},
-          {&h->d_mono_list, &t.mono_list}};
-      for (const auto& x : tables) {
-        MTP_CUDA(h, dalloc(x.first, x.second->size()));
-        if (!x.second->empty())
-          MTP_CUDA(h, cudaMemcpy(*x.first, x.second->data(), x.second->size() * sizeof(int), cudaMemcpyHostToDevice));
-      }
+    if (h->d_tables == nullptr) {
+      const int st = upload_tables(h, ds.sched);
+      if (st != MTP_OK) return st;
     }
     const auto& ent = ds.sched.entries;
     std::vector<int> ws;
@@ -311,9 +331,7 @@ void free_handle(mtp_handle* h) {
   }
   F(h->d_coef);
   if (h->h_coef) cudaFreeHost(h->h_coef);
-  F(h->d_mapping); F(h->d_seed_idx); F(h->d_zero); F(h->d_abc); F(h->d_mk); F(h->d_dm_pos);
-  F(h->d_dm_zero); F(h->d_n3_src);
-  F(h->d_mono_word); F(h->d_mono_list);
+  F(h->d_mapping); F(h->d_seed_idx); F(h->d_tables);
   F(h->d_itypes); F(h->d_js); F(h->d_jtypes); F(h->d_counts); F(h->d_rijs);
   F(h->d_G); F(h->d_E); F(h->d_F); F(h->d_wown); F(h->d_vatom);
   F(h->d_in_cnt); F(h->d_in_ptr); F(h->d_in_slot); F(h->d_blk);

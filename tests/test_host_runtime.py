@@ -250,7 +250,7 @@ def test_requested_threads_fix_the_shape_for_every_size(lib, name, precision):
 
 
 def test_requested_threads_that_do_not_fit_give_way_to_fewer(lib):
-    with Handle(lib, L28, 1000, 450, MIXED) as h:   # 512 threads fit up to 444 slots, 256 up to 452
+    with Handle(lib, L28, 1000, 450, MIXED) as h:   # 512 threads fit up to 448 slots, 256 up to 452
         h.set_launch(512, 1)
         for n in (1, 1000):
             assert h.compute(n)[0] == 0
@@ -273,3 +273,19 @@ def test_row_lengths_that_fit(lib, name, precision, threads, atoms, slots, per_s
         assert h.compute(2)[0] == 0
         got = h.launch()
         assert (got["threads"], got["atoms"]) == (threads, atoms) and got["per_sm"] >= per_sm
+
+
+def test_failed_upload_of_the_tables_is_made_up_for(lib):
+    """Whichever allocation of the first call fails, the next call has all of them."""
+    live = lambda log: log.count("malloc 0x") - log.count("free 0x")
+    with Handle(lib, L16, 100, 12) as h:
+        whole = live(h.compute(100)[1])
+    for n in range(1, whole + 1):
+        with Handle(lib, L16, 100, 12) as h:
+            lib.fake_fail_malloc(n)
+            st, log = h.compute(100)
+            assert st != 0 and "malloc-failed" in log
+            left = live(log)
+            st, log = h.compute(100)
+            assert st == 0, h.error()
+            assert left + live(log) == whole, n
