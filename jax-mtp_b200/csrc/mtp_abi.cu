@@ -87,8 +87,7 @@ struct mtp_handle {
   int *d_mapping = nullptr, *d_seed_idx = nullptr;
   // tables that are the same for every schedule of the potential, and the buffer
   // that holds them (upload_tables)
-  int *d_tables = nullptr, *d_zero = nullptr, *d_abc = nullptr, *d_mk = nullptr;
-  int *d_dm_pos = nullptr, *d_dm_zero = nullptr, *d_n3_src = nullptr;
+  int *d_tables = nullptr, *d_zero = nullptr, *d_dm_zero = nullptr, *d_n3_src = nullptr;
   int *d_mono_word = nullptr, *d_mono_list = nullptr;
   int nseed = 0;
   // input / output / scratch buffers sized by the capacities
@@ -190,12 +189,9 @@ DevModel make_model(mtp_handle* h, const DeviceSchedule& ds) {
   md.nseed = h->nseed;
   md.zero_list = h->d_zero;
   md.nzero = static_cast<int>(s.zero_list.size());
-  md.mono_abc = h->d_abc;
-  md.mono_k = h->d_mk;
   md.mono_word = h->d_mono_word;
   md.mono_list = h->d_mono_list;
   md.n_list = static_cast<int>(s.mono_list.size());
-  md.dm_pos = h->d_dm_pos;
   md.dm_zero = h->d_dm_zero;
   md.ndm_zero = static_cast<int>(s.dm_zero.size());
   md.chain_mode = s.chain_mode;
@@ -204,7 +200,6 @@ DevModel make_model(mtp_handle* h, const DeviceSchedule& ds) {
   std::copy(s.n3_words.begin(), s.n3_words.end(), md.n3_words);
   std::copy(s.n3_off.begin(), s.n3_off.end(), md.n3_off);
   md.warp_steps = ds.d_warp_steps;
-  for (int v = 0; v <= s.D; ++v) md.nmu[v] = s.nmu[v];
   md.S = h->pot.S;
   md.R = h->pot.R;
   md.K = h->pot.K;
@@ -246,9 +241,8 @@ int get_sizes(mtp_handle* h, int lanes, const DeviceSchedule** out) {
 // buffer: on the device as a whole or, after a failure, not at all.
 int upload_tables(mtp_handle* h, const Schedule& t) {
   const std::pair<int**, const std::vector<int>*> tables[] = {
-      {&h->d_abc, &t.mono_abc}, {&h->d_mk, &t.mono_k},   {&h->d_dm_pos, &t.dm_pos},     {&h->d_zero, &t.zero_list},
-      {&h->d_dm_zero, &t.dm_zero}, {&h->d_n3_src, &t.n3_src}, {&h->d_mono_word, &t.mono_word},
-      {&h->d_mono_list, &t.mono_list}};
+      {&h->d_zero, &t.zero_list}, {&h->d_dm_zero, &t.dm_zero}, {&h->d_n3_src, &t.n3_src},
+      {&h->d_mono_word, &t.mono_word}, {&h->d_mono_list, &t.mono_list}};
   std::vector<int> all;
   std::vector<size_t> at;
   for (const auto& x : tables) {

@@ -63,8 +63,6 @@ struct DevModel {
   const int* seed_idx;      // [nseed]
   const double* seed_val;   // [nseed]
   const int* zero_list;     // [nzero]
-  const int* mono_abc;      // [P][4]
-  const int* mono_k;        // [P][kMaxR]
   const int* mono_word;     // [P] Schedule::mono_word
   const int* mono_list;     // [n_list] Schedule::mono_list
   int n_list;
@@ -80,8 +78,6 @@ struct DevModel {
   // possibly divergent branch)
   int n3_words[kMaxChains];
   unsigned char n3_off[kMaxRunOffsets];
-  const int* dm_pos;        // [M] adjoint position of each moment (Schedule::dm_pos)
-  int nmu[kMaxDegree + 1];  // radial functions with a basic moment of each degree
   int v_m, v_dm, n_dm, v_zero, v_one, v_size;  // n_dm: slots of the adjoint region
   double scaling, rmin, rmax;
 };

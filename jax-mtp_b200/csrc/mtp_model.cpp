@@ -539,13 +539,6 @@ bool build_schedule(const Potential& pot, int lanes, Schedule& s, std::string& e
     if (s.mono_k[kMaxR * p + mu] >= 0) { err = "duplicate row in alpha_index_basic"; return false; }
     s.mono_k[kMaxR * p + mu] = k;
   }
-  // radial functions per degree: nmu[v] = 1 + the largest mu of a basic
-  // moment of degree v (0 if none)
-  s.nmu.assign(s.D + 1, 0);
-  for (int k = 0; k < B; ++k) {
-    const int v = pot.basic[4 * k + 1] + pot.basic[4 * k + 2] + pot.basic[4 * k + 3];
-    s.nmu[v] = std::max(s.nmu[v], pot.basic[4 * k] + 1);
-  }
   for (int p = 0; p < s.P; ++p) {
     int n = 0;
     for (int mu = 0; mu < kMaxR; ++mu)

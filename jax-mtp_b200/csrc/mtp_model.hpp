@@ -86,7 +86,6 @@ struct Schedule {
   int D = 0;              // max degree
   int P = 0;              // distinct monomials
   std::vector<int> mono_abc;    // [P][4] (a, b, c, degree), degree descending
-  std::vector<int> nmu;         // [D + 1] radial functions with a basic moment of each degree
   std::vector<int> mono_k;      // [P][kMaxR] basic-moment index for each mu or -1
   // the same for the evaluation kernel: a | b << 4 | c << 8 | n << 12 |
   // (first of n entries in mono_list) << 16 with n = 1 + the monomial's

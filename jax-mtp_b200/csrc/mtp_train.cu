@@ -25,7 +25,6 @@ struct TrainSmem {
   size_t v, rad, st, jt, mono, chain, part, gxi, grad, cnt, total;
 };
 
-template <typename T>
 __host__ __device__ inline TrainSmem train_layout(const DevModel& md, bool vglobal, int n_pad, int qs, int threads) {
   const int S = md.S, R = md.R, K = md.K, D = md.D;
   TrainSmem L;
@@ -45,14 +44,14 @@ __host__ __device__ inline TrainSmem train_layout(const DevModel& md, bool vglob
     o = at + bytes;
     return at;
   };
-  L.v = take(vglobal ? 0 : sizeof(T) * 2 * md.v_size);
-  L.rad = take(sizeof(T) * S * S * R * K);
-  L.st = take(sizeof(T) * L.rows * L.qs);
+  L.v = take(vglobal ? 0 : sizeof(double) * 2 * md.v_size);
+  L.rad = take(sizeof(double) * S * S * R * K);
+  L.st = take(sizeof(double) * L.rows * L.qs);
   L.jt = take(sizeof(int) * L.qs);
   L.mono = take(sizeof(int) * md.P + sizeof(uint16_t) * md.n_list);
-  L.chain = !vglobal && md.chain_mode >= 0 ? L.v + sizeof(T) * 2 * md.v_dm : take(2 * sizeof(T) * md.n3_len);
-  const size_t part = train_group_warps(threads / 32, n_pad) > 1 ? sizeof(T) * 2 * threads : 0;
-  L.part = !vglobal && part <= sizeof(T) * 2 * md.M ? L.v : take(part);
+  L.chain = !vglobal && md.chain_mode >= 0 ? L.v + sizeof(double) * 2 * md.v_dm : take(2 * sizeof(double) * md.n3_len);
+  const size_t part = train_group_warps(threads / 32, n_pad) > 1 ? sizeof(double) * 2 * threads : 0;
+  L.part = !vglobal && part <= sizeof(double) * 2 * md.M ? L.v : take(part);
   L.gxi = take(sizeof(double) * S);
   L.grad = take(sizeof(double) * S * S * R * K);
   L.cnt = take(sizeof(int) * (threads / 32 + 1));
@@ -60,38 +59,23 @@ __host__ __device__ inline TrainSmem train_layout(const DevModel& md, bool vglob
   return L;
 }
 
-// A value and its tangent side by side, so one 16-byte access serves both.
-template <typename T>
-struct Dual2;
-template <>
-struct Dual2<double> {
-  using type = double2;
-  static __device__ __forceinline__ double2 make(double v, double t) { return make_double2(v, t); }
-};
-template <>
-struct Dual2<float> {
-  using type = float2;
-  static __device__ __forceinline__ float2 make(float v, float t) { return make_float2(v, t); }
-};
-
 // Forward pass on duals: (m3, dm3) += c * (m1 m2, dm1 m2 + m1 dm2).
 // Operands are read through Vr and flushes go through V: a pass never reads
 // a slot that it writes, so the two views do not alias (which lets the loads
 // of later entries move ahead of earlier flushes).
-template <typename T>
+// A value and its tangent sit side by side, so one 16-byte access serves both.
 struct DualOperands {
-  typename Dual2<T>::type a, b;
+  double2 a, b;
 };
 
-template <typename T>
 struct DualFwdBody {
-  using Operands = DualOperands<T>;
-  typename Dual2<T>::type* __restrict__ V;
-  const typename Dual2<T>::type* __restrict__ Vr;
-  T acc, tac;
+  using Operands = DualOperands;
+  double2* __restrict__ V;
+  const double2* __restrict__ Vr;
+  double acc, tac;
   __device__ __forceinline__ Operands load(const uint2 e) const { return {Vr[e.x & 0xFFFFu], Vr[e.x >> 16]}; }
   __device__ __forceinline__ void apply(const uint2 e, const Operands& o) {
-    const T c = entry_mult<T>(e.y);
+    const double c = entry_mult<double>(e.y);
     const auto A = o.a, B = o.b;
     acc = dev_fma(c * A.x, B.x, acc);
     tac = dev_fma(c, dev_fma(A.y, B.x, A.x * B.y), tac);
@@ -99,28 +83,27 @@ struct DualFwdBody {
     if (op) {
       const uint32_t d = e.y >> kDstShift;
       if (op == kOpStore) {
-        V[d] = Dual2<T>::make(acc, tac);
+        V[d] = make_double2(acc, tac);
       } else {
         const auto o = V[d];
-        V[d] = Dual2<T>::make(o.x + acc, o.y + tac);
+        V[d] = make_double2(o.x + acc, o.y + tac);
       }
-      acc = T(0);
-      tac = T(0);
+      acc = 0.0;
+      tac = 0.0;
     }
   }
 };
 
 // Reverse pass on duals (entries dst = adj[s], a = adj[t], b = m[o]):
 //   lambda_s += c (lambda_t m_o + tau_t dm_o),  tau_s += c tau_t m_o.
-template <typename T>
 struct DualRevBody {
-  using Operands = DualOperands<T>;
-  typename Dual2<T>::type* __restrict__ V;
-  const typename Dual2<T>::type* __restrict__ Vr;
-  T acc, tac;
+  using Operands = DualOperands;
+  double2* __restrict__ V;
+  const double2* __restrict__ Vr;
+  double acc, tac;
   __device__ __forceinline__ Operands load(const uint2 e) const { return {Vr[e.x & 0xFFFFu], Vr[e.x >> 16]}; }
   __device__ __forceinline__ void apply(const uint2 e, const Operands& o) {
-    const T c = entry_mult<T>(e.y);
+    const double c = entry_mult<double>(e.y);
     const auto A = o.a, B = o.b;   // (lambda_t, tau_t), (m_o, dm_o)
     acc = dev_fma(c, dev_fma(A.x, B.x, A.y * B.y), acc);
     tac = dev_fma(c * A.y, B.x, tac);
@@ -128,13 +111,13 @@ struct DualRevBody {
     if (op) {
       const uint32_t d = e.y >> kDstShift;
       if (op == kOpStore) {
-        V[d] = Dual2<T>::make(acc, tac);
+        V[d] = make_double2(acc, tac);
       } else {
         const auto o = V[d];
-        V[d] = Dual2<T>::make(o.x + acc, o.y + tac);
+        V[d] = make_double2(o.x + acc, o.y + tac);
       }
-      acc = T(0);
-      tac = T(0);
+      acc = 0.0;
+      tac = 0.0;
     }
   }
 };
@@ -258,28 +241,27 @@ struct TrainSlot {
 // from the block's slice of global memory (level 28).  Adjoint and reduction,
 // FP64, with the layout of the evaluation's phases: level 20, 4,968 atoms 0.77
 // -> 0.51 ms; level 28, 18,515 atoms 35.8 -> 31.0 ms.
-template <typename T, bool kVGlobal>
+template <bool kVGlobal>
 __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, int n_pad, void* vscratch,
                                                      double* partials) {
   extern __shared__ __align__(32) unsigned char smem[];
   const int NT = blockDim.x, tid = threadIdx.x;
   const int my_wsteps = warp_steps_of_lane(md, tid, NT);
   const int S = md.S, R = md.R, K = md.K, P = md.P, D1 = md.D + 1;
-  const TrainSmem L = train_layout<T>(md, kVGlobal, n_pad, io.qs, NT);
-  using T2 = typename Dual2<T>::type;
+  const TrainSmem L = train_layout(md, kVGlobal, n_pad, io.qs, NT);
   // program entries in flight per thread; with the value space in global
   // memory their operand gathers are issued before any of their flushes
   // (level 28, 32 configurations: 26.1 ms with two entries in flight and
   // gathers at use -> 19.0 ms)
   constexpr int kStreamDepth = kPrefetch;
-  T2* V = kVGlobal ? reinterpret_cast<T2*>(vscratch) + static_cast<size_t>(blockIdx.x) * md.v_size
-                   : reinterpret_cast<T2*>(smem + L.v);
-  T* sRad = reinterpret_cast<T*>(smem + L.rad);
-  T* sSt = reinterpret_cast<T*>(smem + L.st);
+  double2* V = kVGlobal ? reinterpret_cast<double2*>(vscratch) + static_cast<size_t>(blockIdx.x) * md.v_size
+                        : reinterpret_cast<double2*>(smem + L.v);
+  double* sRad = reinterpret_cast<double*>(smem + L.rad);
+  double* sSt = reinterpret_cast<double*>(smem + L.st);
   int* sJt = reinterpret_cast<int*>(smem + L.jt);
   int* sMono = reinterpret_cast<int*>(smem + L.mono);
   uint16_t* sList = reinterpret_cast<uint16_t*>(sMono + P);
-  T2* sChain = reinterpret_cast<T2*>(smem + L.chain);
+  double2* sChain = reinterpret_cast<double2*>(smem + L.chain);
   double* gXi = reinterpret_cast<double*>(smem + L.gxi);
   double* gRad = reinterpret_cast<double*>(smem + L.grad);
   int* sCnt = reinterpret_cast<int*>(smem + L.cnt);
@@ -291,22 +273,22 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
   double* out = partials + static_cast<size_t>(blockIdx.x) * (md.Sa + S + nrad);
 
   for (int x = tid; x < nrad; x += NT) {
-    sRad[x] = static_cast<T>(md.radial[x]);
+    sRad[x] = md.radial[x];
     gRad[x] = 0.0;
   }
   for (int x = tid; x < P; x += NT) sMono[x] = md.mono_word[x];
   for (int x = tid; x < md.n_list; x += NT) sList[x] = static_cast<uint16_t>(md.mono_list[x]);
   for (int x = tid; x < md.Sa; x += NT) out[x] = 0.0;
   for (int x = tid; x < S; x += NT) gXi[x] = 0.0;
-  for (int x = tid; x < md.ndm_zero; x += NT) V[md.v_dm + md.dm_zero[x]] = Dual2<T>::make(T(0), T(0));
+  for (int x = tid; x < md.ndm_zero; x += NT) V[md.v_dm + md.dm_zero[x]] = make_double2(0.0, 0.0);
   if (tid == 0) {
-    V[md.v_zero] = Dual2<T>::make(T(0), T(0));
-    V[md.v_one] = Dual2<T>::make(T(1), T(0));
+    V[md.v_zero] = make_double2(0.0, 0.0);
+    V[md.v_one] = make_double2(1.0, 0.0);
   }
-  const T rmax = static_cast<T>(md.rmax);
-  const T inv_range = static_cast<T>(1.0 / (md.rmax - md.rmin));
-  const T rsum = static_cast<T>(md.rmin + md.rmax);
-  const T scal = static_cast<T>(md.scaling);
+  const double rmax = md.rmax;
+  const double inv_range = 1.0 / (md.rmax - md.rmin);
+  const double rsum = md.rmin + md.rmax;
+  const double scal = md.scaling;
   auto load_slot = [&](int atom, int s) {
     TrainSlot r{0.0, 0.0, 0.0, -1, -1, 0, 0, 0};
     if (atom < io.natoms) {
@@ -339,25 +321,25 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
       if (tid == 0) atomicOr(io.err, kErrCapacity);
       cfg = 0;
     }
-    const T a_i = static_cast<T>(__ldg(io.gE + cfg));
+    const double a_i = __ldg(io.gE + cfg);
     // C maps r onto the stress-loss direction: sum_v gS_v sigma_v = sum_s (C r_s) . g_s
     const double iv = 1.0 / __ldg(io.volumes + cfg);
     const double* gs = io.gS + 6 * cfg;
-    const T c00 = static_cast<T>(gs[0] * iv), c11 = static_cast<T>(gs[1] * iv), c22 = static_cast<T>(gs[2] * iv);
-    const T c12 = static_cast<T>(0.5 * gs[3] * iv), c02 = static_cast<T>(0.5 * gs[4] * iv);
-    const T c01 = static_cast<T>(0.5 * gs[5] * iv);
-    const T gfx = static_cast<T>(__ldg(io.gF + 3 * atom)), gfy = static_cast<T>(__ldg(io.gF + 3 * atom + 1)),
-            gfz = static_cast<T>(__ldg(io.gF + 3 * atom + 2));
+    const double c00 = gs[0] * iv, c11 = gs[1] * iv, c22 = gs[2] * iv;
+    const double c12 = 0.5 * gs[3] * iv, c02 = 0.5 * gs[4] * iv;
+    const double c01 = 0.5 * gs[5] * iv;
+    const double gfx = __ldg(io.gF + 3 * atom), gfy = __ldg(io.gF + 3 * atom + 1),
+            gfz = __ldg(io.gF + 3 * atom + 2);
     int cnt = ahead.cnt;
     if (cnt > n_pad || cnt < 0) {
       if (tid == 0) atomicOr(io.err, kErrCapacity);
       cnt = cnt < 0 ? 0 : n_pad;
     }
     // (the exchange of the last phase may have used these slots)
-    for (int x = tid; x < md.nzero; x += NT) V[md.v_m + md.zero_list[x]] = Dual2<T>::make(T(0), T(0));
+    for (int x = tid; x < md.nzero; x += NT) V[md.v_m + md.zero_list[x]] = make_double2(0.0, 0.0);
     for (int x = tid; x < md.nseed; x += NT) {
-      const T sv = static_cast<T>(md.seed_val[x]);
-      V[md.v_dm + md.seed_idx[x]] = Dual2<T>::make(a_i * sv, sv);
+      const double sv = md.seed_val[x];
+      V[md.v_dm + md.seed_idx[x]] = make_double2(a_i * sv, sv);
     }
 
     // ---- N1: stage neighbours with their tangents -------------------------
@@ -366,21 +348,21 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
       const int s = s0 + tid;
       const TrainSlot row = s0 == 0 ? ahead : load_slot(atom, s);
       bool valid = false;
-      T rx = T(0), ry = T(0), rz = T(0), d = T(0);
+      double rx = 0.0, ry = 0.0, rz = 0.0, d = 0.0;
       int jt = -1, j = -1;
       if (s < io.nbr_stride && s < cnt) {
         jt = row.jt;
         j = row.j;
-        rx = static_cast<T>(row.x);
-        ry = static_cast<T>(row.y);
-        rz = static_cast<T>(row.z);
+        rx = row.x;
+        ry = row.y;
+        rz = row.z;
         if (jt >= S) {
           atomicOr(io.err, kErrSpecies);
           jt = -1;
         }
-        const T r2 = rx * rx + ry * ry + rz * rz;
+        const double r2 = rx * rx + ry * ry + rz * rz;
         d = dev_sqrt(r2);
-        valid = (jt >= 0) && (r2 > T(0)) && (d < rmax);
+        valid = (jt >= 0) && (r2 > 0.0) && (d < rmax);
       }
       const unsigned bal = __ballot_sync(0xffffffffu, valid);
       const int w = tid >> 5, l = tid & 31;
@@ -391,40 +373,40 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
       const int all = __reduce_add_sync(0xffffffffu, wc);
       if (valid) {
         const int q = nv + before + __popc(bal & ((1u << l) - 1u));
-        T* st = sSt + q;
-        const T inv_d = T(1) / d;
-        const T ux = rx * inv_d, uy = ry * inv_d, uz = rz * inv_d;
+        double* st = sSt + q;
+        const double inv_d = 1.0 / d;
+        const double ux = rx * inv_d, uy = ry * inv_d, uz = rz * inv_d;
         // direction of the neighbour vector: force part + stress part
-        T drx = gfx, dry = gfy, drz = gfz;
+        double drx = gfx, dry = gfy, drz = gfz;
         if (j >= 0 && j < io.natoms) {
-          drx -= static_cast<T>(__ldg(io.gF + 3 * j));
-          dry -= static_cast<T>(__ldg(io.gF + 3 * j + 1));
-          drz -= static_cast<T>(__ldg(io.gF + 3 * j + 2));
+          drx -= __ldg(io.gF + 3 * j);
+          dry -= __ldg(io.gF + 3 * j + 1);
+          drz -= __ldg(io.gF + 3 * j + 2);
         }
         drx += c00 * rx + c01 * ry + c02 * rz;
         dry += c01 * rx + c11 * ry + c12 * rz;
         drz += c02 * rx + c12 * ry + c22 * rz;
-        const T dd = ux * drx + uy * dry + uz * drz;
+        const double dd = ux * drx + uy * dry + uz * drz;
         st[L.du * qs] = (drx - ux * dd) * inv_d;
         st[(L.du + 1) * qs] = (dry - uy * dd) * inv_d;
         st[(L.du + 2) * qs] = (drz - uz * dd) * inv_d;
         st[(L.du + 3) * qs] = dd;
         sJt[q] = jt;
-        const T x = (T(2) * d - rsum) * inv_range;
-        const T dxdd = T(2) * inv_range;
-        const T gap = rmax - d;
-        const T smooth = gap * gap;
-        const T* c = sRad + (static_cast<size_t>(it) * S + jt) * R * K;
-        T base[kMaxR], dbase[kMaxR];
+        const double x = (2.0 * d - rsum) * inv_range;
+        const double dxdd = 2.0 * inv_range;
+        const double gap = rmax - d;
+        const double smooth = gap * gap;
+        const double* c = sRad + (static_cast<size_t>(it) * S + jt) * R * K;
+        double base[kMaxR], dbase[kMaxR];
 #pragma unroll
         for (int mu = 0; mu < kMaxR; ++mu) {
-          base[mu] = T(0);
-          dbase[mu] = T(0);
+          base[mu] = 0.0;
+          dbase[mu] = 0.0;
         }
-        T t_prev = T(0), t_cur = T(1), dt_prev = T(0), dt_cur = T(0);
+        double t_prev = 0.0, t_cur = 1.0, dt_prev = 0.0, dt_cur = 0.0;
         for (int n = 0; n < K; ++n) {
           st[(L.phi + n) * qs] = scal * smooth * t_cur;
-          st[(L.phip + n) * qs] = scal * (T(-2) * gap * t_cur + smooth * dt_cur * dxdd);
+          st[(L.phip + n) * qs] = scal * (-2.0 * gap * t_cur + smooth * dt_cur * dxdd);
 #pragma unroll
           for (int mu = 0; mu < kMaxR; ++mu) {
             if (mu < R) {
@@ -432,13 +414,13 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
               dbase[mu] = dev_fma(c[mu * K + n], dt_cur, dbase[mu]);
             }
           }
-          T t_next, dt_next;
+          double t_next, dt_next;
           if (n == 0) {
             t_next = x;
-            dt_next = T(1);
+            dt_next = 1.0;
           } else {
-            t_next = T(2) * x * t_cur - t_prev;
-            dt_next = T(2) * t_cur + T(2) * x * dt_cur - dt_prev;
+            t_next = 2.0 * x * t_cur - t_prev;
+            dt_next = 2.0 * t_cur + 2.0 * x * dt_cur - dt_prev;
           }
           t_prev = t_cur;
           t_cur = t_next;
@@ -449,11 +431,11 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
         for (int mu = 0; mu < kMaxR; ++mu) {
           if (mu < R) {
             st[(L.f + mu) * qs] = scal * smooth * base[mu];
-            st[(L.fp + mu) * qs] = scal * (T(-2) * gap * base[mu] + smooth * dbase[mu] * dxdd);
+            st[(L.fp + mu) * qs] = scal * (-2.0 * gap * base[mu] + smooth * dbase[mu] * dxdd);
           }
         }
-        T* pw = st + L.pw * qs;
-        T px = T(1), py = T(1), pz = T(1);
+        double* pw = st + L.pw * qs;
+        double px = 1.0, py = 1.0, pz = 1.0;
         for (int e = 0; e < D1; ++e) {
           pw[e * qs] = px;
           pw[(D1 + e) * qs] = py;
@@ -469,7 +451,7 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
     // rows end at a whole 16-byte word: the slot past an odd count adds nothing
     // (all rows zero, the species one that no gradient matches)
     if (nv & 1) {
-      for (int r = tid; r < L.rows; r += NT) sSt[r * qs + nv] = T(0);
+      for (int r = tid; r < L.rows; r += NT) sSt[r * qs + nv] = 0.0;
       if (tid == 0) sJt[nv] = -1;
     }
     __syncthreads();
@@ -481,12 +463,12 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
       const int word = sMono[act ? P - 1 - (t0 + tid) : 0];
       const int nm = __reduce_max_sync(0xffffffffu, act ? word >> 12 & 15 : 0);
       const int ea = word & 15, eb = word >> 4 & 15, ec = word >> 8 & 15;
-      const T* px = sSt + (L.pw + ea) * qs;
-      const T* py = sSt + (L.pw + D1 + eb) * qs;
-      const T* pz = sSt + (L.pw + 2 * D1 + ec) * qs;
-      T acc[kMaxR], tac[kMaxR];
+      const double* px = sSt + (L.pw + ea) * qs;
+      const double* py = sSt + (L.pw + D1 + eb) * qs;
+      const double* pz = sSt + (L.pw + 2 * D1 + ec) * qs;
+      double acc[kMaxR], tac[kMaxR];
 #pragma unroll
-      for (int mu = 0; mu < kMaxR; ++mu) acc[mu] = tac[mu] = T(0);
+      for (int mu = 0; mu < kMaxR; ++mu) acc[mu] = tac[mu] = 0.0;
       switch (nm) {
         case 0: break;
 #define MTP_DUAL(NM) \
@@ -499,21 +481,21 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
         const uint16_t* k = sList + (static_cast<unsigned>(word) >> 16);
 #pragma unroll
         for (int mu = 0; mu < kMaxR; ++mu)
-          if (mu < (word >> 12 & 15) && k[mu] != 0xFFFFu) V[md.v_m + k[mu]] = Dual2<T>::make(acc[mu], tac[mu]);
+          if (mu < (word >> 12 & 15) && k[mu] != 0xFFFFu) V[md.v_m + k[mu]] = make_double2(acc[mu], tac[mu]);
       }
     }
     __syncthreads();
 
     // ---- dual forward tree --------------------------------------------------
     for (int ps = 0; ps < md.nfwd; ++ps) {
-      DualFwdBody<T> body{V, V, T(0), T(0)};
+      DualFwdBody body{V, V, 0.0, 0.0};
       stream_entries_n<kStreamDepth, kVGlobal>(md.entries + md.fwd[ps].offset,
                                                __shfl_sync(0xFFFFFFFFu, my_wsteps, ps), NT, tid, body);
       __syncthreads();
     }
     // four coefficients at a time, so that their loads overlap
     for (int a0 = tid; a0 < md.Sa; a0 += 4 * NT) {
-      T2 v[4];
+      double2 v[4];
       double o[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k)
@@ -524,13 +506,13 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
 #pragma unroll
       for (int k = 0; k < 4; ++k)
         if (a0 + k * NT < md.Sa)
-          out[a0 + k * NT] = o[k] + (static_cast<double>(a_i) * static_cast<double>(v[k].x) + static_cast<double>(v[k].y));
+          out[a0 + k * NT] = o[k] + (a_i * v[k].x + v[k].y);
     }
-    if (tid == 0) gXi[it] += static_cast<double>(a_i);
+    if (tid == 0) gXi[it] += a_i;
 
     // ---- dual reverse tree ---------------------------------------------------
     for (int ps = 0; ps < md.nrev; ++ps) {
-      DualRevBody<T> body{V, V, T(0), T(0)};
+      DualRevBody body{V, V, 0.0, 0.0};
       stream_entries_n<kStreamDepth, kVGlobal>(md.entries + md.rev[ps].offset,
                                                __shfl_sync(0xFFFFFFFFu, my_wsteps, md.nfwd + ps), NT, tid, body);
       __syncthreads();
@@ -540,7 +522,7 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
     const bool in_place = !kVGlobal && md.chain_mode >= 0;
     for (int x = tid; x < (in_place ? 0 : md.n3_len); x += NT) {
       const int k = md.chain_mode >= 0 ? x : __ldg(md.n3_src + x);   // structured: placed in chain order
-      sChain[x] = k >= 0 ? V[md.v_dm + k] : Dual2<T>::make(T(0), T(0));
+      sChain[x] = k >= 0 ? V[md.v_dm + k] : make_double2(0.0, 0.0);
     }
     ahead = load_slot(atom + gridDim.x, tid);
     __syncthreads();
@@ -568,7 +550,7 @@ __global__ void __launch_bounds__(512) k_mtp_adjoint(DevModel md, TrainIO io, in
     // ---- N4: radial coefficient gradient, one thread per (species, mu, n) ----
     for (int x = tid; x < S * R * K; x += NT) {
       const int jt = x / (R * K), mu = x / K % R, n = x % K;
-      const T *pa = sSt + (L.A + mu) * qs, *pb = sSt + (L.B + mu) * qs, *pf = sSt + (L.phi + n) * qs,
+      const double *pa = sSt + (L.A + mu) * qs, *pb = sSt + (L.B + mu) * qs, *pf = sSt + (L.phi + n) * qs,
               *pg = sSt + (L.phip + n) * qs;
       double g = 0.0;
       for (int q = 0; q < nv; q += 2) {
@@ -620,7 +602,7 @@ template <bool G>
 static cudaError_t adjoint_smem_limit(size_t bytes) {
   static size_t granted = 0;
   if (bytes <= granted) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(k_mtp_adjoint<double, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(k_mtp_adjoint<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(bytes));
   if (e == cudaSuccess) granted = bytes;
   return e;
@@ -634,7 +616,7 @@ static int adjoint_occupancy(size_t bytes, int threads) {
     cudaGetLastError();
     return 0;
   }
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_mtp_adjoint<double, G>, threads, bytes) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_mtp_adjoint<G>, threads, bytes) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -643,8 +625,8 @@ static int adjoint_occupancy(size_t bytes, int threads) {
 
 static TrainSmem adjoint_layout_of(const DevModel& md, bool vglobal, int n_pad, int threads) {
   const int qs = row_stride<double>(
-      n_pad, threads, [&](int q) { return train_layout<double>(md, vglobal, n_pad, q, threads).total; });
-  return train_layout<double>(md, vglobal, n_pad, qs, threads);
+      n_pad, threads, [&](int q) { return train_layout(md, vglobal, n_pad, q, threads).total; });
+  return train_layout(md, vglobal, n_pad, qs, threads);
 }
 
 bool adjoint_fits_shared(const DevModel& md, int n_pad, int threads) {
@@ -702,9 +684,9 @@ cudaError_t launch_adjoint(const DevModel& md, const TrainIO& in, int threads, i
   }
   if (io.natoms > 0) {
     if (vglobal)
-      k_mtp_adjoint<double, true><<<blocks, threads, L.total, st>>>(md, io, n_pad, ws.vscratch, ws.partials);
+      k_mtp_adjoint<true><<<blocks, threads, L.total, st>>>(md, io, n_pad, ws.vscratch, ws.partials);
     else
-      k_mtp_adjoint<double, false><<<blocks, threads, L.total, st>>>(md, io, n_pad, ws.vscratch, ws.partials);
+      k_mtp_adjoint<false><<<blocks, threads, L.total, st>>>(md, io, n_pad, ws.vscratch, ws.partials);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     k_adjoint_reduce<<<(np + 31) / 32, 256, 0, st>>>(blocks, md.Sa, md.S, nrad, ws.partials, gmoment, gspecies,
