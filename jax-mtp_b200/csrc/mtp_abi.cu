@@ -365,24 +365,30 @@ int launch_occupancy(mtp_handle* h, int lanes, int stride, bool fp64, bool vglob
   return MTP_OK;
 }
 
-// Expected time (us) of an evaluation of natoms with `bps` blocks of `lanes`
-// threads and A atoms per SM.  A block iteration costs a fixed latency, the
-// program's steps (each lane walks T / lanes of the T products three times
-// over) and the throughput of the atoms that share an SM; the blocks run it
-// once per round.  The constants are fitted to 512, 256 and 128 lanes x 1, 2
-// and 4 atoms on 16 to 32,000 atoms at levels 16, 20 and 24 (T = 969, 6,349
-// and 36,170).  Level 24 mixed, measured / estimated: 512 x 1 alone 36 / 36,
-// 512 x 4 alone 54 / 51, 256 x 2 two on an SM 60 / 61, 128 x 1 alone 68 / 68;
-// level 16 FP64 128 x 1 21 / 24, 128 x 2 24 / 27.
-// The rule it replaces took the most atoms in flight whatever the number of
-// atoms, then the most warps: level 24 mixed ran 256 x 1 (7.35 ms at 55,296
-// atoms; 512 x 4 4.15 ms), 16 atoms of level 16 128 x 4 (29 us; 128 x 1 21 us).
-double launch_estimate(const Potential& pot, bool fp64, int lanes, int A, int bps, int sms, long long natoms) {
+// Expected time (us) of an evaluation of natoms in rows of `slots` with `bps`
+// blocks of `lanes` threads and A atoms per SM; the blocks run an iteration once
+// per round.  An iteration has a latency (each lane walks T / lanes of the T
+// products three times over, and its share of the slots and basic moments B),
+// and the atoms on an SM take their share of its throughput (products, whose
+// program entries a block's atoms share, and slots times moments).  One block's
+// phases add the two up; several blocks fill each other's waits.
+// The constants are fitted to all shapes of levels 16 to 28 (T = 969 to 133,000,
+// B = 130 to 800) on 16 to 300 slots and 16 to 16,000 atoms: the shape taken is
+// within 0.5 % of the best on average, 14 % at worst (a call of 19 us).  Without
+// the slots it was within 2 % and 37 %: level 16 mixed, 4,000 atoms of 200 slots
+// 226 us (128 x 4), now 165 (128 x 1); level 20 FP64, 300 atoms of 200 slots 84 us
+// (512 x 2), now 71 (256 x 1); and the same within 6 % elsewhere.
+double launch_estimate(const Potential& pot, bool fp64, int lanes, int A, int bps, int sms, long long natoms,
+                       int slots) {
   const long long groups = (natoms + A - 1) / A;
   const long long rounds = std::max(1LL, (groups + static_cast<long long>(bps) * sms - 1) / (static_cast<long long>(bps) * sms));
-  const long long resident = std::max(1LL, std::min<long long>(bps, (groups + sms - 1) / sms));
-  const double atom = fp64 ? 2.5 + 2.5e-4 * pot.T : 1.7 + 9e-5 * pot.T;
-  return rounds * (20.0 + 0.15 * pot.T / lanes + atom * A * resident);
+  const double blocks = static_cast<double>(std::max(1LL, std::min<long long>(bps, (groups + sms - 1) / sms)));
+  const double T = pot.T, B = pot.B, share = static_cast<double>(A) * slots / lanes;
+  const double latency = fp64 ? 14.0 + 0.19 * T / lanes + share * (3.4 + 0.023 * B)
+                              : 12.0 + 0.19 * T / lanes + share * (2.2 + 0.013 * B);
+  const double work = fp64 ? blocks * A * (1.0 + 6.7e-5 * T + slots * (2.2e-3 + 8.8e-5 * B))
+                           : blocks * (A * (1.4 + 2.2e-5 * T + slots * (1.7e-3 + 3.4e-5 * B)) + 3e-5 * T);
+  return rounds * (latency + work - (1.0 - 1.0 / blocks) * std::min(latency, work));
 }
 
 // Value spaces in global memory, one slice of A atoms per SM, and the most atoms
@@ -420,7 +426,7 @@ int shared_shapes(mtp_handle* h, long long natoms, int stride, bool fp64, std::v
       if (bps <= 0) continue;
       const double rank = 1e5 * (512 / lanes) - (1024 * A * bps + bps * lanes / 32);   // at most 16 atoms in flight
       out->push_back({lanes, A, bps,
-                      h->threads > 0 ? rank : launch_estimate(h->pot, fp64, lanes, A, bps, h->sm_count, natoms)});
+                      h->threads > 0 ? rank : launch_estimate(h->pot, fp64, lanes, A, bps, h->sm_count, natoms, stride)});
     }
   }
   return MTP_OK;
