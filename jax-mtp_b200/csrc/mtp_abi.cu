@@ -398,7 +398,7 @@ size_t global_space_bytes(const mtp_handle* h, const DeviceSchedule& ds, int A, 
 }
 
 int global_atoms(const mtp_handle* h, const DeviceSchedule& ds, bool fp64) {
-  return global_space_bytes(h, ds, 2, fp64) <= h->l2_bytes / 4 * 3 ? 2 : 1;
+  return eval_variant_exists(fp64, true, 2) && global_space_bytes(h, ds, 2, fp64) <= h->l2_bytes / 4 * 3 ? 2 : 1;
 }
 
 // One launch shape that fits, and what the choice goes by: the least of the
@@ -433,12 +433,15 @@ int shared_shapes(mtp_handle* h, long long natoms, int stride, bool fp64, std::v
 }
 
 // The same with the value space in global memory: 512 lanes give an SM 16 warps
-// with one block, so the blocks' value spaces stay within L2.  Two atoms share
-// every program entry (4.5 MB an iteration at level 28, as much L2 traffic as
-// the operands) and fill more of each 32-byte sector a gather touches: an
-// iteration takes 1.78x (FP64, 2.20 -> 1.96 ms for 2,048 atoms) or 1.09x (FP32)
-// one atom's time, so they win where that saves a round, as long as the value
-// spaces stay in L2 (four atoms' do not: 3.47 ms).
+// with one block, so the blocks' value spaces stay within L2.  In FP64 two atoms
+// share every program entry (4.5 MB an iteration at level 28, as much L2 traffic
+// as the operands) and fill more of each 32-byte sector a gather touches: an
+// iteration takes 1.78x one atom's time (2.20 -> 1.96 ms for 2,048 atoms), so
+// they win where that saves a round, as long as the value spaces stay in L2
+// (four atoms' do not: 3.47 ms).  FP32 gets here with rows too long for shared
+// memory, whose staging leaves little L1 to the gathers: two atoms take 2.3x one
+// atom's time (level 28, 148 / 296 atoms of 500 slots 180 / 402 us), so there is
+// no such kernel.
 int global_shapes(mtp_handle* h, long long natoms, int stride, bool fp64, std::vector<Shape>* out) {
   const DeviceSchedule* sz = nullptr;
   int st = get_sizes(h, 512, &sz);
@@ -451,7 +454,7 @@ int global_shapes(mtp_handle* h, long long natoms, int stride, bool fp64, std::v
     if (st != MTP_OK) return st;
     if (bps <= 0) continue;
     const long long per = static_cast<long long>(A) * h->sm_count;
-    const double rounds = static_cast<double>((natoms + per - 1) / per) * (A == 1 ? 1.0 : fp64 ? 1.78 : 1.09);
+    const double rounds = static_cast<double>((natoms + per - 1) / per) * (A == 1 ? 1.0 : 1.78);
     const double rank = A == (h->apb == 2 ? 2 : 1) ? 0.0 : 1.0;
     out->push_back({512, A, 1, h->threads > 0 ? rank : rounds});
   }

@@ -71,7 +71,7 @@ cudaError_t launch_t(const DevModel& md, const DevIO& io, int threads, int block
 // Supported (precision, placement, atoms per block) combinations.
 #define MTP_EVAL_VARIANTS(X) \
   X(double, false, 1) X(double, false, 2) X(double, true, 1) X(double, true, 2) X(float, false, 1) X(float, false, 2) \
-  X(float, false, 4) X(float, true, 1) X(float, true, 2)
+  X(float, false, 4) X(float, true, 1)
 
 bool eval_variant_exists(bool fp64, bool vglobal, int A) {
 #define X(T, G, AA) \

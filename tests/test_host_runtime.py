@@ -289,3 +289,13 @@ def test_failed_upload_of_the_tables_is_made_up_for(lib):
             st, log = h.compute(100)
             assert st == 0, h.error()
             assert left + live(log) == whole, n
+
+
+@pytest.mark.parametrize("n", [100, 296, 600])
+def test_mixed_rows_in_global_memory_take_one_atom_per_block(lib, n):
+    """Two take 2.3 times as long as one (level 28, rows of 500 slots)."""
+    with Handle(lib, L28, 600, 500, MIXED) as h:
+        for threads, atoms in ((0, 0), (512, 2)):
+            if threads:
+                h.set_launch(threads, atoms)
+            assert h.compute(n)[0] == 0 and h.launch()["atoms"] == 1
