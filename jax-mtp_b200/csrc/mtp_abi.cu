@@ -64,6 +64,19 @@ cudaError_t dalloc(T** p, size_t n) {
 
 }  // namespace
 
+// One launch shape that fits, and what the choice goes by: the least of the
+// expected times or, with the value space in global memory, of the expected
+// one-atom rounds.  A request (mtp_set_launch) goes by a rank that does not
+// depend on the number of atoms, so that an atom's rounding does not either: the
+// threads asked for, or else the next fewer that fit; of several atoms per block
+// the one with the most atoms in flight per SM, then the most warps.
+struct Shape {
+  int lanes = 0, A = 1;
+  EvalFit fit;
+  double cost = 0.0;
+  bool vglobal = false;
+};
+
 struct mtp_handle {
   Potential pot;
   int max_atoms = 0, max_nbr = 0, debug = 0, precision = 0;
@@ -72,10 +85,7 @@ struct mtp_handle {
   size_t l2_bytes = 0;
   cudaStream_t own_stream = nullptr, stream = nullptr;
   int threads = 0, blocks_per_sm = 0;   // requested launch (mtp_set_launch); 0 threads: automatic
-  int last_threads = 0, last_blocks = 0, last_bps = 0;
-  bool last_vglobal = false;
   void* d_vscratch = nullptr;   // value spaces in global memory, allocated once (pick_launch)
-  size_t last_smem = 0;
   std::map<int, DeviceSchedule> scheds;
   std::map<int, DeviceSchedule> sizes;   // by lanes: schedules without programs, to size launches
   // potential tables on the device
@@ -104,12 +114,12 @@ struct mtp_handle {
   int* h_err = nullptr;      // the flags' word of h_tot
   TrainWorkspace train;
   CellScratch cells;
-  // blocks per SM of a (lanes, atoms per block, stride, precision, value-space
-  // placement): no occupancy queries after the first, so later calls can be
-  // graph-captured
   int apb = 0;          // requested atoms per block (0: chosen by occupancy)
-  int last_apb = 1;
-  std::map<long long, int> occupancy;
+  Shape last;           // the last evaluation's launch
+  int last_blocks = 0;
+  // how a (lanes, atoms per block, stride, precision, value-space placement)
+  // fits: worked out and asked once, so later calls can be graph-captured
+  std::map<long long, EvalFit> fits;
   // profiling of the evaluation kernel
   bool profiling = false;
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> prof_events;
@@ -351,17 +361,18 @@ void free_handle(mtp_handle* h) {
   delete h;
 }
 
-// Blocks of one launch shape an SM holds (0: it does not fit), asked once.
-int launch_occupancy(mtp_handle* h, int lanes, int stride, bool fp64, bool vglobal, int A, int* bps) {
+// How one launch shape fits, within the handle's blocks per SM.
+int launch_fit(mtp_handle* h, int lanes, int stride, bool fp64, bool vglobal, int A, EvalFit* fit) {
   const long long key = (static_cast<long long>(stride) << 20) | (lanes << 4) | (A << 2) | (vglobal ? 2 : 0) | (fp64 ? 1 : 0);
-  auto it = h->occupancy.find(key);
-  if (it == h->occupancy.end()) {
+  auto it = h->fits.find(key);
+  if (it == h->fits.end()) {
     const DeviceSchedule* ds = nullptr;
     int st = get_sizes(h, lanes, &ds);
     if (st != MTP_OK) return st;
-    it = h->occupancy.emplace(key, eval_blocks_per_sm(make_model(h, *ds), stride, lanes, fp64, vglobal, A)).first;
+    it = h->fits.emplace(key, eval_fit(make_model(h, *ds), stride, lanes, fp64, vglobal, A)).first;
   }
-  *bps = h->blocks_per_sm > 0 ? std::min(it->second, h->blocks_per_sm) : it->second;
+  *fit = it->second;
+  if (h->blocks_per_sm > 0) fit->per_sm = std::min(fit->per_sm, h->blocks_per_sm);
   return MTP_OK;
 }
 
@@ -401,17 +412,6 @@ int global_atoms(const mtp_handle* h, const DeviceSchedule& ds, bool fp64) {
   return eval_variant_exists(fp64, true, 2) && global_space_bytes(h, ds, 2, fp64) <= h->l2_bytes / 4 * 3 ? 2 : 1;
 }
 
-// One launch shape that fits, and what the choice goes by: the least of the
-// expected times or, with the value space in global memory, of the expected
-// one-atom rounds.  A request (mtp_set_launch) goes by a rank that does not
-// depend on the number of atoms, so that an atom's rounding does not either: the
-// threads asked for, or else the next fewer that fit; of several atoms per block
-// the one with the most atoms in flight per SM, then the most warps.
-struct Shape {
-  int lanes = 0, A = 1, bps = 0;
-  double cost = 0.0;
-};
-
 // The shapes of the handle's request that fit for natoms, with the value space
 // in shared memory.
 int shared_shapes(mtp_handle* h, long long natoms, int stride, bool fp64, std::vector<Shape>* out) {
@@ -420,13 +420,15 @@ int shared_shapes(mtp_handle* h, long long natoms, int stride, bool fp64, std::v
     for (int A : {4, 2, 1}) {
       if (h->apb > 0 && A != h->apb) continue;
       if (!eval_variant_exists(fp64, false, A)) continue;
-      int bps = 0;
-      const int st = launch_occupancy(h, lanes, stride, fp64, false, A, &bps);
+      EvalFit fit;
+      const int st = launch_fit(h, lanes, stride, fp64, false, A, &fit);
       if (st != MTP_OK) return st;
+      const int bps = fit.per_sm;
       if (bps <= 0) continue;
       const double rank = 1e5 * (512 / lanes) - (1024 * A * bps + bps * lanes / 32);   // at most 16 atoms in flight
-      out->push_back({lanes, A, bps,
-                      h->threads > 0 ? rank : launch_estimate(h->pot, fp64, lanes, A, bps, h->sm_count, natoms, stride)});
+      out->push_back({lanes, A, fit,
+                      h->threads > 0 ? rank : launch_estimate(h->pot, fp64, lanes, A, bps, h->sm_count, natoms, stride),
+                      false});
     }
   }
   return MTP_OK;
@@ -449,14 +451,15 @@ int global_shapes(mtp_handle* h, long long natoms, int stride, bool fp64, std::v
   for (int A : {1, 2}) {
     if (h->apb > 0 && A > h->apb) continue;
     if (A > global_atoms(h, *sz, fp64)) continue;
-    int bps = 0;
-    st = launch_occupancy(h, 512, stride, fp64, true, A, &bps);
+    EvalFit fit;
+    st = launch_fit(h, 512, stride, fp64, true, A, &fit);
     if (st != MTP_OK) return st;
-    if (bps <= 0) continue;
+    if (fit.per_sm <= 0) continue;
+    fit.per_sm = 1;
     const long long per = static_cast<long long>(A) * h->sm_count;
     const double rounds = static_cast<double>((natoms + per - 1) / per) * (A == 1 ? 1.0 : 1.78);
     const double rank = A == (h->apb == 2 ? 2 : 1) ? 0.0 : 1.0;
-    out->push_back({512, A, 1, h->threads > 0 ? rank : rounds});
+    out->push_back({512, A, fit, h->threads > 0 ? rank : rounds, true});
   }
   return MTP_OK;
 }
@@ -501,46 +504,41 @@ Shape best_uploaded_shape(const mtp_handle* h, const std::vector<Shape>& shapes,
 // memory; when none fits, the value space moves to global memory.  While the stream is being captured nothing can be
 // uploaded, so a shape whose programs are not on the device yet gives way to
 // the best one whose are.
-int pick_launch(mtp_handle* h, long long natoms, int stride, const DeviceSchedule** ds_out, int* blocks_out, bool fp64,
-                bool* vglobal_out) {
+int pick_launch(mtp_handle* h, long long natoms, int stride, bool fp64, Shape* shape, const DeviceSchedule** ds) {
   std::vector<Shape> shapes;
+  shapes.reserve(9);
   int st = shared_shapes(h, natoms, stride, fp64, &shapes);
   if (st != MTP_OK) return st;
-  const bool vglobal = shapes.empty();
-  if (vglobal && (st = global_shapes(h, natoms, stride, fp64, &shapes)) != MTP_OK) return st;
+  if (shapes.empty() && (st = global_shapes(h, natoms, stride, fp64, &shapes)) != MTP_OK) return st;
   if (shapes.empty())
     return fail(h, MTP_E_CAPACITY, "the evaluation block does not fit in shared memory for this basis and max_nbr");
   Shape best = best_shape(shapes);
-  const DeviceSchedule* ds = programs_on_device(h, best.lanes, access_width(fp64, best.A), false);
-  if (!ds) {
+  *ds = programs_on_device(h, best.lanes, access_width(fp64, best.A), false);
+  if (!*ds) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) cudaGetLastError();
     if (cs != cudaStreamCaptureStatusNone) {
-      const Shape ready = best_uploaded_shape(h, shapes, fp64, &ds);
-      if (ds) best = ready;
+      const Shape ready = best_uploaded_shape(h, shapes, fp64, ds);
+      if (*ds) best = ready;
     }
   }
-  if (!ds && (st = get_schedule(h, best.lanes, access_width(fp64, best.A), &ds)) != MTP_OK) return st;
-  const long long groups = (natoms + best.A - 1) / best.A;
-  const long long blocks = std::max(1LL, std::min<long long>(static_cast<long long>(best.bps) * h->sm_count, groups));
-  if (vglobal && !h->d_vscratch) {
+  if (!*ds && (st = get_schedule(h, best.lanes, access_width(fp64, best.A), ds)) != MTP_OK) return st;
+  if (best.vglobal && !h->d_vscratch) {
     // for the largest launch any call of this handle can take (one block per SM
     // with the most atoms), once: a graph that a caller captured holds the
     // address, so the buffer must not move when a later call needs more of it
-    const size_t bytes = global_space_bytes(h, *ds, global_atoms(h, *ds, fp64), fp64);
+    const size_t bytes = global_space_bytes(h, **ds, global_atoms(h, **ds, fp64), fp64);
     MTP_CUDA(h, cudaMalloc(&h->d_vscratch, bytes));
     ++h->gen;
   }
-  *ds_out = ds;
-  *blocks_out = static_cast<int>(blocks);
-  *vglobal_out = vglobal;
-  h->last_threads = best.lanes;
-  h->last_blocks = static_cast<int>(blocks);
-  h->last_bps = best.bps;
-  h->last_vglobal = vglobal;
-  h->last_smem = eval_smem_bytes(make_model(h, *ds), stride, best.lanes, fp64, vglobal, best.A);
-  h->last_apb = best.A;
+  *shape = best;
   return MTP_OK;
+}
+
+// Blocks of a launch on natoms: every SM full, or one group of atoms each.
+int launch_blocks(const mtp_handle* h, const Shape& s, long long natoms) {
+  const long long most = static_cast<long long>(s.fit.per_sm) * h->sm_count;
+  return static_cast<int>(std::max(1LL, std::min(most, (natoms + s.A - 1) / s.A)));
 }
 
 // Evaluation kernel on atoms [lo, lo + n) of a system of `natoms` in device
@@ -550,12 +548,10 @@ int eval_range(mtp_handle* h, int natoms, int lo, int n, int stride, const int* 
                const int* counts) {
   const bool fp64 = h->precision == MTP_PRECISION_FP64;
   const DeviceSchedule* ds = nullptr;
-  int blocks = 0;
-  bool vglobal = false;
-  int st = pick_launch(h, natoms, stride, &ds, &blocks, fp64, &vglobal);
+  const int st = pick_launch(h, natoms, stride, fp64, &h->last, &ds);
   if (st != MTP_OK) return st;
-  blocks = std::max(1, std::min(blocks, (n + h->last_apb - 1) / h->last_apb));
-  DevModel md = make_model(h, *ds);
+  h->last_blocks = launch_blocks(h, h->last, natoms);
+  const DevModel md = make_model(h, *ds);
   const size_t rows = static_cast<size_t>(lo) * stride;
   DevIO io{};
   io.natoms = n;
@@ -569,7 +565,8 @@ int eval_range(mtp_handle* h, int natoms, int lo, int n, int stride, const int* 
   io.pair_grad = h->d_G + 3 * rows;
   io.err = h->d_err;
   io.vscratch = h->d_vscratch;
-  MTP_CUDA(h, launch_eval(md, io, h->last_threads, blocks, fp64, vglobal, h->last_apb, h->stream));
+  MTP_CUDA(h, launch_eval(md, io, h->last.fit, h->last.lanes, launch_blocks(h, h->last, n), fp64, h->last.vglobal,
+                          h->last.A, h->stream));
   return MTP_OK;
 }
 
@@ -1087,11 +1084,11 @@ int mtp_set_launch(mtp_handle* h, int threads, int bps, int apb) {
 
 int mtp_get_launch(const mtp_handle* h, int* out5) {
   if (!h || !out5) return MTP_E_INVALID;
-  out5[0] = h->last_threads;
+  out5[0] = h->last.lanes;
   out5[1] = h->last_blocks;
-  out5[2] = static_cast<int>(h->last_smem);
-  out5[3] = h->last_bps;
-  out5[4] = h->last_apb;
+  out5[2] = static_cast<int>(h->last.fit.smem);
+  out5[3] = h->last.fit.per_sm;
+  out5[4] = h->last.A;
   return MTP_OK;
 }
 
@@ -1719,11 +1716,9 @@ int mtp_compute_device_noalloc(mtp_handle* h, int natoms, int stride, const int*
   io.pair_grad = grad;
   io.err = h->d_err;
   io.vscratch = nullptr;
-  const long long groups = (static_cast<long long>(natoms) + shape.A - 1) / shape.A;
-  const int blocks = static_cast<int>(std::max(1LL, std::min<long long>(static_cast<long long>(shape.bps) * h->sm_count,
-                                                                         groups)));
   MTP_CUDA(h, launch_incoming(natoms, stride, d_js, d_jtypes, d_counts, in_cnt, in_ptr, in_slot, blk, false, h->stream));
-  MTP_CUDA(h, launch_eval(md, io, shape.lanes, blocks, fp64, false, shape.A, h->stream));
+  MTP_CUDA(h, launch_eval(md, io, shape.fit, shape.lanes, launch_blocks(h, shape, natoms), fp64, false, shape.A,
+                          h->stream));
   MTP_CUDA(h, launch_force_gather(natoms, stride, d_rijs, d_counts, grad, in_ptr, in_slot, true, d_forces, wown, nullptr,
                                   h->stream));
   st = write_totals(h, natoms, energy, wown, partials, tot, d_energy, d_virial);

@@ -86,7 +86,7 @@ struct DevIO {
   int natoms;
   int nbr_stride;
   int n_pad;                // slots of a staging row (>= max count, <= nbr_stride rounded)
-  int qs;                   // its stride (row_stride; set by launch_eval)
+  int qs;                   // its stride (EvalFit; set by launch_eval)
   const int* itypes;        // [natoms]
   const double* rijs;       // [natoms][nbr_stride][3]
   const int* jtypes;        // [natoms][nbr_stride]

@@ -20,14 +20,6 @@ static SmemLayout eval_layout(const DevModel& md, int n_pad, int threads, bool v
   return layout(row_stride<T>(n_pad, threads, [&](int qs) { return layout(qs).total; }));
 }
 
-static SmemLayout eval_layout(const DevModel& md, int n_pad, int threads, bool fp64, bool vglobal, int A) {
-  return fp64 ? eval_layout<double>(md, n_pad, threads, vglobal, A) : eval_layout<float>(md, n_pad, threads, vglobal, A);
-}
-
-size_t eval_smem_bytes(const DevModel& md, int n_pad, int threads, bool fp64, bool vglobal, int A) {
-  return eval_layout(md, n_pad, threads, fp64, vglobal, A).total;
-}
-
 namespace {
 
 // The dynamic shared-memory limit of each instantiation only ever grows, so a
@@ -81,24 +73,28 @@ bool eval_variant_exists(bool fp64, bool vglobal, int A) {
   return false;
 }
 
-int eval_blocks_per_sm(const DevModel& md, int n_pad, int threads, bool fp64, bool vglobal, int A) {
-  const size_t bytes = eval_smem_bytes(md, n_pad, threads, fp64, vglobal, A);
-#define X(T, G, AA) \
-  if ((fp64 == std::is_same<T, double>::value) && vglobal == G && A == AA) return occupancy_t<T, G, AA>(bytes, threads);
-  MTP_EVAL_VARIANTS(X)
-#undef X
-  return 0;
-}
-
-cudaError_t launch_eval(const DevModel& md, const DevIO& io, int threads, int blocks, bool fp64, bool vglobal, int A,
-                        cudaStream_t st) {
-  if (io.natoms <= 0) return cudaSuccess;
-  const SmemLayout L = eval_layout(md, io.n_pad, threads, fp64, vglobal, A);
-  DevIO rows = io;
-  rows.qs = L.qs;
+EvalFit eval_fit(const DevModel& md, int n_pad, int threads, bool fp64, bool vglobal, int A) {
+  const SmemLayout L = fp64 ? eval_layout<double>(md, n_pad, threads, vglobal, A)
+                            : eval_layout<float>(md, n_pad, threads, vglobal, A);
+  EvalFit fit;
+  fit.qs = L.qs;
+  fit.smem = L.total;
 #define X(T, G, AA) \
   if ((fp64 == std::is_same<T, double>::value) && vglobal == G && A == AA) \
-    return launch_t<T, G, AA>(md, rows, threads, blocks, L.total, st);
+    fit.per_sm = occupancy_t<T, G, AA>(L.total, threads);
+  MTP_EVAL_VARIANTS(X)
+#undef X
+  return fit;
+}
+
+cudaError_t launch_eval(const DevModel& md, const DevIO& io, const EvalFit& fit, int threads, int blocks, bool fp64,
+                        bool vglobal, int A, cudaStream_t st) {
+  if (io.natoms <= 0) return cudaSuccess;
+  DevIO rows = io;
+  rows.qs = fit.qs;
+#define X(T, G, AA) \
+  if ((fp64 == std::is_same<T, double>::value) && vglobal == G && A == AA) \
+    return launch_t<T, G, AA>(md, rows, threads, blocks, fit.smem, st);
   MTP_EVAL_VARIANTS(X)
 #undef X
   return cudaErrorInvalidValue;

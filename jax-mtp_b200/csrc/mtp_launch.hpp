@@ -9,15 +9,18 @@ namespace mtp {
 
 constexpr int kReduceBlocks = 256;   // fixed: the reduction order never depends on the GPU
 
-// Dynamic shared memory of the evaluation kernel for A atoms per block
+bool eval_variant_exists(bool fp64, bool vglobal, int A);
+// How a launch shape of the evaluation kernel fits: blocks per SM (0: not at
+// all), the stride of a staging row and a block's dynamic shared memory
 // (vglobal: value space in global memory, io.vscratch holding
 // blocks * A * v_size values).
-size_t eval_smem_bytes(const DevModel& md, int n_pad, int threads, bool fp64, bool vglobal, int A);
-bool eval_variant_exists(bool fp64, bool vglobal, int A);
-// Blocks per SM that fit for the evaluation kernel (0 if it does not fit).
-int eval_blocks_per_sm(const DevModel& md, int n_pad, int threads, bool fp64, bool vglobal, int A);
-cudaError_t launch_eval(const DevModel& md, const DevIO& io, int threads, int blocks, bool fp64, bool vglobal, int A,
-                        cudaStream_t st);
+struct EvalFit {
+  int per_sm = 0, qs = 0;
+  size_t smem = 0;
+};
+EvalFit eval_fit(const DevModel& md, int n_pad, int threads, bool fp64, bool vglobal, int A);
+cudaError_t launch_eval(const DevModel& md, const DevIO& io, const EvalFit& fit, int threads, int blocks, bool fp64,
+                        bool vglobal, int A, cudaStream_t st);
 
 // Incoming-slot lists: for every atom k, the slots (i, s) whose neighbour is k,
 // in any order (launch_force_gather sorts them).  in_ptr [natoms + 1].
