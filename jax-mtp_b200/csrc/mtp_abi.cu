@@ -438,9 +438,10 @@ int shared_shapes(mtp_handle* h, long long natoms, int stride, bool fp64, std::v
 // with one block, so the blocks' value spaces stay within L2.  In FP64 two atoms
 // share every program entry (4.5 MB an iteration at level 28, as much L2 traffic
 // as the operands) and fill more of each 32-byte sector a gather touches: an
-// iteration takes 1.78x one atom's time (2.20 -> 1.96 ms for 2,048 atoms), so
-// they win where that saves a round, as long as the value spaces stay in L2
-// (four atoms' do not: 3.47 ms).  FP32 gets here with rows too long for shared
+// iteration takes 1.45x one atom's time on 64 slots and 1.87x on 200 (1.78 stands
+// for all; 1,200 atoms of 64 slots 1.39 -> 1.11 ms), so they win where that saves
+// a round, as long as the value spaces stay in L2 (four atoms' do not: 2,048
+// atoms 3.47 ms, two 1.96).  FP32 gets here with rows too long for shared
 // memory, whose staging leaves little L1 to the gathers: two atoms take 2.3x one
 // atom's time (level 28, 148 / 296 atoms of 500 slots 180 / 402 us), so there is
 // no such kernel.
